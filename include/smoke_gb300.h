@@ -216,12 +216,14 @@ int smk_get_sweep_kernel(const smk_sim* sim, int* depth, int* zchunk);
 int smk_set_sweep_shape(smk_sim* sim, int depth, int rows, int zchunk);
 int smk_get_sweep_shape(const smk_sim* sim, int* depth, int* rows, int* zchunk);
 /* Projection kernel of the REFERENCE scheme (the reference's in-place velocity red-black SOR,
- * smokeSimulation.cu:356-394 run max_sweeps times, :795-801).  depth 0 (default): one colour pass
- * per launch, as the reference launches it; depth 2 or 4: temporally blocked, `depth` colour
- * passes per pass over HBM on z-chunks of `zchunk` planes (0: chosen from the grid), with the
- * simulation's pressure buffers as scratch (a later PRESSURE step then restarts its pressure from
- * zero); smk_autotune picks the fastest.  Results are bit-identical for every choice.  FP32
- * storage only.  No counterpart in the reference's API. */
+ * smokeSimulation.cu:356-394 run max_sweeps times, :795-801).  depth 0: one colour pass per launch,
+ * as the reference launches it; depth 2 or 4: temporally blocked, `depth` colour passes per pass
+ * over HBM on z-chunks of `zchunk` planes (0: chosen from the grid), with the simulation's pressure
+ * buffers as scratch (a later PRESSURE step then restarts its pressure from zero).  Until it is
+ * called the grid decides: blocked with depth 4 above about 110^3 cells while no PRESSURE step has
+ * left a pressure in those buffers, else one pass per launch.  smk_autotune times them and picks the
+ * fastest.  Results are bit-identical for every choice.  FP32 storage only.
+ * smk_get_velocity_sweep gives the kernel the next step uses.  No counterpart in the reference's API. */
 int smk_set_velocity_sweep(smk_sim* sim, int depth, int zchunk);
 int smk_get_velocity_sweep(const smk_sim* sim, int* depth, int* zchunk);
 /* Replay steady-state steps as a captured CUDA graph (default on).  A graph is re-captured

@@ -369,7 +369,7 @@ class Simulation:
     def set_velocity_sweep(self, depth: int, zchunk: int = 0):
         """REFERENCE-scheme projection kernel: depth 0 = one colour pass per launch, 2 or 4 =
         temporally blocked (depth passes per pass over HBM, z-chunks of zchunk planes, 0 = from
-        the grid); results are identical."""
+        the grid); until it is called the grid decides.  Results are identical."""
         _check(lib().smk_set_velocity_sweep(self.h, depth, zchunk))
 
     def velocity_sweep(self):

@@ -385,6 +385,7 @@ bool grouped_eligible(smk_sim* const* sims, int n) {
 bool grouped_eligible(const smk_batch* b) { return grouped_eligible(b->sims.data(), (int)b->sims.size()); }
 
 void after_step(smk_sim* s) {
+    s->pressure_used = true;
     s->index_now ^= 1;
     ++s->steps;
     ++s->hist_steps;
@@ -557,6 +558,7 @@ int branches_step(smk_batch* b, const float* dts, float dt_all, cudaStream_t st)
     SMK_CUDA(cudaGraphLaunch(b->exec, st));
     for (int i = 0; i < n; ++i) {
         smk_sim* s = b->sims[i];
+        s->mark_scratch();
         s->index_now ^= 1;
         s->launches += b->branch_launches[i];
         b->launches += b->branch_launches[i];
@@ -630,6 +632,10 @@ int group_runner_step(GroupRunner* r, smk_sim* const* sims, const float* dts, in
     if (!grouped_eligible(sims, n))
         return smk_fail(SMK_ERR_INVALID, "a grouped step needs the PRESSURE projection in every member");
     int k = 0;
+    for (int i = 0; i < n; ++i) {
+        const int rc = sims[i]->settle_pressure(st);
+        if (rc) return rc;
+    }
     for (int i = 0; i < n; ++i)
         if (sims[i]->mask_dirty || sims[i]->obstacles_dirty) k += sims[i]->prepare_mask(st);
     TableImage t;
@@ -770,6 +776,10 @@ int smk_batch_step(smk_batch* b, const float* dts, float dt_all, void* stream) {
     // stage timing is per member: per-member steps
     for (const smk_sim* s : b->sims)
         if (s->timing) grouped = false;
+    for (smk_sim* s : b->sims) {
+        const int rc = s->settle_pressure(st);
+        if (rc) return rc;
+    }
     if (grouped) return grouped_step(b, dts, dt_all, st);
     return branches_step(b, dts, dt_all, st);
 }

@@ -1,227 +1,133 @@
 // Exact float arithmetic of the reference's projection step without the FP64 pipe (host and
 // device).  The reference computes p_t = (-div / acc) * OVER_RELAXATION with a float quotient and
-// a double constant (project/smokeSimulation.cu:38, :384): float(double(q) * omega), one
-// rounding to 53 bits and one to 24.  GB300's FP64 rate is a small fraction of its FP32 and
-// integer rates, and the one-pass projection kernel is bound by it (its FP64 pipe runs at ~48 %
-// of peak), so:
-//   omega_scale  forms the 24 x 53-bit significand product with two 32 x 32-bit integer
-//                multiplies, rounds it to 53 and then to 24 bits with ties to even, and builds the
-//                float; zeros directly.  Operands whose result can fall below the normal range
-//                (subnormal q included) take omega_scale_tiny: q normalised, the same product
-//                rounded to 53 bits, then to a multiple of 2^-149 where the result is below
-//                2^-126.  Operands whose result could overflow take the double product.  (Checked
-//                against the double product on every non-NaN float for omega = 1.9 and on
-//                strided samples for other omegas: same bits);
-//   div_small    x / d for d = 1..6, correctly rounded: y = x * RN(1/d) corrected once by the
-//                exact remainder fma(-y, d, x) (Markstein's correction step), on 2^-100 <= |x|
-//                < 2^100 (every float x in that range gave the IEEE quotient's bits for each d);
-//                below that range div_tiny applies the same step to x * 2^64 and scales back
-//                where the quotient is normal, and rounds m / d to the nearest integer (ties to
-//                even) for the quotients below 2^-126, x = m * 2^-149; zeros return x, other
-//                operands take the IEEE division.
-// In a fresh simulation the red-black passes spread values far below 2^-100 (subnormals among
-// them) ahead of the first smoke: about 1 % of the faces for a few steps, so that about half the
-// warps of a pass hold such a lane.  div_scale_fast keeps the common lanes free of branches and
-// the tiny paths keep the rare ones off the FP64 pipe and the general division.
+// a double constant (project/smokeSimulation.cu:38, :384): q = x / d in float, d = 1..6, then
+// float(double(q) * omega): the product rounded to 53 bits and then to 24.  An FP64 product with
+// its two conversions costs three passes through GB300's FP64 pipe (a few lanes per clock and SM),
+// and the IEEE quotient about ten instructions; here a cell takes five FP32 multiplies and FMAs.
+//
+//   Quotient: q = fma(x, zh, x * zl) with zh = 1/d rounded toward zero and zl = 1/d - zh rounded
+//   (division by a known constant as an unevaluated sum, after Brisebarre, Muller and Raina,
+//   "Accelerating correctly rounded floating-point division when the divisor is known in
+//   advance", IEEE Trans. Computers 53(8), 2004).  Before the last rounding the error is below
+//   2^-46 |x/d|, while x/d for d = 3, 5, 6 is never a midpoint of two floats and keeps a distance
+//   of at least 2^-28 |x/d| from every midpoint (d odd: d * midpoint needs 26 bits); d = 1, 2, 4
+//   are exact.  So q is the IEEE quotient while x * zl does not underflow.
+//
+//   Product: with omega = wh + wl, wh rounded toward zero to float (|wl| below its last place) and
+//   wl = wl1 + wl2 as two floats,
+//     c = fma(q, wl1, q * wl2)   q * wl rounded to float, off by 2^-24 |c| at most,
+//     p = fma(q, wh, c)          q * wh + c rounded once.
+//   Let omega be the double nearest to n / D, D <= 1000 (every constant of up to three decimals; 1.9 =
+//   19 / 10).  q n / D keeps a distance of at least 1 / (2 D) of a place from every midpoint of
+//   two floats that it does not equal, far more than the error of c, so p and float(double(q) *
+//   omega) are the same neighbour there.  Midpoints it does equal are common (for 1.9 one q in
+//   ten): q n / D - q wh is then a multiple of the last place of q * wh and smaller than 2^24 of
+//   them, so c is exactly that number, the FMA meets the exact midpoint and rounds to even, as the
+//   conversion does provided that the double product is the midpoint itself.  It is when omega's
+//   own error is below half a last place of every product: |omega - n / D| < m 2^(e - 54), omega
+//   = m 2^e with m in [1, 2) (omega_split checks this).
+//   An omega without such n / D has midpoints only by chance: there p is taken where the results
+//   with c enlarged and diminished by 2^-21 c agree (Ziv's rounding test; they disagree about
+//   once in 2^20 cells), else the FP64 product.
+//
+// A cell whose |x| is below 2^-96 but not zero (underflow would void the argument; in a fresh
+// simulation the passes spread such values, subnormal ones among them, ahead of the first smoke)
+// takes the same steps on x * 2^64 and scales the result back, exact where it is normal (pt_scaled).
+// Results below 2^-125 lie on the grid of 2^-149: quotient and product are rounded to whole numbers
+// of it, each from an estimate corrected by its exact remainder (pt_grid).  What is left (values that
+// are not finite, a failed rounding test) takes FP64: the quotient corrected once by its exact
+// remainder and rounded (a float or a midpoint that x / d equals is then exact, the others are far
+// away), and the double product itself.  Zeros keep their sign: zl has the sign of zh, wl1 and wl2
+// that of wh.
 #pragma once
+#include <math.h>
 #include <stdint.h>
-#include <string.h>
-
-#include <cmath>
 
 #include "kernels.h"
 
 namespace smk {
 
-__host__ __device__ __forceinline__ uint32_t es_funnel_r(uint32_t lo, uint32_t hi, int s) {
-#ifdef __CUDA_ARCH__
-    return __funnelshift_r(lo, hi, (unsigned)s);
-#else
-    return (uint32_t)((((uint64_t)hi << 32) | lo) >> s);
-#endif
-}
+constexpr float ES_TINY = 0x1p-96f, ES_HUGE = 0x1p120f;
 
-__host__ __device__ __forceinline__ float es_bits(uint32_t u) {
-#ifdef __CUDA_ARCH__
-    return __uint_as_float(u);
-#else
-    float f;
-    memcpy(&f, &u, 4);
-    return f;
-#endif
-}
-
-__host__ __device__ __forceinline__ int es_clz(uint32_t v) {
-#ifdef __CUDA_ARCH__
-    return __clz(v);
-#else
-    return __builtin_clz(v);
-#endif
-}
-
-__host__ __device__ __forceinline__ uint32_t es_uint(float f) {
-#ifdef __CUDA_ARCH__
-    return __float_as_uint(f);
-#else
-    uint32_t u;
-    memcpy(&u, &f, 4);
-    return u;
-#endif
-}
-
-// The operands outside the fast paths' range, out of line (a device call the compiler cannot
-// evaluate for every lane and select).
-#ifdef __CUDA_ARCH__
-__device__ __noinline__ float es_scale_slow(float q, double omega) { return __double2float_rn((double)q * omega); }
-__device__ __noinline__ float es_div_slow(float x, float d) { return x / d; }
-#else
-inline float es_scale_slow(float q, double omega) { return (float)((double)q * omega); }
-inline float es_div_slow(float x, float d) { return x / d; }
-#endif
-
-// The significand product of omega_scale: mq (24 bits, leading bit 23) times omega's 53-bit
-// significand, P = w2:w1:w0 in [2^75, 2^77); t24 = its leading 24 bits, rh = the next 29 bits
-// rounded (ties to even) on the rest, so that t24 * 2^29 + rh is P rounded to 53 bits; big = 1
-// when P has 77 bits.
-struct EsProduct {
-    uint32_t t24, rh;
-    int big;
+// zh, zl of the divisor d = 1..6 (host: the table of a kernel is filled from these).
+struct DivSplit {
+    float zh, zl;
 };
 
-__host__ __device__ __forceinline__ EsProduct es_product(uint32_t mq, uint32_t mo_hi, uint32_t mo_lo) {
-    const uint64_t A = (uint64_t)mq * mo_lo;  // < 2^56
-    const uint64_t B = (uint64_t)mq * mo_hi;  // < 2^45
-    const uint32_t w0 = (uint32_t)A;
-    const uint64_t mid = (A >> 32) + (uint32_t)B;
-    const uint32_t w1 = (uint32_t)mid;
-    const uint32_t w2 = (uint32_t)(B >> 32) + (uint32_t)(mid >> 32);
-    EsProduct r;
-    r.big = w2 >= (1u << 12) ? 1 : 0;                                  // P has 76 + big bits
-    r.t24 = es_funnel_r(w1, w2, 20 + r.big);                           // P >> (52 + big): 24 bits
-    r.rh = es_funnel_r(w0, w1, 23 + r.big) & 0x1fffffffu;              // the next 29 bits
-    const uint32_t fr = w0 << (9 - r.big);                             // the lowest 23 + big, left-aligned
-    r.rh += (fr > 0x80000000u || (fr == 0x80000000u && (r.rh & 1u))) ? 1u : 0u;  // to 53 bits
-    return r;
-}
-
-// omega_scale for the operands whose result can fall below the normal float range (biased
-// exponent E < emin, subnormal q included; q != 0 and omega_split gave a valid split).  The
-// result's biased exponent is Eb = Eq + eo + big (Eq = E, or 1 - shift for a subnormal q whose
-// significand was shifted left to bit 23); below 1 the 53-bit value V * 2^(Eb - 179),
-// V = t24 * 2^29 + rh, is rounded to a multiple of 2^-149 as the conversion of the double does.
-__host__ __device__ __forceinline__ float omega_scale_tiny(uint32_t bits, uint32_t mo_hi, uint32_t mo_lo, int eo,
-                                                           uint32_t osign) {
-    const uint32_t E = (bits >> 23) & 0xffu;
-    const uint32_t sign = (bits ^ (osign << 31)) & 0x80000000u;
-    const uint32_t mant = bits & 0x7fffffu;
-    int Eq = (int)E;
-    uint32_t mq = mant | 0x800000u;
-    if (E == 0) {
-        const int sh = es_clz(mant) - 8;  // mant != 0: its leading bit moves to bit 23
-        mq = mant << sh;
-        Eq = 1 - sh;
+__host__ __device__ __forceinline__ DivSplit div_split(int d) {
+    // 1/d rounded toward zero to 24 bits, and the rest: 1/3 = 0xAAAAAA * 2^-25 + ..., 1/5 =
+    // 0xCCCCCC * 2^-26 + ..., 1/6 = 0xAAAAAA * 2^-26 + ...; the rest of 1/d after n/2^k is
+    // (2^k - n d) / (d 2^k), here (2/3) 2^-25, (4/5) 2^-26 and (2/3) 2^-26
+    DivSplit s;
+    switch (d) {
+        case 1: s.zh = 1.0f; s.zl = 0.0f; break;
+        case 2: s.zh = 0.5f; s.zl = 0.0f; break;
+        case 3: s.zh = 11184810.0f * 0x1p-25f; s.zl = (2.0f / 3.0f) * 0x1p-25f; break;
+        case 4: s.zh = 0.25f; s.zl = 0.0f; break;
+        case 5: s.zh = 13421772.0f * 0x1p-26f; s.zl = (4.0f / 5.0f) * 0x1p-26f; break;
+        default: s.zh = 11184810.0f * 0x1p-26f; s.zl = (2.0f / 3.0f) * 0x1p-26f; break;
     }
-    EsProduct p = es_product(mq, mo_hi, mo_lo);
-    const int Eb = Eq + eo + p.big;
-    if (Eb >= 1) {
-        p.t24 += (p.rh > 0x10000000u || (p.rh == 0x10000000u && (p.t24 & 1u))) ? 1u : 0u;
-        return es_bits(sign + ((uint32_t)(Eb - 1) << 23) + p.t24);
+    return s;
+}
+
+// Whether x / d and its product need the FP64 path (a value that is not finite does too).
+__host__ __device__ __forceinline__ bool es_rare(float x) {
+    const float a = fabsf(x);
+    return !(a >= ES_TINY && a <= ES_HUGE) && a != 0.0f;
+}
+
+__host__ __device__ __forceinline__ float div_fast(float x, float zh, float zl) { return fmaf(x, zh, x * zl); }
+
+__host__ __device__ __forceinline__ float scale_rest(float q, const OmegaSplit& s) { return fmaf(q, s.wl1, q * s.wl2); }
+// Ziv's test of the product for an omega that is no n / D.
+__host__ __device__ __forceinline__ bool scale_sure(float q, float c, const OmegaSplit& s) {
+    return fmaf(q, s.wh, c * (1.0f + 0x1p-21f)) == fmaf(q, s.wh, c * (1.0f - 0x1p-21f));
+}
+
+// x / d rounded to float, through FP64, for any x; d = 1..6 and r = RN(1/d) in double.
+__host__ __device__ __forceinline__ float div_exact(float x, double d, double r) {
+    const double X = (double)x;
+    double y = X * r;
+    if (fabsf(x) <= 3.4028234663852886e38f) y = fma(fma(-y, d, X), r, y);
+    return x == 0.0f ? x : (float)y;
+}
+
+// p_t for 0 < |x| < 2^-96 where the result is normal and safely so; ok says whether it is.
+__host__ __device__ __forceinline__ float pt_scaled(float x, float zh, float zl, const OmegaSplit& s, bool& ok) {
+    const float q = div_fast(x * 0x1p64f, zh, zl);
+    const float c = scale_rest(q, s);
+    const float p = fmaf(q, s.wh, c);
+    ok = fabsf(p) >= 0x1p-61f && fabsf(q) >= 0x1p-61f && (s.rational || scale_sure(q, c, s));
+    return p * 0x1p-64f;
+}
+
+// p_t for 0 < |x| < 2^-118 where quotient and product are below 2^-125 (whole numbers of 2^-149, at most 2^24),
+// omega n / D; d = 1..6.  ok says whether the operands are such.
+__host__ __device__ __forceinline__ float pt_grid(float x, int d, float zh, float zl, const OmegaSplit& s, bool& ok) {
+    const float m = fabsf(x) * 0x1p64f * 0x1p85f;  // |x| = m 2^-149, a whole number
+    ok = s.rational != 0 && m < 0x1p31f;
+    const float mf = ok ? m : 0.0f;
+    // k = m / d to the nearest whole number, ties to even: the estimate is within 1 of it
+    int k = (int)rintf(div_fast(mf, zh, zl));
+    const int rem = 2 * ((int)mf - k * d);
+    if (rem > d || (rem == d && (k & 1))) k += 1;
+    else if (rem < -d || (rem == -d && (k & 1))) k -= 1;
+    // j = k |omega| to the nearest whole number; in the tie case the remainder is exactly 1/2
+    const float kf = (float)k;
+    const float c = scale_rest(kf, s);
+    const float t = fmaf(kf, s.wh, c);
+    const float e = rintf(t);
+    int j = (int)e;
+    if (fabsf(t) < 0x1p23f) {
+        const float r = fmaf(kf, s.wh, -e) + c;
+        if (r > 0.5f || (r == 0.5f && (j & 1))) j += 1;
+        else if (r < -0.5f || (r == -0.5f && (j & 1))) j -= 1;
     }
-    const uint64_t V = ((uint64_t)p.t24 << 29) + p.rh;  // <= 2^53
-    const int sh = 30 - Eb;                              // the value in units of 2^-149 is V / 2^sh
-    if (sh >= 55) return es_bits(sign);                  // below half of 2^-149 (V / 2^55 < 1/4)
-    uint64_t qv = V >> sh;
-    const uint64_t rem = V & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-    qv += (rem > half || (rem == half && (qv & 1u))) ? 1u : 0u;
-    return es_bits(sign | (uint32_t)qv);  // qv <= 2^23: a subnormal, or the smallest normal
+    ok = ok && k <= (1 << 24) && j <= (1 << 24) && j >= -(1 << 24);
+    const float p = (float)(j < 0 ? -j : j) * 0x1p-85f * 0x1p-64f;  // exact
+    return (x < 0.0f) != (s.wh < 0.0f) ? -p : p;
 }
 
-// float(double(q) * omega) with omega split by omega_split (kernels_vsweep_tb.cu).
-__host__ __device__ __forceinline__ float omega_scale(float q, const OmegaSplit& s, double omega) {
-    const uint32_t bits = es_uint(q);
-    const uint32_t E = (bits >> 23) & 0xffu;
-    const uint32_t sign = (bits ^ (s.sign << 31)) & 0x80000000u;
-    if ((bits << 1) == 0u) return es_bits(sign);
-    if ((uint32_t)((int)E - s.emin) > (uint32_t)(s.emax - s.emin)) {
-        if ((int)E < s.emin && s.emin <= s.emax) return omega_scale_tiny(bits, s.mo_hi, s.mo_lo, s.eo, s.sign);
-        return es_scale_slow(q, omega);
-    }
-    EsProduct p = es_product((bits & 0x7fffffu) | 0x800000u, s.mo_hi, s.mo_lo);
-    p.t24 += (p.rh > 0x10000000u || (p.rh == 0x10000000u && (p.t24 & 1u))) ? 1u : 0u;  // to 24 bits
-    // value = t24 * 2^((E - 127) + eo + big - 23); adding t24 (implicit bit included) to the
-    // exponent field one below carries into it correctly, also when t24 rounded up to 2^24
-    return es_bits(sign + ((uint32_t)((int)E + s.eo + p.big - 1) << 23) + p.t24);
-}
-
-// x / d for 0 < |x| < 2^-100, d = 1..6 given as the float df, r = RN(1/d).  x * 2^64 is exact
-// and inside the corrected multiply's range; the quotient ys scales back exactly when it is at
-// least 2^-62 (the result is normal).  Below, |x / d| < 2^-126 and |x| < 6 * 2^-126, so
-// x = m * 2^-149 with m < 2^26, and the result is RN(m / d) * 2^-149 (<= 2^-126).
-__host__ __device__ __forceinline__ float div_tiny(float x, float df, float r) {
-    const float xs = x * 0x1p64f;
-    const float y = xs * r;
-    const float e = fmaf(-y, df, xs);
-    const float ys = fmaf(e, r, y);
-    if (fabsf(ys) >= 0x1p-62f) return ys * 0x1p-64f;
-    const uint32_t bits = es_uint(x);
-    const uint32_t E = (bits >> 23) & 0xffu;
-    const uint32_t mant = bits & 0x7fffffu;
-    const uint32_t m = E == 0 ? mant : ((mant | 0x800000u) << (E - 1));
-    const uint32_t d = (uint32_t)df;
-    uint32_t qi = m / d;
-    const uint32_t rem = m - qi * d;
-    qi += (2u * rem > d || (2u * rem == d && (qi & 1u))) ? 1u : 0u;
-    return es_bits((bits & 0x80000000u) | qi);
-}
-
-// x / d, d = 1..6 given as the float df, r = RN(1/d).
-__host__ __device__ __forceinline__ float div_small(float x, float df, float r) {
-    const float ax = fabsf(x);
-    if (ax == 0.0f) return x;
-    if (ax < 0x1p-100f) return div_tiny(x, df, r);
-    if (!(ax < 0x1p100f)) return es_div_slow(x, df);
-    const float y = x * r;
-    const float e = fmaf(-y, df, x);
-    return fmaf(e, r, y);
-}
-
-// float(double(x / d) * omega) for a cell update, without branches on the common operands:
-// the corrected multiply and the integer product run for every lane, and a select gives zeros
-// (signed as the quotient and product of a zero are).  `rare` is set for the operands that need
-// the full functions (|x| below 2^-100 or not below 2^100, a quotient outside the integer
-// product's exponent range): the caller then takes div_scale_full, so that a warp diverges only
-// where one of its lanes has such an operand.
-__host__ __device__ __forceinline__ float div_scale_fast(float x, float df, float r, const OmegaSplit& s,
-                                                        bool& rare) {
-    const float ax = fabsf(x);
-    const float y = x * r;
-    const float e = fmaf(-y, df, x);
-    float q = fmaf(e, r, y);
-    q = ax == 0.0f ? x : q;
-    const uint32_t bits = es_uint(q);
-    const uint32_t E = (bits >> 23) & 0xffu;
-    const uint32_t sign = (bits ^ (s.sign << 31)) & 0x80000000u;
-    EsProduct p = es_product((bits & 0x7fffffu) | 0x800000u, s.mo_hi, s.mo_lo);
-    p.t24 += (p.rh > 0x10000000u || (p.rh == 0x10000000u && (p.t24 & 1u))) ? 1u : 0u;
-    const uint32_t pt = sign + ((uint32_t)((int)E + s.eo + p.big - 1) << 23) + p.t24;
-    const bool zero = ax == 0.0f;
-    rare = !zero && (!(ax >= 0x1p-100f && ax < 0x1p100f) ||
-                     (uint32_t)((int)E - s.emin) > (uint32_t)(s.emax - s.emin));
-    return es_bits(zero ? sign : pt);
-}
-
-// The same value through the full functions (every operand), out of line on the device.  The
-// split is passed as scalars: the call then needs no stack frame.
-__host__ __device__ __forceinline__ float div_scale_full(float x, float df, float r, uint32_t mo_hi, uint32_t mo_lo, int eo, uint32_t osign, int emin,
-                     int emax, double omega) {
-    OmegaSplit s;
-    s.mo_hi = mo_hi;
-    s.mo_lo = mo_lo;
-    s.eo = eo;
-    s.sign = osign;
-    s.emin = emin;
-    s.emax = emax;
-    return omega_scale(div_small(x, df, r), s, omega);
-}
+__host__ __device__ __forceinline__ float scale_exact(float q, double omega) { return (float)((double)q * omega); }
 
 }  // namespace smk

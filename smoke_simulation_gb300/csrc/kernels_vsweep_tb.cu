@@ -32,19 +32,31 @@
 // cross-thread update reads the sender's projectable bit from the flag boxes when it loads the
 // plane (left neighbour: a shuffle of the flag word; row above: the shared-memory flag box).
 //
-// Halo, windows, z-chunks and the TMA ring with bounded mbarrier waits are those of the pressure
-// form (tb_common.cuh); positions that no pass changes (the boundary ring and everything outside
-// the grid) make windows that reach the grid's edge need no halo there.  A launch reads u, v, w
-// and the flags and writes u, v, w to a second set of face arrays (the simulation's pressure and
-// rhs buffers, unused by this scheme): 25 bytes per position for T/2 iterations.
+// Halo, windows and the TMA ring with bounded mbarrier waits are those of the pressure form
+// (tb_common.cuh); positions that no pass changes (the boundary ring and everything outside the grid)
+// make windows that reach the grid's edge need no halo there.  A launch reads u, v, w and the flags and
+// writes u, v, w to a second set of face arrays (the simulation's pressure and rhs buffers, unused by
+// this scheme): 25 bytes per position for T/2 iterations.
 //
-// p_t = float(double(-div / acc) * omega) is evaluated exactly without the FP64 pipe, which bounds
-// the one-pass kernel on GB300 (exact_scale.cuh: the quotient by the small integer acc with one
-// FMA correction, the double product with integer arithmetic).
+// Arithmetic.  p_t = float(double(-div / acc) * omega) costs five FP32 multiplies and FMAs
+// (exact_scale.cuh); a face update is one predicated add; the divergence and the product of a
+// thread's two cells are packed FP32 pairs.  Operands that need more go through cell_pt_rare, out of
+// line so that its code stays out of the unrolled march (inlined, instruction fetches made a launch
+// 15 % slower).
+//
+// What bounds it: instruction issue (256^3, T = 4, z-chunk 52: 171 us a launch, 61 % of the issue
+// slots busy over two uneven waves, 70 % while active; ~120 warp instructions per two cells and pass, halo included;
+// HBM at 32 %).  256^3, 30 iterations: one pass per launch 5.20 ms (86.7 us a pass, 0.73 of the
+// measured HBM bandwidth and 48 % of the FP64 pipe), T = 4 2.60 ms, T = 2 3.1 ms.  The former form
+// (integer 24 x 53-bit product, both corrections and the FP64 path evaluated for every cell) took
+// 9.8 ms with T = 4.  Not kept: multipliers 0 / 1 per face from a shared table instead of predicated
+// adds (L1 at 72 %, 3.5 ms); passes left out for warps outside a pass's cone (3.8 ms: the branches
+// stop the compiler from interleaving the passes).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -58,9 +70,9 @@ namespace {
 
 using namespace tb;
 
-// Tile geometry: TY warps (tile rows of threads) of 2-row patches, ROWS = 2 TY face-grid rows.
-// TY = 16: one CTA of 16 warps per SM (T = 4 needs ~120 registers a thread); TY = 12: two CTAs
-// of 12 warps per SM (T = 2 within 80 registers), more warps to hide the update chains' latency.
+// Tile geometry: TY warps (tile rows of threads) of 2-row patches, ROWS = 2 TY face-grid rows, one CTA
+// per SM.  T = 4 holds six planes of three fields in registers (128 a thread: 16 warps); T = 2 holds four
+// (80: 24 warps, whose 48-row tile keeps 0.86 of its cells as owned instead of 0.78 with 24 rows).
 template <int TY>
 struct VTGeom {
     static constexpr int ROWS = 2 * TY;
@@ -79,56 +91,91 @@ struct VMaps {
 
 // ---- one pass on one cell ----------------------------------------------------------------------
 
-__device__ __forceinline__ float fsel(unsigned f, unsigned bit) { return (f & bit) ? 1.0f : 0.0f; }
-
-// Per neighbour pattern (the flag byte's six neighbour bits, e = (f >> 1) & 63): the divisor acc
-// (>= 1, so a non-projectable cell's quotient stays finite) as a float, RN(1/acc), and the six 0/1
-// face multipliers s(x-1), s(y-1), s(z-1) | s(x+1), s(y+1), s(z+1), from a shared table
-// (two 16-byte reads instead of a population count, a conversion and six selects per update).
-struct CellCoef {
-    float4 a;  // acc, RN(1/acc), s(x-1), s(y-1)
-    float4 b;  // s(z-1), s(x+1), s(y+1), s(z+1)
-};
-
-__device__ __forceinline__ CellCoef make_coef(int e) {
-    const int acc = max(__popc((unsigned)e), 1);
-    CellCoef c;
-    c.a = make_float4((float)acc, 1.0f / (float)acc, (e & 1) ? 1.f : 0.f, (e & 4) ? 1.f : 0.f);
-    c.b = make_float4((e & 16) ? 1.f : 0.f, (e & 2) ? 1.f : 0.f, (e & 8) ? 1.f : 0.f, (e & 32) ? 1.f : 0.f);
-    return c;
-}
-
-// p_t of a cell from its six faces; 0 for a cell that is not projectable (every use of p_t is
-// predicated on the projectable bit).
-__device__ __forceinline__ float cell_pt(unsigned f, const CellCoef& c, float uc, float ux, float vc, float vy,
-                                         float wc, float wz, const OmegaSplit& os, double omega) {
-    const float div = -uc + ux + -vc + vy + -wc + wz;
-    bool rare;
-    float pt = div_scale_fast(-div, c.a.x, c.a.y, os, rare);
-    if (rare) pt = div_scale_full(-div, c.a.x, c.a.y, os.mo_hi, os.mo_lo, os.eo, os.sign, os.emin, os.emax, omega);
-    return (f & F_PROJ) ? pt : 0.0f;
-}
-
-// Own (lower) faces of an updated cell: u_x -= p_t*s(x-1), v_y -= p_t*s(y-1), w_z -= p_t*s(z-1).
-__device__ __forceinline__ void own_faces(unsigned f, const CellCoef& c, float pt, float& u, float& v, float& w) {
-    if (f & F_PROJ) {
-        u = u - pt * c.a.z;
-        v = v - pt * c.a.w;
-        w = w - pt * c.b.x;
-    }
-}
-
-// Predicate bits of the faces a plane's patch receives from cells held by another thread.
+// A cell's ring entry is 16 bits, the byte offset of its quotient's zh, zl (exact_scale.cuh) in a
+// shared table with one copy per lane: (f >> 1 & 127) * 256 + lane * 8 for the flag byte f, so that
+// a warp's 8-byte reads never meet in a bank whatever its flag bytes are.  The neighbour bits and the
+// projectable bit are tested in place:
 enum : unsigned {
-    G_XA0 = 1u,  // A0's left neighbour (lane - 1's B0) is projectable
-    G_XA1 = 2u,  // A1's left neighbour (lane - 1's B1)
-    G_YA0 = 4u,  // A0's neighbour at y - 1 (the thread above's A1, or the row above the tile)
-    G_YB0 = 8u,  // B0's neighbour at y - 1
+    C_XM = 1u << 8, C_XP = 1u << 9, C_YM = 1u << 10, C_YP = 1u << 11, C_ZM = 1u << 12, C_ZP = 1u << 13,
+    C_PROJ = 1u << 14,
 };
+constexpr int COEF_BYTES = 128 * 256;
 
-__device__ __forceinline__ unsigned fbyte(unsigned f, int k) { return (f >> (8 * k)) & 0xffu; }
+__device__ __forceinline__ unsigned cell_entry(unsigned f, unsigned lane8) { return ((f & 0xfeu) << 7) | lane8; }
+
+// Faces of an updated cell.  The reference adds p_t * s with s = 0 or 1; a face with s = 1 (open)
+// takes one predicated add.  With s = 0 the product is a zero, which changes nothing but a face
+// that holds -0 (-0 + +0 = +0): closed faces are visited only by warps that hold a -0 somewhere
+// (`neg0`; no update makes one from other values).  pl is p_t, or +0 on a cell that is not
+// projectable, pu the same with -0: u - +0 and u + -0 leave every u as it is.
+__device__ __forceinline__ void face_lower(unsigned c, unsigned bit, float pl, float& u) {
+    if (c & bit) u = u - pl;
+}
+__device__ __forceinline__ void face_upper(unsigned c, unsigned bit, float pu, float& u) {
+    if (c & bit) u = u + pu;
+}
+__device__ __forceinline__ void closed_lower(unsigned c, unsigned bit, float p, float& u) {
+    if ((c & (bit | C_PROJ)) == C_PROJ) u = u - p * 0.0f;
+}
+__device__ __forceinline__ void closed_upper(unsigned c, unsigned bit, float p, float& u) {
+    if ((c & (bit | C_PROJ)) == C_PROJ) u = u + p * 0.0f;
+}
+// What an upper face held by another thread receives: p_t * s, or -0 from a cell that is not projectable.
+__device__ __forceinline__ float face_sent(unsigned c, unsigned bit, float pu) { return (c & bit) ? pu : pu * 0.0f; }
+
+// A cell that the common path does not decide (es_rare, or the rounding test): zh, zl as in its table
+// entry, pt the common path's value, kept where `rare` is not set.  pt_scaled, pt_grid, then FP64
+// (exact_scale.cuh; zh + zl stands for 1/acc, whose 2^-48 the correction by the exact remainder makes up
+// for).  The FP64 part is one block of PTX: as plain code the compiler evaluates it for every lane
+// and selects, which puts the FP64 instructions on every cell.
+__device__ __noinline__ float cell_pt_rare(float pt, bool rare, float x, unsigned ofs, float zh, float zl,
+                                             const OmegaSplit& os, double omega) {
+    rare = rare && (ofs & C_PROJ);
+    const int acc = max(__popc((ofs >> 8) & 63u), 1);
+    bool ok;
+    const bool tiny = rare && fabsf(x) < ES_TINY;
+    const float ps = pt_scaled(x, zh, zl, os, ok);
+    if (tiny && ok) pt = ps;
+    rare = rare && !(tiny && ok);
+    if (!__any_sync(0xffffffffu, rare)) return pt;
+    const float pg = pt_grid(x, acc, zh, zl, os, ok);
+    if (rare && ok) pt = pg;
+    const bool left = rare && !ok;
+    if (!__any_sync(0xffffffffu, left)) return pt;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred mine, fin;\n\t"
+        ".reg .f32 ax, r;\n\t"
+        ".reg .f64 X, d, i, y, c, e;\n\t"
+        "setp.ne.u32 mine, %1, 0;\n\t"
+        "cvt.rn.f64.u32 d, %3;\n\t"
+        "cvt.f64.f32 i, %5;\n\t"
+        "cvt.f64.f32 e, %6;\n\t"
+        "add.rn.f64 i, i, e;\n\t"
+        "cvt.f64.f32 X, %2;\n\t"
+        "mul.rn.f64 y, X, i;\n\t"
+        "neg.f64 c, y;\n\t"
+        "fma.rn.f64 e, c, d, X;\n\t"
+        "fma.rn.f64 c, e, i, y;\n\t"
+        "abs.f32 ax, %2;\n\t"
+        "setp.lt.f32 fin, ax, 0f7f800000;\n\t"
+        "selp.f64 y, c, y, fin;\n\t"
+        "cvt.rn.f32.f64 r, y;\n\t"
+        "cvt.f64.f32 y, r;\n\t"
+        "mul.rn.f64 y, y, %4;\n\t"
+        "cvt.rn.f32.f64 r, y;\n\t"
+        "selp.f32 %0, r, %0, mine;\n\t"
+        "}"
+        : "+f"(pt)
+        : "r"((unsigned)left), "f"(x), "r"(acc), "d"(omega), "f"(zh), "f"(zl));
+    return pt;
+}
 
 // One tile of a launch: T colour passes (nhalf of them when not FULL) starting at colour0.
+//
+// A thread's 2 x 2 patch is held as two pairs per field, E = (A0, B1) and O = (B0, A1): one
+// pattern updates the cells of E, the other those of O, and the divergence and the product of both
+// cells are packed FP32 pairs (one issue slot for two cells).
 template <int T, int TY, bool FULL>
 __device__ __forceinline__ void vsweep_tile(const VMaps& maps, const Grid& g, float* __restrict__ uo,
                                             float* __restrict__ vo, float* __restrict__ wo, int nhalf,
@@ -143,17 +190,22 @@ __device__ __forceinline__ void vsweep_tile(const VMaps& maps, const Grid& g, fl
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* stages = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     float* pub = reinterpret_cast<float*>(stages + S * VT_STAGE);
+    unsigned char* ctab = reinterpret_cast<unsigned char*>(pub + 2 * NPUB * VT_PROW);
     __shared__ __align__(8) uint64_t mbar[S];
-    __shared__ CellCoef ctab[64];  // per neighbour pattern (make_coef)
 
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int tid = ty * TX + tx;
     const bool leader = tid == 0;
-    if (tid < 64) ctab[tid] = make_coef(tid);
-    // zero the padding rows of every published plane (never written afterwards)
+    for (int i = tid; i < 128 * TX; i += VT_THREADS) {
+        const int acc = __popc((unsigned)((i / TX) & 63));
+        const DivSplit z = div_split(acc < 1 ? 1 : acc);
+        reinterpret_cast<float2*>(ctab)[i] = make_float2(z.zh, z.zl);
+    }
+    // the padding rows of every published plane (never written afterwards): nothing received from
+    // above the tile (adding -0 leaves a face as it is), and any value below it
     for (int i = tid; i < 2 * NPUB * 2 * TX; i += VT_THREADS) {
         const int lane = i % TX, edge = (i / TX) % 2, set = i / (2 * TX);
-        pub[set * VT_PROW + (edge ? (TY + 1) * TX : 0) + lane] = 0.0f;
+        pub[set * VT_PROW + (edge ? (TY + 1) * TX : 0) + lane] = -0.0f;
     }
 
     // windows over the face grid: (nx+1) x (ny+1) positions, planes 0..nz
@@ -175,16 +227,14 @@ __device__ __forceinline__ void vsweep_tile(const VMaps& maps, const Grid& g, fl
     const int off0 = x0 + g.X * y0;
 
     // a plane q is finished at iteration q + 1 + T; planes below 0 are never changed and the
-    // zero-initialised ring stands for them, so a chunk near z = 0 may start at plane 0 where that
-    // saves a pass of the unrolled loop
+    // zero-initialised ring stands for them, so a chunk near z = 0 starts at plane 0
     const int qend = zb + T;
-    int qbeg = (za - T < 0 && (qend + R) / R < (qend - (za - T) + R) / R) ? 0 : za - T;
+    int qbeg = za - T < 0 ? 0 : za - T;
     // start one plane lower where needed so that iteration k of every unrolled pass has the
     // update pattern of k's parity (fixed at compile time: one pattern's code per iteration); the
     // extra plane is one more halo plane (zero-filled below plane 0)
     qbeg -= (qbeg + colour0 - 1) & 1;
-    const int nouter = (qend - qbeg + R) / R;
-    const int qfinal = qbeg + nouter * R - 1;
+    const int qfinal = qend;  // last iteration executed
 
     auto issue = [&](int s, int z) {
         unsigned char* st = stages + s * VT_STAGE;
@@ -199,63 +249,68 @@ __device__ __forceinline__ void vsweep_tile(const VMaps& maps, const Grid& g, fl
         for (int s = 0; s < S; ++s) mbar_init(smem_u32(&mbar[s]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        for (int s = 0; s < S; ++s) issue(s, qbeg + s);
+        for (int s = 0; s < S && qbeg + s <= qfinal; ++s) issue(s, qbeg + s);
     }
 
-    float2 U[2][R], V[2][R], W[2][R];  // per patch row (x = column A, y = column B), slot = plane mod R
-    unsigned ff[R], gg[R];               // flag bytes A0, B0, A1, B1 and the G_* predicate bits
+    // slot = plane mod R; [0] = E = (A0, B1), [1] = O = (B0, A1)
+    float2 U[2][R], V[2][R], W[2][R];
+    unsigned ff[2][R];  // the pair's entries (cell_entry), the first cell's in the low half
+    const unsigned lane8 = (unsigned)tx * 8u;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
 #pragma unroll
-        for (int r = 0; r < 2; ++r) U[r][j] = V[r][j] = W[r][j] = make_float2(0.f, 0.f);
-        ff[j] = gg[j] = 0u;
+        for (int e = 0; e < 2; ++e) {
+            U[e][j] = V[e][j] = W[e][j] = make_float2(0.f, 0.f);
+            ff[e][j] = lane8 | (lane8 << 16);
+        }
     }
     const int me0 = (ty + 1) * TX + tx;
+    const float2 wh = make_float2(os.wh, os.wh), wl1 = make_float2(os.wl1, os.wl1), wl2 = make_float2(os.wl2, os.wl2);
     int par = 0;
+    int neg0 = 0;  // iterations until the last plane with a -0 in this warp has left the ring
     __syncthreads();  // barriers initialised, table and padding visible
 
     for (int base = qbeg; base <= qend; base += R) {
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const int q = base + k;
+            if (q > qend) break;
             const int st = k % S;
             const uint32_t phase = (uint32_t)((k / S) & 1);
-            // updated cells of every stage of this iteration: A0 and B1 (sA), else B0 and A1; the
-            // pattern follows (q + colour0 - 1), which qbeg's choice makes k's parity
-            const bool sA = (k & 1) == 0;
+            // the pair every stage of this iteration updates: E on even k, O on odd k (qbeg)
+            const int e = k & 1;
             float* cur = pub + par * NPUB * VT_PROW;              // written this iteration
             const float* prv = pub + (par ^ 1) * NPUB * VT_PROW;  // written by the last one
 
-            // ---- plane q into slot k, with the predicates of the faces it receives
+            // ---- plane q into slot k
             const bool ok = mbar_wait(smem_u32(&mbar[st]), phase);
             {
                 const unsigned char* S_ = stages + st * VT_STAGE;
-                const float* su = reinterpret_cast<const float*>(S_);
-                const float* sv = reinterpret_cast<const float*>(S_ + VT_BOX_F);
-                const float* sw = reinterpret_cast<const float*>(S_ + 2 * VT_BOX_F);
-                const unsigned char* sf = S_ + 3 * VT_BOX_F;
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    const int rr = (2 * ty + r) * BOX_F + of;
-                    U[r][k] = *reinterpret_cast<const float2*>(su + rr);
-                    V[r][k] = *reinterpret_cast<const float2*>(sv + rr);
-                    W[r][k] = *reinterpret_cast<const float2*>(sw + rr);
-                }
-                const unsigned f0 = *reinterpret_cast<const unsigned short*>(sf + (2 * ty) * BOX_U8 + ob);
-                const unsigned f1 = *reinterpret_cast<const unsigned short*>(sf + (2 * ty + 1) * BOX_U8 + ob);
-                const unsigned f = f0 | (f1 << 16);
-                ff[k] = f;
-                const unsigned fl = __shfl_up_sync(0xffffffffu, f, 1);  // lane - 1's A0, B0, A1, B1
-                const unsigned fa = ty > 0 ? *reinterpret_cast<const unsigned short*>(sf + (2 * ty - 1) * BOX_U8 + ob)
-                                           : 0u;  // the row above: A, B
-                unsigned gb = 0u;
-                if (tx > 0) {
-                    if (fbyte(fl, 1) & F_PROJ) gb |= G_XA0;
-                    if (fbyte(fl, 3) & F_PROJ) gb |= G_XA1;
-                }
-                if (fa & F_PROJ) gb |= G_YA0;
-                if ((fa >> 8) & F_PROJ) gb |= G_YB0;
-                gg[k] = gb;
+                const float* sf32 = reinterpret_cast<const float*>(S_) + 2 * ty * BOX_F + of;
+                const unsigned char* sf = S_ + 3 * VT_BOX_F + 2 * ty * BOX_U8 + ob;
+                const float2 u0 = *reinterpret_cast<const float2*>(sf32),
+                             u1 = *reinterpret_cast<const float2*>(sf32 + BOX_F);
+                const float2 v0 = *reinterpret_cast<const float2*>(sf32 + VT_BOX_F / 4),
+                             v1 = *reinterpret_cast<const float2*>(sf32 + VT_BOX_F / 4 + BOX_F);
+                const float2 w0 = *reinterpret_cast<const float2*>(sf32 + 2 * (VT_BOX_F / 4)),
+                             w1 = *reinterpret_cast<const float2*>(sf32 + 2 * (VT_BOX_F / 4) + BOX_F);
+                U[0][k] = make_float2(u0.x, u1.y);
+                U[1][k] = make_float2(u0.y, u1.x);
+                V[0][k] = make_float2(v0.x, v1.y);
+                V[1][k] = make_float2(v0.y, v1.x);
+                W[0][k] = make_float2(w0.x, w1.y);
+                W[1][k] = make_float2(w0.y, w1.x);
+                // a -0 is the least 32-bit integer
+                auto least = [](float2 a, float2 b) {
+                    return min(min(__float_as_int(a.x), __float_as_int(a.y)),
+                               min(__float_as_int(b.x), __float_as_int(b.y)));
+                };
+                const int least_bits = min(min(least(u0, u1), least(v0, v1)), least(w0, w1));
+                if (__any_sync(0xffffffffu, least_bits == (int)0x80000000)) neg0 = T + 2;
+                const unsigned f0 = *reinterpret_cast<const unsigned short*>(sf);           // A0, B0
+                const unsigned f1 = *reinterpret_cast<const unsigned short*>(sf + BOX_U8);  // A1, B1
+                ff[0][k] = cell_entry(f0, lane8) | (cell_entry(f1 >> 8, lane8) << 16);
+                ff[1][k] = cell_entry(f0 >> 8, lane8) | (cell_entry(f1, lane8) << 16);
             }
             if (__syncthreads_or(!ok)) {
                 // a TMA stage never completed: record it, drain what is in flight, stop
@@ -275,103 +330,121 @@ __device__ __forceinline__ void vsweep_tile(const VMaps& maps, const Grid& g, fl
             // "pass 0": the v of this plane's row-0 cell that this iteration's pattern updates, read
             // by the thread above at its first pass on this plane (next iteration).  Written after
             // the barrier: the previous iteration's reads of this buffer are all done.
-            cur[me0] = sA ? V[0][k].x : V[0][k].y;
+            cur[me0] = V[e][k].x;
 
             // ---- passes t = 1..T on plane q - t (slot j), reaching into plane q - t + 1 (slot jn)
 #pragma unroll
             for (int t = 1; t <= T; ++t) {
                 const int j = (k - t + 2 * R) % R;
                 const int jn = (k - t + 1 + 2 * R) % R;
-                const unsigned f = ff[j], gb = gg[j];
-                // the pass before (t - 1, at the previous iteration) changed the v face of this
-                // plane's row-0 cell updated now through the thread above's last-row cell
-                if (t >= 2 && (FULL || t - 1 <= nhalf)) {
-                    const float pa = prv[(2 * (t - 1) + 1) * VT_PROW + me0 - TX];
-                    if (sA) {
-                        if (gb & G_YA0) V[0][j].x = V[0][j].x + pa * fsel(fbyte(f, 0), F_SELF);
-                    } else {
-                        if (gb & G_YB0) V[0][j].y = V[0][j].y + pa * fsel(fbyte(f, 1), F_SELF);
-                    }
-                }
+                // what the thread above's last-row cell added to this plane's row-0 v face in the
+                // pass before (t - 1, at the previous iteration; p_t * s already)
+                if (t >= 2 && (FULL || t - 1 <= nhalf)) V[e][j].x += prv[(2 * (t - 1) + 1) * VT_PROW + me0 - TX];
                 if (!(FULL || t <= nhalf)) continue;
                 // v of the thread below's row-0 cell at the end of the previous pass
                 const float vb = prv[(2 * (t - 1)) * VT_PROW + me0 + TX];
-                if (sA) {
-                    const unsigned fA0 = fbyte(f, 0), fB1 = fbyte(f, 3), fA1 = fbyte(f, 2);
-                    const CellCoef cA0 = ctab[(fA0 >> 1) & 63u], cB1 = ctab[(fB1 >> 1) & 63u];
-                    const float uR = __shfl_down_sync(0xffffffffu, U[1][j].x, 1);  // lane + 1's A1
-                    const float pA0 = cell_pt(fA0, cA0, U[0][j].x, U[0][j].y, V[0][j].x, V[1][j].x, W[0][j].x,
-                                              W[0][jn].x, os, omega);
-                    const float pB1 = cell_pt(fB1, cB1, U[1][j].y, uR, V[1][j].y, vb, W[1][j].y, W[1][jn].y, os,
-                                              omega);
-                    own_faces(fA0, cA0, pA0, U[0][j].x, V[0][j].x, W[0][j].x);
-                    own_faces(fB1, cB1, pB1, U[1][j].y, V[1][j].y, W[1][j].y);
-                    const float pL = __shfl_up_sync(0xffffffffu, pB1, 1);  // lane - 1's B1
-                    if (fA0 & F_PROJ) {
-                        U[0][j].y = U[0][j].y + pA0 * cA0.b.y;    // B0's u
-                        V[1][j].x = V[1][j].x + pA0 * cA0.b.z;    // A1's v
-                        W[0][jn].x = W[0][jn].x + pA0 * cA0.b.w;  // w above A0
-                    }
-                    if (gb & G_XA1) U[1][j].x = U[1][j].x + pL * fsel(fA1, F_SELF);
-                    if (fB1 & F_PROJ) W[1][jn].y = W[1][jn].y + pB1 * cB1.b.w;
-                    cur[(2 * t) * VT_PROW + me0] = V[0][j].x;
-                    cur[(2 * t + 1) * VT_PROW + me0] = pB1;
+                const unsigned o0 = ff[e][j] & 0xffffu, o1 = ff[e][j] >> 16;
+                const float2 z0 = *reinterpret_cast<const float2*>(ctab + o0);
+                const float2 z1 = *reinterpret_cast<const float2*>(ctab + o1);
+                // the upper faces of the two cells.  E: A0's are B0's u, A1's v; B1's the next
+                // lane's A1 u, the thread below's v.  O: B0's are the next lane's A0 u, B1's v; A1's
+                // B1's u, the thread below's v
+                float2 ux, vy;
+                if (e == 0) {
+                    ux = make_float2(U[1][j].x, __shfl_down_sync(0xffffffffu, U[1][j].y, 1));
+                    vy = make_float2(V[1][j].y, vb);
                 } else {
-                    const unsigned fB0 = fbyte(f, 1), fA1 = fbyte(f, 2), fA0 = fbyte(f, 0);
-                    const CellCoef cB0 = ctab[(fB0 >> 1) & 63u], cA1 = ctab[(fA1 >> 1) & 63u];
-                    const float uR = __shfl_down_sync(0xffffffffu, U[0][j].x, 1);  // lane + 1's A0
-                    const float pB0 = cell_pt(fB0, cB0, U[0][j].y, uR, V[0][j].y, V[1][j].y, W[0][j].y, W[0][jn].y,
-                                              os, omega);
-                    const float pA1 = cell_pt(fA1, cA1, U[1][j].x, U[1][j].y, V[1][j].x, vb, W[1][j].x, W[1][jn].x,
-                                              os, omega);
-                    own_faces(fB0, cB0, pB0, U[0][j].y, V[0][j].y, W[0][j].y);
-                    own_faces(fA1, cA1, pA1, U[1][j].x, V[1][j].x, W[1][j].x);
-                    const float pL = __shfl_up_sync(0xffffffffu, pB0, 1);  // lane - 1's B0
-                    if (fB0 & F_PROJ) {
-                        V[1][j].y = V[1][j].y + pB0 * cB0.b.z;    // B1's v
-                        W[0][jn].y = W[0][jn].y + pB0 * cB0.b.w;  // w above B0
-                    }
-                    if (gb & G_XA0) U[0][j].x = U[0][j].x + pL * fsel(fA0, F_SELF);
-                    if (fA1 & F_PROJ) {
-                        U[1][j].y = U[1][j].y + pA1 * cA1.b.y;    // B1's u
-                        W[1][jn].x = W[1][jn].x + pA1 * cA1.b.w;  // w above A1
-                    }
-                    cur[(2 * t) * VT_PROW + me0] = V[0][j].y;
-                    cur[(2 * t + 1) * VT_PROW + me0] = pA1;
+                    ux = make_float2(__shfl_down_sync(0xffffffffu, U[0][j].x, 1), U[0][j].y);
+                    vy = make_float2(V[0][j].y, vb);
                 }
+                // div = -u + ux + -v + vy + -w + wz in the reference's order (a zero's sign
+                // included); a negated term is an exact product with -1 inside an FMA
+                const float2 neg = make_float2(-1.0f, -1.0f);
+                float2 dv = __ffma2_rn(U[e][j], neg, ux);
+                dv = __fadd2_rn(__ffma2_rn(V[e][j], neg, dv), vy);
+                dv = __fadd2_rn(__ffma2_rn(W[e][j], neg, dv), W[e][jn]);
+                const float2 qq = make_float2(div_fast(-dv.x, z0.x, z0.y), div_fast(-dv.y, z1.x, z1.y));
+                const float2 c2 = __ffma2_rn(qq, wl1, __fmul2_rn(qq, wl2));
+                const float2 pp = __ffma2_rn(qq, wh, c2);
+                float p0 = pp.x, p1 = pp.y;
+                bool r0 = es_rare(dv.x), r1 = es_rare(dv.y);
+                if (!os.rational) {
+                    r0 = r0 || !scale_sure(qq.x, c2.x, os);
+                    r1 = r1 || !scale_sure(qq.y, c2.y, os);
+                }
+                if (__any_sync(0xffffffffu, r0 || r1)) {
+                    p0 = cell_pt_rare(p0, r0, -dv.x, o0, z0.x, z0.y, os, omega);
+                    p1 = cell_pt_rare(p1, r1, -dv.y, o1, z1.x, z1.y, os, omega);
+                }
+                const unsigned w = ff[e][j], w1 = w >> 16;
+                const float pl0 = (w & C_PROJ) ? p0 : 0.0f, pl1 = (w1 & C_PROJ) ? p1 : 0.0f;
+                const float pu0 = (w & C_PROJ) ? p0 : -0.0f, pu1 = (w1 & C_PROJ) ? p1 : -0.0f;
+                // own (lower) faces, and the upper w faces (the next plane's)
+                face_lower(w, C_XM, pl0, U[e][j].x);
+                face_lower(w1, C_XM, pl1, U[e][j].y);
+                face_lower(w, C_YM, pl0, V[e][j].x);
+                face_lower(w1, C_YM, pl1, V[e][j].y);
+                face_lower(w, C_ZM, pl0, W[e][j].x);
+                face_lower(w1, C_ZM, pl1, W[e][j].y);
+                face_upper(w, C_ZP, pu0, W[e][jn].x);
+                face_upper(w1, C_ZP, pu1, W[e][jn].y);
+                // upper u and v faces; the ones another thread holds receive their p_t * s from it
+                float m;
+                if (e == 0) {
+                    m = __shfl_up_sync(0xffffffffu, face_sent(w1, C_XP, pu1), 1);  // lane - 1's B1, for A1
+                    face_upper(w, C_XP, pu0, U[1][j].x);
+                    U[1][j].y += tx > 0 ? m : -0.0f;
+                    face_upper(w, C_YP, pu0, V[1][j].y);
+                } else {
+                    m = __shfl_up_sync(0xffffffffu, face_sent(w, C_XP, pu0), 1);  // lane - 1's B0, for A0
+                    U[0][j].x += tx > 0 ? m : -0.0f;
+                    face_upper(w1, C_XP, pu1, U[0][j].y);
+                    face_upper(w, C_YP, pu0, V[0][j].y);
+                }
+                if (neg0 > 0) {
+                    closed_lower(w, C_XM, p0, U[e][j].x);
+                    closed_lower(w1, C_XM, p1, U[e][j].y);
+                    closed_lower(w, C_YM, p0, V[e][j].x);
+                    closed_lower(w1, C_YM, p1, V[e][j].y);
+                    closed_lower(w, C_ZM, p0, W[e][j].x);
+                    closed_lower(w1, C_ZM, p1, W[e][j].y);
+                    closed_upper(w, C_ZP, p0, W[e][jn].x);
+                    closed_upper(w1, C_ZP, p1, W[e][jn].y);
+                    if (e == 0) closed_upper(w, C_XP, p0, U[1][j].x);
+                    else closed_upper(w1, C_XP, p1, U[0][j].y);
+                    closed_upper(w, C_YP, p0, V[e ^ 1][j].y);
+                }
+                cur[(2 * t) * VT_PROW + me0] = V[e][j].x;
+                cur[(2 * t + 1) * VT_PROW + me0] = face_sent(w1, C_YP, pu1);
             }
 
             // ---- plane q - 1 - T: its last update (from the thread above's pass T) and the store
             {
                 const int js = (k - 1 - T + 2 * R) % R;
-                if (FULL) {
-                    const float pa = prv[(2 * T + 1) * VT_PROW + me0 - TX];
-                    const unsigned f = ff[js], gb = gg[js];
-                    if (sA) {
-                        if (gb & G_YA0) V[0][js].x = V[0][js].x + pa * fsel(fbyte(f, 0), F_SELF);
-                    } else {
-                        if (gb & G_YB0) V[0][js].y = V[0][js].y + pa * fsel(fbyte(f, 1), F_SELF);
-                    }
-                }
+                if (FULL) V[e][js].x += prv[(2 * T + 1) * VT_PROW + me0 - TX];
                 const int zo = q - 1 - T;
                 if (zo >= za && zo < zb) {
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        if (!in[r]) continue;
-                        const size_t o = (size_t)off0 + (size_t)r * g.X + (size_t)g.XY * zo;
-                        *reinterpret_cast<float2*>(uo + o) = U[r][js];
-                        *reinterpret_cast<float2*>(vo + o) = V[r][js];
-                        *reinterpret_cast<float2*>(wo + o) = W[r][js];
+                    const size_t at = (size_t)off0 + (size_t)g.XY * zo;
+                    if (in[0]) {
+                        *reinterpret_cast<float2*>(uo + at) = make_float2(U[0][js].x, U[1][js].x);
+                        *reinterpret_cast<float2*>(vo + at) = make_float2(V[0][js].x, V[1][js].x);
+                        *reinterpret_cast<float2*>(wo + at) = make_float2(W[0][js].x, W[1][js].x);
+                    }
+                    if (in[1]) {
+                        *reinterpret_cast<float2*>(uo + at + g.X) = make_float2(U[1][js].y, U[0][js].y);
+                        *reinterpret_cast<float2*>(vo + at + g.X) = make_float2(V[1][js].y, V[0][js].y);
+                        *reinterpret_cast<float2*>(wo + at + g.X) = make_float2(W[1][js].y, W[0][js].y);
                     }
                 }
             }
             par ^= 1;
+            --neg0;
         }
     }
 }
 
 template <int T, int TY, bool FULL>
-__global__ void __launch_bounds__(VTGeom<TY>::THREADS, TY == 16 ? 1 : 2)
+__global__ void __launch_bounds__(VTGeom<TY>::THREADS, 1)
 k_vsweep_tb(const __grid_constant__ VMaps maps, Grid g, float* __restrict__ uo, float* __restrict__ vo,
             float* __restrict__ wo, int nhalf, int colour0, int zchunk, OmegaSplit os, double omega,
             int* __restrict__ kerr) {
@@ -381,62 +454,58 @@ k_vsweep_tb(const __grid_constant__ VMaps maps, Grid g, float* __restrict__ uo, 
 template <int T, int TY>
 constexpr size_t vt_smem_bytes() {
     using G = VTGeom<TY>;
-    return 128 + (size_t)((T + 2) / 2) * G::STAGE + sizeof(float) * 2 * 2 * (T + 1) * G::PROW;
+    return 128 + (size_t)((T + 2) / 2) * G::STAGE + sizeof(float) * 2 * 2 * (T + 1) * G::PROW + COEF_BYTES;
 }
 
-// The tile height used with depth T: 12 warps (two CTAs per SM) for T = 2, 16 for T = 4.
-constexpr int vt_ty(int T) { return T == 2 ? 12 : 16; }
+// The tile height used with depth T.
+constexpr int vt_ty(int T) { return T == 2 ? 24 : 16; }
 
 }  // namespace
 
 OmegaSplit omega_split(double w) {
     OmegaSplit s;
     memset(&s, 0, sizeof(s));
-    uint64_t b;
-    memcpy(&b, &w, 8);
-    const int E = (int)((b >> 52) & 0x7ff);
-    if (E == 0 || E == 0x7ff) {  // zero, subnormal or not finite: every q takes the double product
-        s.emin = 256;
-        s.emax = -1;
+    const double a = std::fabs(w);
+    if (!(a >= 0x1p-20 && a <= 0x1p20)) {  // zero, extreme or not finite: no cell passes the rounding test
+        s.wh = s.wl1 = s.wl2 = NAN;
         return s;
     }
-    const uint64_t m = (b & ((1ull << 52) - 1)) | (1ull << 52);
-    s.mo_hi = (uint32_t)(m >> 32);
-    s.mo_lo = (uint32_t)m;
-    s.eo = E - 1023;
-    s.sign = (uint32_t)(b >> 63);
-    // the integer path keeps biased float exponents whose result stays a normal float: the
-    // result lies in [2^(eq + eo), 2^(eq + eo + 2)], whose exponents must stay in [-126, 127]
-    s.emin = -126 - s.eo + 127;
-    s.emax = 125 - s.eo + 127;
-    if (s.emin < 1) s.emin = 1;
-    if (s.emax > 254) s.emax = 254;
+    s.wh = (float)w;
+    if (std::fabs((double)s.wh) > a) s.wh = std::nextafterf(s.wh, 0.0f);
+    const double wl = w - (double)s.wh;  // exact, at most 29 bits, with the sign of w
+    s.wl1 = (float)wl;  // toward zero: wl2 keeps the sign, so that a zero q keeps its own
+    if (std::fabs((double)s.wl1) > std::fabs(wl)) s.wl1 = std::nextafterf(s.wl1, 0.0f);
+    s.wl2 = (float)(wl - (double)s.wl1);  // exact
+    // the least D with |w - n / D| < m 2^(e - 54): fma(w, D, -n) is D times that error, exactly
+    const double lim = std::ldexp(a, -54);
+    for (int D = 1; D <= 1000 && !s.rational; ++D)
+        if (std::fabs(std::fma(w, (double)D, -std::nearbyint(w * D))) < lim * D) s.rational = 1;
     return s;
 }
 
 struct VSweepMaps {
-    // per box height (0: 32 rows, 1: 24 rows)
+    // per box height (0: 32 rows, 1: 48 rows)
     CUtensorMap su[2][2], sv[2][2], sw[2][2];  // [height][state buffer 0/1]
     CUtensorMap xu[2], xv[2], xw[2];           // the scratch face arrays
     CUtensorMap f[2];                          // neighbour flags
 };
 
 int vsweep_depth_supported(int T) { return T == 2 || T == 4; }
+int vsweep_tile_rows(int T) { return 2 * vt_ty(T); }
 
 int prepare_vsweep_kernels() {
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const bool ok =
-        cudaFuncSetAttribute(k_vsweep_tb<2, 12, true>, a, (int)vt_smem_bytes<2, 12>()) == cudaSuccess &&
-        cudaFuncSetAttribute(k_vsweep_tb<2, 12, false>, a, (int)vt_smem_bytes<2, 12>()) == cudaSuccess &&
-        cudaFuncSetAttribute(k_vsweep_tb<4, 16, true>, a, (int)vt_smem_bytes<4, 16>()) == cudaSuccess &&
-        cudaFuncSetAttribute(k_vsweep_tb<4, 16, false>, a, (int)vt_smem_bytes<4, 16>()) == cudaSuccess;
+        cudaFuncSetAttribute(k_vsweep_tb<2, 24, true>, a, (int)vt_smem_bytes<2, 24>()) == cudaSuccess &&
+        cudaFuncSetAttribute(k_vsweep_tb<2, 24, false>, a, (int)vt_smem_bytes<2, 24>()) == cudaSuccess &&
+        cudaFuncSetAttribute(k_vsweep_tb<4, 16, true>, a, (int)vt_smem_bytes<4, 16>()) == cudaSuccess;
     return ok ? 0 : -1;
 }
 
 VSweepMaps* create_vsweep_maps(const Grid& g, float* const* u, float* const* v, float* const* w, const float* xu,
                                const float* xv, const float* xw, const uint8_t* flags) {
     VSweepMaps* m = new VSweepMaps();
-    const int rows[2] = {VTGeom<16>::ROWS, VTGeom<12>::ROWS};
+    const int rows[2] = {VTGeom<16>::ROWS, VTGeom<24>::ROWS};
     bool ok = true;
     for (int h = 0; h < 2 && ok; ++h) {
         ok = tb::encode_3d(&m->f[h], flags, true, g, rows[h]) && tb::encode_3d(&m->xu[h], xu, false, g, rows[h]) &&
@@ -471,7 +540,10 @@ static int launch_vt(const VSweepMaps* m, const Grid& g, int buf, bool from_stat
                     (unsigned)((g.nz + 1 + zchunk - 1) / zchunk));
     const dim3 block(TX, TY);
     const size_t smem = vt_smem_bytes<T, TY>();
-    if (nhalf == T)
+    if constexpr (T == 4)
+        k_vsweep_tb<T, TY, true><<<grid, block, smem, st>>>(maps, g, uo, vo, wo, nhalf, colour0, zchunk, os, omega,
+                                                            kerr);
+    else if (nhalf == T)
         k_vsweep_tb<T, TY, true><<<grid, block, smem, st>>>(maps, g, uo, vo, wo, nhalf, colour0, zchunk, os, omega,
                                                             kerr);
     else
@@ -483,7 +555,7 @@ static int launch_vt(const VSweepMaps* m, const Grid& g, int buf, bool from_stat
 int launch_vsweep_tb(const VSweepMaps* m, const Grid& g, int buf, bool from_state, float* uo, float* vo, float* wo,
                      int T, int nhalf, int colour0, int zchunk, double omega, const OmegaSplit& os, int* kerr,
                      cudaStream_t st) {
-    if (!vsweep_depth_supported(T) || nhalf < 1 || nhalf > T || zchunk < 1) return -1;
+    if (!vsweep_depth_supported(T) || nhalf < 1 || nhalf > T || (T == 4 && nhalf != 4) || zchunk < 1) return -1;
     if (T == 2) return launch_vt<2>(m, g, buf, from_state, uo, vo, wo, nhalf, colour0, zchunk, omega, os, kerr, st);
     return launch_vt<4>(m, g, buf, from_state, uo, vo, wo, nhalf, colour0, zchunk, omega, os, kerr, st);
 }
@@ -493,15 +565,41 @@ int launch_vsweep_tb(const VSweepMaps* m, const Grid& g, int buf, bool from_stat
 // ---- testing: the exact arithmetic's host instances, compared with the double product and the
 // IEEE quotient by the CPU tests ----------------------------------------------------------------
 
+namespace {
+float host_scale(float q, const smk::OmegaSplit& os, double omega) {
+    const float c = smk::scale_rest(q, os);
+    if (smk::es_rare(q) || (!os.rational && !smk::scale_sure(q, c, os))) return smk::scale_exact(q, omega);
+    return fmaf(q, os.wh, c);
+}
+
+// A cell's p_t as the kernel's common and rare paths give it.
+float host_pt(float x, int d, const smk::OmegaSplit& os, double omega) {
+    const smk::DivSplit z = smk::div_split(d);
+    bool ok = false;
+    if (!smk::es_rare(x)) {
+        const float q = smk::div_fast(x, z.zh, z.zl);
+        const float c = smk::scale_rest(q, os);
+        if (os.rational || smk::scale_sure(q, c, os)) return fmaf(q, os.wh, c);
+    } else if (fabsf(x) < smk::ES_TINY) {
+        float p = smk::pt_scaled(x, z.zh, z.zl, os, ok);
+        if (ok) return p;
+        p = smk::pt_grid(x, d, z.zh, z.zl, os, ok);
+        if (ok) return p;
+    }
+    return smk::scale_exact(smk::div_exact(x, (double)d, 1.0 / d), omega);
+}
+}  // namespace
+
 extern "C" int smk_test_exact_arith(const float* x, const int* d, int n, double omega, float* scaled,
                                     float* quotient) {
     if (!x || n < 0) return 1;
     const smk::OmegaSplit os = smk::omega_split(omega);
     for (int i = 0; i < n; ++i) {
-        if (scaled) scaled[i] = smk::omega_scale(x[i], os, omega);
+        if (scaled) scaled[i] = d ? host_scale(x[i], os, omega) : host_pt(x[i], 1, os, omega);
         if (quotient && d) {
             const int k = d[i] < 1 ? 1 : (d[i] > 6 ? 6 : d[i]);
-            quotient[i] = smk::div_small(x[i], (float)k, 1.0f / (float)k);
+            const smk::DivSplit z = smk::div_split(k);
+            quotient[i] = smk::es_rare(x[i]) ? smk::div_exact(x[i], (double)k, 1.0 / k) : smk::div_fast(x[i], z.zh, z.zl);
         }
     }
     return 0;
@@ -510,13 +608,6 @@ extern "C" int smk_test_exact_arith(const float* x, const int* d, int n, double 
 extern "C" int smk_test_exact_cell(const float* x, const int* d, int n, double omega, float* pt) {
     if (!x || !d || !pt || n < 0) return 1;
     const smk::OmegaSplit os = smk::omega_split(omega);
-    for (int i = 0; i < n; ++i) {
-        const int k = d[i] < 1 ? 1 : (d[i] > 6 ? 6 : d[i]);
-        const float df = (float)k, r = 1.0f / (float)k;
-        bool rare = false;
-        float v = smk::div_scale_fast(x[i], df, r, os, rare);
-        if (rare) v = smk::div_scale_full(x[i], df, r, os.mo_hi, os.mo_lo, os.eo, os.sign, os.emin, os.emax, omega);
-        pt[i] = v;
-    }
+    for (int i = 0; i < n; ++i) pt[i] = host_pt(x[i], d[i] < 1 ? 1 : (d[i] > 6 ? 6 : d[i]), os, omega);
     return 0;
 }

@@ -19,6 +19,7 @@
 #include "../../include/smoke_gb300.h"
 #include "kernels.h"
 #include "sim_internal.h"
+#include "tb_common.cuh"
 
 using namespace smk;
 
@@ -65,18 +66,41 @@ int check_params(const smk_params* p) {
     return SMK_OK;
 }
 
-// z-chunk of the blocked velocity sweep when none was chosen: about four CTAs' worth of planes
-// per SM-wave of x-y tiles, at least 2T + 8 planes so the chunk's halo stays a minor part.
-int default_vsweep_zchunk(const Grid& g, int T) {
-    const int rows = T == 2 ? 24 : 32;
-    const int tiles = ((g.nx + 1 + 63 - 2 * T) / (64 - 2 * T)) * ((g.ny + 1 + rows - 1 - 2 * T) / (rows - 2 * T));
-    const int planes = g.nz + 1;
-    int chunks = (4 * 152 + tiles - 1) / (tiles > 0 ? tiles : 1);
-    if (chunks < 1) chunks = 1;
-    int zc = (planes + chunks - 1) / chunks;
-    if (zc < 2 * T + 8) zc = 2 * T + 8;
-    return zc;
+// SMs of the current device.
+int device_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaGetLastError();
+    return n > 0 ? n : 152;
 }
+
+// Device time of one launch of the blocked velocity sweep (us): CTAs run in waves of one per SM,
+// each marching its chunk and the T planes of halo on both sides; a march iteration takes 1.4 us
+// with T = 4 and 1.65 with T = 2 (measured at 256^3: 171 us in two waves of 61 iterations, 94 us in
+// one of 57).
+float vsweep_launch_us(const Grid& g, int T, int zchunk, int sms) {
+    const int rows = vsweep_tile_rows(T);
+    const int tiles = tb::sweep_windows(g.nx + 1, 2 * tb::TX, T) * tb::sweep_windows(g.ny + 1, rows, T);
+    const int chunks = (g.nz + zchunk) / zchunk;
+    const int waves = (tiles * chunks + sms - 1) / sms;
+    return 2.0f + (T == 4 ? 1.4f : 1.65f) * (float)waves * (float)(std::min(zchunk, g.nz + 1) + 2 * T + 1);
+}
+
+// The z-chunk with the least vsweep_launch_us.
+int default_vsweep_zchunk(const Grid& g, int T) {
+    const int planes = g.nz + 1, sms = device_sms();
+    int best = planes;
+    for (int n = 1; n <= planes; ++n) {
+        const int zc = (planes + n - 1) / n;
+        if (vsweep_launch_us(g, T, zc, sms) < vsweep_launch_us(g, T, best, sms)) best = zc;
+        if (zc <= 2) break;
+    }
+    return best;
+}
+
+// One colour pass per launch: 25 bytes a cell at 5.3 TB/s (measured: 86.7 us at 256^3, 18.5 at
+// 160^3) and 2 us (4.3 us at 80^3).
+float one_pass_us(const Grid& g) { return 2.0f + 25.0f * (float)g.nx * (float)g.ny * (float)g.nz / 5.3e6f; }
 
 cudaMemcpy3DParms copy3d(void* dst, size_t dpitch, size_t dy, const void* src, size_t spitch,
                          size_t sy, size_t width_bytes, size_t h, size_t d, cudaMemcpyKind kind) {
@@ -160,6 +184,11 @@ int smk_sim::alloc() {
     if (!bf16) {
         vmaps = create_vsweep_maps(g, u, v, w, P, P2, b, flags);
         if (!vmaps) return fail(SMK_ERR_CUDA, "could not encode the TMA tensor maps of the velocity sweep kernel");
+        // blocked above about 110^3: 256^3 x 30 iterations 2.6 ms (5.2 ms with one pass per launch);
+        // below it a march has too few planes to fill the SMs (80^3: 17 us per 4 passes either way)
+        const int zc = default_vsweep_zchunk(g, 4);
+        if (vsweep_launch_us(g, 4, zc, device_sms()) < 0.9f * 4.0f * one_pass_us(g))
+            vsweep_auto = VelocitySweep{4, zc, default_vsweep_zchunk(g, 2)};
         const float* au[2] = {u[0], u[1]};
         const float* av[2] = {v[0], v[1]};
         const float* aw[2] = {w[0], w[1]};
@@ -297,38 +326,40 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     SMK_CUDA(cudaMemsetAsync(status, 0, status_bytes, st));
     last_groups = 0;
     if (p.projection == SMK_PROJECT_REFERENCE) {
-        if (vsweep_depth > 0 && vmaps != nullptr && p.max_sweeps > 0) {
+        const VelocitySweep vs = velocity_sweep();
+        if (vs.depth > 0) {
             // temporally blocked: launches of up to T colour passes alternating between the state
             // (u, v, w)[now] and the scratch arrays (P, P2, b), an even number of them so that the
             // result ends in the state; the passes are those of the loop below, in the same order
-            const int T = vsweep_depth;
             const int H = 2 * p.max_sweeps;
             std::vector<int> plan;
-            for (int h = 0; h < H; h += T) plan.push_back(H - h < T ? H - h : T);
-            if (plan.size() % 2 == 1) {  // split one launch in two (both keep >= 1 pass)
-                if (plan.back() >= 2) {
-                    plan.back() -= 1;
-                    plan.push_back(1);
-                } else {
-                    plan[plan.size() - 2] -= 1;
-                    plan.push_back(1);
-                }
+            if (vs.depth == 4) {
+                // as many launches of 4 as leave an even number in all, then launches of 2 (H is even)
+                int fours = H / 4;
+                if ((fours + (H % 4 ? 1 : 0)) % 2 == 1 && fours > 0) --fours;
+                plan.assign(fours, 4);
+                plan.insert(plan.end(), (H - 4 * fours) / 2, 2);
+            } else {
+                plan.assign(H / 2, 2);
+            }
+            if (plan.size() % 2 == 1) {  // a launch of 2 becomes two of 1
+                plan.back() = 1;
+                plan.push_back(1);
             }
             const OmegaSplit os = omega_split(p.omega);
-            const int zc = vsweep_zchunk > 0 ? vsweep_zchunk : default_vsweep_zchunk(g, T);
             int h = 0;
             for (size_t l = 0; l < plan.size(); ++l) {
                 const bool from_state = (l % 2) == 0;
                 float* uo = from_state ? P : u[now];
                 float* vo = from_state ? P2 : v[now];
                 float* wo = from_state ? b : w[now];
-                if (launch_vsweep_tb(vmaps, g, now, from_state, uo, vo, wo, T, plan[l], h & 1, zc, p.omega, os, kerr,
-                                     st) != 0)
+                const int T = plan[l] == 4 ? 4 : 2;
+                if (launch_vsweep_tb(vmaps, g, now, from_state, uo, vo, wo, T, plan[l], h & 1,
+                                     T == vs.depth ? vs.zchunk : vs.zchunk2, p.omega, os, kerr, st) != 0)
                     return fail(SMK_ERR_CUDA, "velocity sweep kernel launch failed");
                 h += plan[l];
                 ++launches;
             }
-            pressure_clobbered = true;
         } else {
             for (int it = 0; it < p.max_sweeps; ++it) {
                 launch_project_velocity(g, u[now], v[now], w[now], flags, 0, p.omega, st);
@@ -337,6 +368,7 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
             }
         }
     } else {
+        pressure_used = true;
         float wacc[7];
         wacc[0] = 0.0f;
         const double om = pressure_omega();  // omega, or omega_warm once the history is long enough
@@ -569,6 +601,7 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     }
     if (timed) SMK_CUDA(rec(ev[4]));
     SMK_CUDA(cudaGetLastError());
+    mark_scratch();
     ++steps;
     ++hist_steps;
     last_projection = p.projection;
@@ -576,6 +609,25 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     last_max_sweeps = p.max_sweeps;
     last_check_every = p.check_every;
     last_refine = p.projection == SMK_PROJECT_PRESSURE ? p.refine : 0;
+    return SMK_OK;
+}
+
+void smk_sim::set_velocity_sweep(int depth, int zchunk) {
+    vsweep_set = true;
+    vsweep_chosen = VelocitySweep{depth, 0, 0};
+    if (depth == 0) return;
+    vsweep_chosen.zchunk = zchunk > 0 ? zchunk : default_vsweep_zchunk(g, depth);
+    vsweep_chosen.zchunk2 = zchunk > 0 ? zchunk : default_vsweep_zchunk(g, 2);
+}
+
+int smk_sim::settle_pressure(cudaStream_t st) {
+    if (p.projection != SMK_PROJECT_PRESSURE || !(pressure_clobbered || scratch_used)) return SMK_OK;
+    SMK_CUDA(cudaMemsetAsync(P, 0, elems() * sizeof(float), st));
+    SMK_CUDA(cudaMemsetAsync(P2, 0, elems() * sizeof(float), st));
+    SMK_CUDA(cudaMemsetAsync(pcur, 0, sizeof(int), st));
+    // as after smk_write_state where the sweep was one that was set
+    if (pressure_clobbered) hist_steps = 0;
+    pressure_clobbered = scratch_used = false;
     return SMK_OK;
 }
 
@@ -615,8 +667,11 @@ std::string smk_sim::graph_signature(float dt) const {
     put(&sweep_depth, sizeof(sweep_depth));
     put(&sweep_zchunk, sizeof(sweep_zchunk));
     put(&sweep_rows, sizeof(sweep_rows));
-    put(&vsweep_depth, sizeof(vsweep_depth));
-    put(&vsweep_zchunk, sizeof(vsweep_zchunk));
+    if (p.projection == SMK_PROJECT_REFERENCE) {
+        const VelocitySweep v = velocity_sweep();
+        put(&v, sizeof(v));
+        put(&vsweep_set, sizeof(vsweep_set));
+    }
     const char t = timing ? 1 : 0;
     put(&t, 1);
     put(&rb_host, sizeof(rb_host));  // the host readback's copies are nodes of the graph
@@ -632,15 +687,8 @@ std::string smk_sim::graph_signature(float dt) const {
 // obstacles changed runs directly (it includes the one-off mask kernels), and so does a step
 // with stage timing on (events recorded inside a capture cannot be queried afterwards).
 int smk_sim::step(float dt, cudaStream_t st) {
-    if (pressure_clobbered && p.projection == SMK_PROJECT_PRESSURE) {
-        // the blocked velocity sweep of earlier REFERENCE steps left its scratch in P, P2, b: the
-        // pressure history starts over, as after smk_write_state
-        SMK_CUDA(cudaMemsetAsync(P, 0, elems() * sizeof(float), st));
-        SMK_CUDA(cudaMemsetAsync(P2, 0, elems() * sizeof(float), st));
-        SMK_CUDA(cudaMemsetAsync(pcur, 0, sizeof(int), st));
-        pressure_clobbered = false;
-        hist_steps = 0;
-    }
+    const int src = settle_pressure(st);
+    if (src) return src;
     if (!use_graphs || mask_dirty || obstacles_dirty) return enqueue(dt, st);
     GraphSlot& gs = graphs[index_now];
     std::string sig = graph_signature(dt);
@@ -675,6 +723,7 @@ int smk_sim::step(float dt, cudaStream_t st) {
         gs.sig.swap(sig);
     }
     SMK_CUDA(cudaGraphLaunch(gs.exec, st));
+    mark_scratch();
     index_now ^= 1;
     launches += gs.launches;
     ++steps;
@@ -1043,6 +1092,7 @@ int smk_write_state(smk_sim* sim, const smk_host_state* st) {
     SMK_CUDA(cudaMemset(sim->pcur, 0, sizeof(int)));
     SMK_CUDA(cudaDeviceSynchronize());
     sim->hist_steps = 0;
+    sim->pressure_used = false;
     return SMK_OK;
 }
 
@@ -1167,16 +1217,15 @@ int smk_set_velocity_sweep(smk_sim* sim, int depth, int zchunk) {
     if (zchunk < 0) return fail(SMK_ERR_INVALID, "zchunk must be >= 0 (0: chosen from the grid)");
     if (depth != 0 && sim->vmaps == nullptr)
         return fail(SMK_ERR_INVALID, "the blocked velocity sweep needs FP32 storage");
-    sim->vsweep_depth = depth;
-    sim->vsweep_zchunk = zchunk;
+    sim->set_velocity_sweep(depth, zchunk);
     return SMK_OK;
 }
 
 int smk_get_velocity_sweep(const smk_sim* sim, int* depth, int* zchunk) {
     if (!sim) return fail(SMK_ERR_INVALID, "sim is null");
-    const int d = sim->vmaps ? sim->vsweep_depth : 0;
-    if (depth) *depth = d;
-    if (zchunk) *zchunk = d == 0 ? 0 : (sim->vsweep_zchunk > 0 ? sim->vsweep_zchunk : default_vsweep_zchunk(sim->g, d));
+    const smk_sim::VelocitySweep v = sim->velocity_sweep();
+    if (depth) *depth = v.depth;
+    if (zchunk) *zchunk = v.zchunk;
     return SMK_OK;
 }
 
@@ -1253,7 +1302,7 @@ std::map<std::tuple<int, int, int, int, int>, TunedShape> g_tune_cache;
 extern "C" {
 
 // REFERENCE scheme: time the velocity sweep's forms -- one colour pass per launch, and the
-// temporally blocked kernel with depth 2 and 4 over z-chunks without unroll padding -- per
+// temporally blocked kernel with depth 2 and 4 over equal z-chunks -- per
 // iteration (red + black pass) and keep the fastest.  The blocked launches read the state and
 // write the scratch arrays (P, P2, b); the one-pass kernel runs in place on the scratch arrays,
 // so the state is untouched.  Cached per grid shape and device.
@@ -1266,10 +1315,9 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
-            sim->vsweep_depth = sim->vmaps ? it->second.depth : 0;
-            sim->vsweep_zchunk = it->second.zchunk;
-            if (depth_out) *depth_out = sim->vsweep_depth;
-            if (zchunk_out) *zchunk_out = sim->vsweep_zchunk;
+            sim->set_velocity_sweep(sim->vmaps ? it->second.depth : 0, it->second.zchunk);
+            if (depth_out) *depth_out = sim->vsweep_chosen.depth;
+            if (zchunk_out) *zchunk_out = it->second.zchunk;
             if (us_out) *us_out = -1.0f;
             return SMK_OK;
         }
@@ -1320,13 +1368,12 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
     std::vector<Cand> cands{Cand{0, 0, 1e30f}};
     const int depths[2] = {2, 4};
     for (int di = 0; di < 2 && sim->vmaps != nullptr; ++di) {
-        const int T = depths[di], R = T + 2;
-        for (int m = 2; m <= 40; ++m) {
-            const int zc = R * m - 2 * T - 1;
-            if (zc < 4) continue;
-            if (zc > g.nz + 1 + R) break;
-            cands.push_back(Cand{T, zc, 1e30f});
-            if (zc > g.nz + 1) break;
+        const int T = depths[di], planes = g.nz + 1;
+        for (int n = 1, last = 0; n <= 32; ++n) {
+            const int zc = (planes + n - 1) / n;
+            if (zc < 4) break;
+            if (zc != last) cands.push_back(Cand{T, zc, 1e30f});
+            last = zc;
         }
     }
     int rc = SMK_OK;
@@ -1353,8 +1400,7 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
     sim->pressure_clobbered = true;
     int krc = check_kernel_error(sim);
     if (krc) return krc;
-    sim->vsweep_depth = best_d;
-    sim->vsweep_zchunk = best_z;
+    sim->set_velocity_sweep(best_d, best_z);
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         g_tune_cache[key] = TunedShape{best_d, 2, best_z};

@@ -93,12 +93,34 @@ struct smk_sim {
     int sweep_rows = 2;  // cell rows of a thread's patch in the blocked kernel (2 or 4)
     // reference scheme: 0 = one colour pass per launch (k_project_velocity); T = 2 or 4 = the
     // temporally blocked velocity sweep, T passes per launch over z-chunks of vsweep_zchunk planes
-    // (the pressure buffers P, P2, b hold the intermediate face arrays); smk_autotune chooses
-    int vsweep_depth = 0;
-    int vsweep_zchunk = 0;  // 0: chosen from the grid
-    // the blocked velocity sweep used P, P2, b as scratch: a PRESSURE step must restart its
-    // pressure from zero (cleared in step(), outside any captured graph)
+    // (the pressure buffers P, P2, b hold the intermediate face arrays).  Until one is set
+    // (smk_set_velocity_sweep, smk_autotune) velocity_sweep() picks from the grid.
+    bool vsweep_set = false;
+    struct VelocitySweep {
+        int depth, zchunk, zchunk2;  // zchunk2: of the two-pass launches that even out a plan
+    };
+    VelocitySweep vsweep_auto{0, 0, 0};              // from the grid (alloc)
+    VelocitySweep vsweep_chosen{0, 0, 0};            // the one that was set, its chunks resolved
+    VelocitySweep velocity_sweep() const {
+        if (vmaps == nullptr || p.max_sweeps <= 0) return VelocitySweep{0, 0, 0};
+        if (vsweep_set) return vsweep_chosen;
+        return pressure_used || p.max_sweeps < 4 ? VelocitySweep{0, 0, 0} : vsweep_auto;
+    }
+    void set_velocity_sweep(int depth, int zchunk);
+    // P or P2 may hold a pressure history (a PRESSURE step ran): the sweep picked from the grid then
+    // leaves them alone
+    bool pressure_used = false;
+    // a blocked velocity sweep used P, P2, b as scratch: a PRESSURE step must restart its pressure
+    // from zero (settle_pressure, outside any captured graph).  scratch_used: by the sweep picked
+    // from the grid, when there was no history to lose (the pressure was zero and its step count runs
+    // on); pressure_clobbered: by one that was set, and the history starts over
+    bool scratch_used = false;
     bool pressure_clobbered = false;
+    int settle_pressure(cudaStream_t st);
+    void mark_scratch() {  // after a REFERENCE step
+        if (p.projection == SMK_PROJECT_REFERENCE && velocity_sweep().depth > 0)
+            (vsweep_set ? pressure_clobbered : scratch_used) = true;
+    }
     // steps since the pressure history started (creation, smk_write_state, a pressure reset):
     // decides between omega and omega_warm (pressure_omega)
     long long hist_steps = 0;
