@@ -199,8 +199,9 @@ long long smk_launch_count(const smk_sim* sim);
 
 /* Pressure sweep kernel (PRESSURE projection).  depth 0: one colour pass per launch.
  * depth 2, 4 or 6: temporally blocked, `depth` colour passes per pass over HBM, the grid
- * cut into z-chunks of `zchunk` planes (>= 1).  Results are bit-identical for every choice;
- * only speed differs.  No counterpart in the reference (its projection is fixed,
+ * cut into z-chunks of `zchunk` planes (>= 1).  A new simulation has the shape that fits its grid
+ * (a request of a server: its share of the GPU).  Results are bit-identical for every choice; only
+ * speed differs.  No counterpart in the reference (its projection is fixed,
  * smokeSimulation.cu:795-801). */
 int smk_set_sweep_kernel(smk_sim* sim, int depth, int zchunk);
 int smk_get_sweep_kernel(const smk_sim* sim, int* depth, int* zchunk);

@@ -20,6 +20,7 @@
 #include <climits>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/smoke_gb300.h"
@@ -47,6 +48,7 @@ struct smk_batch {
     cudaEvent_t fork = nullptr;
     cudaGraphExec_t exec = nullptr;
     std::string sig;
+    std::vector<std::pair<int, int>> branch_shape;  // BranchShapes: depth, z-chunk per member
     std::vector<long long> branch_launches;
     std::vector<int> groups;
 
@@ -478,8 +480,32 @@ int grouped_step(smk_batch* b, const float* dts, float dt_all, cudaStream_t st) 
     return SMK_OK;
 }
 
+// The sweep shapes of concurrent branches: a member whose shape was not set takes its share of the
+// chip (smk_sim::sweep_share) while the batch issues its step.
+struct BranchShapes {
+    std::vector<smk_sim*> sims;
+    std::vector<std::pair<int, int>> kept;  // depth, z-chunk
+    explicit BranchShapes(const smk_batch* b) {
+        for (size_t i = 0; i < b->sims.size(); ++i) {
+            smk_sim* s = b->sims[i];
+            if (s->sweep_set || b->sims.size() < 2) continue;
+            sims.push_back(s);
+            kept.emplace_back(s->sweep_depth, s->sweep_zchunk);
+            s->sweep_depth = b->branch_shape[i].first;
+            s->sweep_zchunk = b->branch_shape[i].second;
+        }
+    }
+    ~BranchShapes() {
+        for (size_t i = 0; i < sims.size(); ++i) {
+            sims[i]->sweep_depth = kept[i].first;
+            sims[i]->sweep_zchunk = kept[i].second;
+        }
+    }
+};
+
 int branches_step(smk_batch* b, const float* dts, float dt_all, cudaStream_t st) {
     const int n = (int)b->sims.size();
+    const BranchShapes shapes(b);
     bool direct = !b->use_graphs;
     std::string sig;
     for (int i = 0; i < n; ++i) {
@@ -715,6 +741,17 @@ int smk_batch_create(int count, smk_sim* const* sims, smk_batch** out) {
     }
     b->branch_launches.assign(count, 0);
     b->groups.assign(count, 0);
+    double total = 0.0;
+    for (smk_sim* s : b->sims) total += (double)s->g.nx * s->g.ny * s->g.nz;
+    for (smk_sim* s : b->sims) {
+        const std::pair<int, int> own(s->sweep_depth, s->sweep_zchunk);
+        const int rows = s->sweep_rows;
+        s->choose_sweep(s->sweep_share(total));
+        b->branch_shape.emplace_back(s->sweep_depth, s->sweep_zchunk);
+        s->sweep_depth = own.first;
+        s->sweep_zchunk = own.second;
+        s->sweep_rows = rows;
+    }
     *out = b;
     return SMK_OK;
 }
@@ -870,7 +907,7 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
             }
         }
     }
-    // the blocked solve (when every member can use it): depth-6 launches over all grids' tiles,
+    // the blocked solve (when every member can use it): launches over all grids' tiles,
     // timed without tolerance checks, reading P and writing the scratch P2 (no status, no pcur)
     const int zchunks[] = {17, 27, 37, 57, 117, 137, 257};  // 10 m - 13: no padding of the 10-plane unroll
     if (!rc && blocked_eligible(b->sims.data(), n)) {
@@ -900,7 +937,7 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
             rc = upload_table(t, dev, a, n);
             if (rc) break;
             const GroupTBLaunch tb = tb_launch(t, dev, n, nullptr);
-            const int reps = 3, launches = 3;  // 9 sweeps per repetition
+            const int reps = 3, launches = 3;  // GROUP_TB_DEPTH / 2 sweeps each
             int lrc = launch_group_tb_sweeps(tb, launches, st);  // warm
             if (!lrc) lrc = (int)cudaEventRecord(e0, st);
             for (int r = 0; r < reps && !lrc; ++r) lrc = launch_group_tb_sweeps(tb, launches, st);
@@ -912,7 +949,7 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
             }
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, e0, e1);
-            const float us = 1e3f * ms / (reps * launches * 3);
+            const float us = 1e3f * ms / (reps * launches * GROUP_TB_DEPTH / 2);
             if (us < best) {
                 best = us;
                 best_s = GroupSchedule{0, 4, 0, zc};

@@ -105,7 +105,7 @@ struct GroupArgs {
 
 // The blocked form of the grouped solve (host side): instead of the cooperative kernel's colour
 // passes, launches of the temporally blocked sweep kernel over every grid's tiles, each
-// launch depth 6, a tolerance check in the first launch of each group (all grids share the
+// launch GROUP_TB_DEPTH passes, a tolerance check in the first launch of each group (all grids share the
 // group size and the sweep cap), the full groups as a device-side WHILE loop when captured.
 struct GroupTBLaunch {
     const void* grids;   // device records (group_tb_record_bytes() each)

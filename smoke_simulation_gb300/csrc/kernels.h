@@ -93,6 +93,7 @@ constexpr int SWEEP_YCLUSTER = 0x100;
 constexpr int SWEEP_YCLUSTER_N_SHIFT = 9;
 inline int sweep_ycluster_n(int rows) { return (rows >> SWEEP_YCLUSTER_N_SHIFT) & 0xf; }
 int sweep_tb_shape_supported(int T, int rows);
+int sweep_tile_rows(int T);  // cell rows of a tile of the pair form
 // Clusters of the y-cluster form with n_req CTAs each (0: one spanning y) that can be resident
 // at once for grid g (0: not usable).
 int sweep_ycluster_usable(const Grid& g, int n_req);
@@ -100,7 +101,12 @@ int sweep_ycluster_usable(const Grid& g, int n_req);
 int prepare_sweep_kernels();
 struct SweepMaps;
 SweepMaps* create_sweep_maps(const Grid& g, const float* Pa, const float* Pb, const float* b,
-                             const uint8_t* flags);
+                             const uint8_t* flags, const uint16_t* codes);
+// Sweep codes: 16 bits per 2 x 2 patch of cells, derived from the flags whenever they change
+// (kernels_sweep_tb.cu); X/2 x sweep_code_rows x (nz + 1) of them.
+inline int sweep_code_rows(const Grid& g) { return (g.ny + 1) / 2; }
+inline size_t sweep_code_count(const Grid& g) { return (size_t)(g.X / 2) * (size_t)sweep_code_rows(g) * (size_t)(g.nz + 1); }
+void launch_build_codes(const Grid& g, const uint8_t* flags, uint16_t* codes, cudaStream_t st);
 void destroy_sweep_maps(SweepMaps* m);
 // The gradient subtract fused into the last launch of a solve: u, v, w (FP32, the grid's
 // layout) move by the final pressure's gradient inside the launch that applies the last colour
@@ -127,8 +133,9 @@ int launch_sweep_tb(const SweepMaps* m, const Grid& g, bool in_is_a, float* Pout
                     int nhalf, int colour0, int zchunk, const float* wacc7, StepStatus* status,
                     int check, int group, float tol, int* pcur, int out_idx, int* kerr,
                     const int* group_base, cudaStream_t st, const SweepFuse* fuse = nullptr);
-// Grouped blocked solve over many grids (depth 6, 2-row patches): one record per grid (its
+// Grouped blocked solve over many grids (GROUP_TB_DEPTH colour passes per launch): one record per grid (its
 // tensor maps, buffers and tolerance), tiles of all grids in one launch.
+constexpr int GROUP_TB_DEPTH = 4;
 size_t group_tb_record_bytes();
 // Fill one record (rec: group_tb_record_bytes(), 64-byte aligned in the device copy); returns
 // the grid's tile count for `zchunk`-plane chunks.

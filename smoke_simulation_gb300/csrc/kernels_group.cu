@@ -581,11 +581,11 @@ int group_occupancy(int* coop_per_sm, int* stage_per_sm, int* sms) {
 }
 
 // The blocked solve's launches for groups [g0, g1): group k covers sweeps [k G, (k+1) G) (the
-// last one may be partial), depth-6 launches, the first of each with the tolerance check.
+// last one may be partial), launches of GROUP_TB_DEPTH passes, the first of each with the tolerance check.
 // Inside a loop body (group_base set) the group index is relative to *group_base; `nl` counts
 // launches so far (the input buffer alternates, starting from P).
 int issue_tb_groups(const GroupTBLaunch& tb, int g0, int g1, const int* group_base, int& nl, cudaStream_t st) {
-    constexpr int T = 6;
+    constexpr int T = GROUP_TB_DEPTH;
     for (int grp = g0; grp < g1; ++grp) {
         const int first = grp * tb.check_every;
         const int end = first + tb.check_every < tb.max_sweeps ? first + tb.check_every : tb.max_sweeps;
@@ -604,7 +604,7 @@ int issue_tb_groups(const GroupTBLaunch& tb, int g0, int g1, const int* group_ba
 // captured (the loop stops when every grid's tolerance rule is satisfied), then the groups
 // left (a partial last group), whose launches exit at entry for grids that are done.
 int launch_tb_solve(GroupTBLaunch& tb, cudaStream_t st) {
-    constexpr int T = 6;
+    constexpr int T = GROUP_TB_DEPTH;
     const int G = tb.check_every;
     const int nlg = (2 * G + T - 1) / T;
     const int U = (nlg % 2 == 0) ? 1 : 2;
@@ -672,9 +672,9 @@ int launch_group_step(const GroupArgs& a, const GroupLaunch& L, cudaStream_t st,
 }
 
 int launch_group_tb_sweeps(const GroupTBLaunch& tb, int launches, cudaStream_t st) {
-    // tuning: `launches` depth-6 launches without tolerance checks, each reading P and writing P2
+    // tuning: `launches` launches of GROUP_TB_DEPTH passes without tolerance checks, each reading P and writing P2
     for (int k = 0; k < launches; ++k) {
-        const int rc = launch_group_sweep_tb(tb.grids, tb.starts, tb.n, tb.total, true, 6, 0, tb.zchunk, 0, 0,
+        const int rc = launch_group_sweep_tb(tb.grids, tb.starts, tb.n, tb.total, true, GROUP_TB_DEPTH, 0, tb.zchunk, 0, 0,
                                              nullptr, st);
         if (rc) return rc;
     }

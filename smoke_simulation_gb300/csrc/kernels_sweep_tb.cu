@@ -42,13 +42,15 @@
 // flag byte (six neighbour bits + "projectable"), kept in shared memory once per lane so that
 // lookups never conflict.
 //
-// Forms (one tile body, sweep_tile): k_sweep_tb<T, PY, FULL, CHK> (one grid, tensor maps as
-// kernel parameters), k_group_sweep_tb<6, FULL, CHK> (the tiles of every grid of a batch in one
-// launch, each grid's tensor maps in global memory), k_sweep_tb_ycl<6> (runs of 2, 4 or all of
-// the CTAs of an x-z column as thread-block clusters that exchange boundary rows through
-// distributed shared memory instead of recomputing a y-halo between them).  Launches of all T
-// colour passes run the FULL instantiations (no per-stage tests), with the tolerance-check code
-// compiled in (CHK = 1) or out (CHK = 0); partial launches test both at run time.
+// Forms.  The one that steps run is the pair form (sweep_pair_tile, below: k_sweep_pair<T, FULL, CHK> for
+// one grid, k_group_sweep_tb<T, FULL, CHK> for the tiles of every grid of a batch in one launch, each
+// grid's tensor maps in global memory); the description above is that of sweep_tile, which the other
+// shapes still use: k_sweep_tb<4, 4, ...> (4-row patches by rows), k_sweep_tb_fused (the gradient
+// subtract in the last launch), k_sweep_tb_ycl<6> (runs of 2, 4 or all of the CTAs of an x-z column
+// as thread-block clusters that exchange boundary rows through distributed shared memory instead of
+// recomputing a y-halo between them).  Launches of all T colour passes run the FULL instantiations
+// (no per-stage tests), with the tolerance-check code compiled in (CHK = 1) or out (CHK = 0); partial
+// launches test both at run time.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -83,13 +85,20 @@ struct TBGeom {
 
 struct WAcc8 { float w[8]; };
 
-constexpr int GROUP_TB_DEPTH = 6;  // colour passes per launch of the grouped blocked solve
 
 struct TBMaps {
     CUtensorMap pin;  // P_in
     CUtensorMap b;
     CUtensorMap f;
 };
+
+// The pair form's: P_in, b and the sweep codes.
+struct PairMaps {
+    CUtensorMap pin;
+    CUtensorMap b;
+    CUtensorMap c;
+};
+constexpr int CODE_BOX = 40;  // code box width in patches: 32 + up to 7 alignment patches (16 bytes = 8)
 
 // Issue the three boxes of plane z into stage `st` (thread 0 only).
 template <int PY>
@@ -622,6 +631,339 @@ __device__ __forceinline__ void sweep_tile(const TBMaps& maps, const Grid& g, fl
     if (YCLUSTER) cluster_sync_all();  // no CTA leaves while a neighbour may still address it
 }
 
+// ---- the pair form ----------------------------------------------------------------------------
+//
+// The kernel of the plain shapes (depth 2, 4, 6) and of the grouped solve.  What bounds it is the
+// shared-memory pipe (every shuffle, neighbour row, coefficient and published row of a stage is one
+// pass through it) and, close behind, instruction issue; so:
+//   - a cell's coefficients cost one shared word: a 2 x 2 patch has a 12-bit code (its cells' numbers
+//     of fluid neighbours, 0 where not projectable; sweep codes, launch_build_codes), loaded instead
+//     of four flag bytes; omega/acc of both cells of a pair is one 8-byte read indexed by their six
+//     code bits, and -acc comes from the bits themselves;
+//   - the cells a stage updates are held as pairs (E = (A0, B1), O = (B0, A1) of rows 0, 1, and so on
+//     for rows 2, 3): sums of both cells are packed FP32 pairs, one issue slot for two cells;
+//   - T = 4 and 2 hold patches of 4 rows a thread: the y neighbours between its two row pairs are
+//     its own registers, and only the outer rows are published (3 instead of 4 passes a cell);
+//   - a stage publishes what it updated, for the neighbours' next stage on that plane (next
+//     iteration), so one barrier an iteration separates them;
+//   - the tolerance check's residual costs one stage: for the cells of stage 1 it is the residual
+//     that stage computes; for the others it is computed just before, from the planes still at time
+//     0 and the values that stage 1 overwrote in the plane below (prev).
+
+// 256^3, 5 % solids, us a sweep without / with a check every 6 sweeps: T = 4, 64-plane chunks (one wave
+// of 140 CTAs) 33.4 / 35.7; the former 2-row kernel 37.7 / 43.1 at T = 6 (65 CTA columns of half-owned
+// tiles), 42.1 / 46.2 at T = 4.  At 33 us: L1 / shared pipe 62 %, issue 48 % (56 % while active), HBM 39 %;
+// 12 warps hide the stages' latencies only in part.  Not kept: 24 warps of 2-row patches with four
+// coefficients from the table (shared pipe 80 %, 43.5 us), R instead of R / 2 TMA stages at T = 4
+// (36.8 us), a ring two planes longer for the check (52.7 us with checks).
+
+// Patch rows and tile rows (warps) of depth T: 48-row tiles of 12 warps (168 registers a thread) for
+// T = 4, 0.73 of whose cells are owned; 64-row tiles of 16 warps for T = 2 (0.88); T = 6 holds two
+// planes more and keeps 2-row patches (16 warps of 128 registers, 32 rows, 0.51).
+template <int T>
+struct PairGeom {
+    static constexpr int PY = T == 6 ? 2 : 4;
+    static constexpr int H = PY / 2;                  // row pairs of a patch
+    static constexpr int TY = T == 4 ? 12 : 16;
+    static constexpr int ROWS = PY * TY;
+    static constexpr int STAGE_P = ROWS * BOX_F * 4;        // bytes (a multiple of 128)
+    static constexpr int STAGE_C = ROWS / 2 * CODE_BOX * 2;  // bytes (a multiple of 128)
+    static constexpr int STAGE_BYTES = 2 * STAGE_P + STAGE_C;
+    static constexpr int S = T == 2 ? 4 : (T + 2) / 2;  // planes in flight
+    static constexpr int PROW = (TY + 2) * TB_TX;     // floats per published row set
+    static constexpr int THREADS = TB_TX * TY;
+    static constexpr int MAPS = T == 6 ? 0 : T == 4 ? 1 : 2;  // tensor-map set (box height)
+    static_assert(STAGE_P % 128 == 0 && STAGE_C % 128 == 0, "TMA destinations stay 128-byte aligned");
+};
+
+// A plane's ring entry: the patch's codes, six bits a pair: E of rows 0, 1 at bit 7, O at 13, E of
+// rows 2, 3 at 19, O at 25.  Shifted so that a pair's bits lie at 7..12, they are (with this lane's
+// copy or'ed in) the byte offset of its (omega/acc, omega/acc) in the shared table, which has one
+// copy per lane of a half-warp (its 8-byte reads never meet in a bank); and or'ed into 65536.0f (bits
+// 7..9) and 8192.0f (bits 10..12) they count ones, so -acc is one subtraction away.
+constexpr int PAIR_COPIES = 16;
+constexpr int PAIR_TABLE = 64 * PAIR_COPIES * 8;
+constexpr unsigned PAIR_C0 = 0x380u, PAIR_C1 = 0x1c00u;
+__device__ __forceinline__ float pair_nacc0(unsigned c) { return 65536.0f - __uint_as_float((c & PAIR_C0) | 0x47800000u); }
+__device__ __forceinline__ float pair_nacc1(unsigned c) { return 8192.0f - __uint_as_float((c & PAIR_C1) | 0x46000000u); }
+
+// Shared memory: the TMA ring, two buffers of published rows (the row-0 and the last-row value of the
+// stages 0..T-1, and for the residual the other pair's), the coefficient table.
+template <int T>
+constexpr size_t pair_smem_bytes() {
+    using G = PairGeom<T>;
+    return 128 + (size_t)G::S * G::STAGE_BYTES + sizeof(float) * 2 * (2 * T + 2) * G::PROW + PAIR_TABLE;
+}
+
+// One tile (bx, by, bz) of a blocked launch.  At iteration q it takes plane q and brings plane q - t
+// from time t - 1 to time t, t = 1..T; plane q - T is then finished.  CHK, FULL, GLOBAL_MAPS as for
+// sweep_tile.
+template <int T, bool GLOBAL_MAPS, bool FULL, int CHK>
+__device__ __forceinline__ void sweep_pair_tile(const PairMaps& maps, const Grid& g, float* __restrict__ Pout, int nhalf,
+                                                int colour0, int zchunk, const WAcc8& wa, StepStatus* status, int check,
+                                                int group, float tol, int* __restrict__ pcur, int out_idx,
+                                                int* __restrict__ kerr, int bx, int by, int bz, unsigned ntiles) {
+    using G = PairGeom<T>;
+    constexpr int R = T + 2;  // register ring: planes q - T - 1 .. q (even)
+    constexpr int S = G::S;   // TMA stages: R or R/2 (a stage is fixed per unrolled iteration)
+    static_assert(S == R || S == R / 2, "stages");
+    constexpr int TY = G::TY, PROW = G::PROW, PY = G::PY, H = G::H;
+    constexpr int NPUB = 2 * T + 2;
+    const bool chk = CHK < 0 ? check != 0 : CHK == 1;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char* stages = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    float* pub = reinterpret_cast<float*>(stages + S * G::STAGE_BYTES);
+    unsigned char* table = reinterpret_cast<unsigned char*>(pub + 2 * NPUB * PROW);
+    __shared__ __align__(8) uint64_t mbar[S];
+
+    // the solve ended at an earlier check (check_decide at the end of a check launch)
+    if (status != nullptr && *(volatile int*)&status->done) return;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int tid = ty * TB_TX + tx;
+    const bool leader = tid == 0;
+
+    // owned columns [xlo, xhi) and rows [ylo, yhi); X0, Y0 (even) = the window's first column and row
+    int X0, xlo, xhi, Y0, ylo, yhi;
+    sweep_window(g.nx, 2 * TB_TX, T, bx, X0, xlo, xhi);
+    sweep_window(g.ny, G::ROWS, T, by, Y0, ylo, yhi);
+    const int xf = X0 - (X0 & 3);                    // 16-byte aligned float box start
+    const int xc = X0 / 2, xcb = xc - (xc & 7);      // ... and code box start (X0 is even)
+    const int za = bz * zchunk, zb = min(za + zchunk, g.nz);
+    // Planes below 0 are never projectable, so a chunk near z = 0 starts at plane 0 (the zero-initialised
+    // ring stands for the planes below); one plane lower where that gives iteration k of the unrolled
+    // march the pattern of k's parity
+    const int qend = zb - 1 + T;
+    int qbeg = za - T < 0 ? 0 : za - T;
+    qbeg -= (qbeg + colour0 - 1) & 1;
+
+    auto issue = [&](int s, int z) {
+        unsigned char* st = stages + s * G::STAGE_BYTES;
+        const uint32_t bar = smem_u32(&mbar[s]);
+        mbar_expect_tx(bar, (uint32_t)G::STAGE_BYTES);
+        tma_load_3d(smem_u32(st), &maps.pin, xf, Y0, z, bar);
+        tma_load_3d(smem_u32(st + G::STAGE_P), &maps.b, xf, Y0, z, bar);
+        tma_load_3d(smem_u32(st + 2 * G::STAGE_P), &maps.c, xcb, Y0 / 2, z, bar);
+    };
+    if (leader) {
+        if (GLOBAL_MAPS) {
+            tensormap_acquire(&maps.pin);
+            tensormap_acquire(&maps.b);
+            tensormap_acquire(&maps.c);
+        }
+        for (int s = 0; s < S; ++s) mbar_init(smem_u32(&mbar[s]), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        for (int s = 0; s < S && qbeg + s <= qend; ++s) issue(s, qbeg + s);
+        if (pcur != nullptr && (bx | by | bz) == 0) *pcur = out_idx;
+    }
+    for (int i = tid; i < 64 * PAIR_COPIES; i += G::THREADS) {
+        const int e = i / PAIR_COPIES;
+        reinterpret_cast<float2*>(table)[i] = make_float2(wa.w[e & 7], wa.w[e >> 3]);  // w[0] = w[7] = 0
+    }
+    // the padding rows of the published row sets (never written afterwards)
+    for (int i = tid; i < 2 * NPUB * 2 * TB_TX; i += G::THREADS) {
+        const int lane = i % TB_TX, edge = (i / TB_TX) % 2, set = i / (2 * TB_TX);
+        pub[set * PROW + (edge ? (TY + 1) * TB_TX : 0) + lane] = 0.0f;
+    }
+
+    const int x0 = X0 + 2 * tx, y0 = Y0 + PY * ty;
+    const bool inx = x0 >= xlo && x0 < xhi;
+    bool in[PY];  // row r of the patch is a row this tile owns
+#pragma unroll
+    for (int r = 0; r < PY; ++r) in[r] = inx && y0 + r >= ylo && y0 + r < yhi && y0 + r >= 0 && y0 + r < g.ny;
+    const int lofs = PY * ty * BOX_F + (X0 - xf + 2 * tx);  // this thread's patch in a float box
+    const int cofs = H * ty * CODE_BOX + (xc - xcb + tx);   // ... in a code box
+    float* const out0 = Pout + (x0 + g.X * y0);
+    const unsigned lane8 = (unsigned)(tx % PAIR_COPIES) * 8u;
+    const int me0 = (ty + 1) * TB_TX + tx;  // my slot in a padded published row set
+
+    float2 P[2][H][R], B[2][H][R];  // [0] = E, [1] = O; slot = plane mod R
+    unsigned C[R];
+    float2 prev[H];  // the pair that stage 1 updated last, before it did
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) P[0][h][j] = P[1][h][j] = B[0][h][j] = B[1][h][j] = make_float2(0.f, 0.f);
+        C[j] = 0u;
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) prev[h] = make_float2(0.f, 0.f);
+    unsigned rmax = 0u;
+    int par = 0;
+    uint32_t lap = 0;  // laps of the unrolled march, mod 2
+    __syncthreads();  // barriers, table and padding visible
+
+    for (int base = qbeg; base <= qend; base += R, lap ^= 1u) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int q = base + k;
+            if (q > qend) break;
+            const int st = k % S;
+            const int e = k & 1;  // the pair this iteration's stages update
+            float* cur = pub + par * NPUB * PROW;              // written this iteration
+            const float* prv = pub + (par ^ 1) * NPUB * PROW;  // written by the last one
+
+            // ---- plane q into slot k
+            const bool ok = mbar_wait(smem_u32(&mbar[st]), S == R ? lap : (uint32_t)((k / S) & 1));
+            {
+                const unsigned char* S_ = stages + st * G::STAGE_BYTES;
+                const float* sp = reinterpret_cast<const float*>(S_) + lofs;
+                const float* sb = reinterpret_cast<const float*>(S_ + G::STAGE_P) + lofs;
+                const unsigned short* sc = reinterpret_cast<const unsigned short*>(S_ + 2 * G::STAGE_P) + cofs;
+                unsigned c = 0u;
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const float2 p0 = *reinterpret_cast<const float2*>(sp + 2 * h * BOX_F),
+                                 p1 = *reinterpret_cast<const float2*>(sp + (2 * h + 1) * BOX_F);
+                    const float2 b0 = *reinterpret_cast<const float2*>(sb + 2 * h * BOX_F),
+                                 b1 = *reinterpret_cast<const float2*>(sb + (2 * h + 1) * BOX_F);
+                    P[0][h][k] = make_float2(p0.x, p1.y);
+                    P[1][h][k] = make_float2(p0.y, p1.x);
+                    B[0][h][k] = make_float2(b0.x, b1.y);
+                    B[1][h][k] = make_float2(b0.y, b1.x);
+                    c |= (unsigned)sc[h * CODE_BOX] << (7 + 12 * h);
+                }
+                C[k] = c;
+            }
+            if (__syncthreads_or(!ok)) {
+                // a TMA stage never completed: record it, drain what is in flight, stop
+                if (leader) {
+                    atomicExch(kerr, 1);
+                    for (int pq = q; pq <= min(q + S - 1, qend); ++pq) {
+                        const int d = pq - qbeg;
+                        mbar_wait(smem_u32(&mbar[d % S]), (uint32_t)((d / S) & 1));
+                    }
+                }
+                __syncthreads();
+                return;
+            }
+            // every thread has read stage st: refill it with plane q + S
+            if (leader && q + S <= qend) issue(st, q + S);
+
+            // ---- plane q at time 0, for the next iteration's stage 1: the pair of this pattern (the
+            // neighbours of the cells that stage updates), and the other one for its residual
+            cur[me0] = P[e][0][k].x;
+            cur[PROW + me0] = P[e][H - 1][k].y;
+            if (chk) {
+                cur[2 * T * PROW + me0] = P[e ^ 1][0][k].x;
+                cur[(2 * T + 1) * PROW + me0] = P[e ^ 1][H - 1][k].y;
+            }
+
+            // the neighbour sum of the cells of pair pe in plane slot j: n = the other pair there, above
+            // (of the first row) and below (of the last one) from the published rows, zd and zu the same
+            // cells of the planes below and above; plus b
+            auto rhs_sum = [&](int pe, int h, int j, const float2 (&n)[H], float above, float below, float2 zd,
+                               float2 zu) {
+                // x neighbours outside the patch: E: A's left (B of the lane to the left), B's right (A of
+                // the lane to the right); O: B's right (A), A's left (B).  A cell's other x neighbour is
+                // its row's element of n, its y neighbour inside the row pair the other row's
+                float2 xs;
+                if (pe == 0) {
+                    xs.x = __shfl_up_sync(0xffffffffu, n[h].x, 1);
+                    xs.y = __shfl_down_sync(0xffffffffu, n[h].y, 1);
+                } else {
+                    xs.x = __shfl_down_sync(0xffffffffu, n[h].x, 1);
+                    xs.y = __shfl_up_sync(0xffffffffu, n[h].y, 1);
+                }
+                const float2 sx = __fadd2_rn(xs, n[h]);
+                const float2 sy = make_float2((h > 0 ? n[h > 0 ? h - 1 : 0].y : above) + n[h].y,
+                                              n[h].x + (h < H - 1 ? n[h < H - 1 ? h + 1 : h].x : below));
+                return __fadd2_rn(B[pe][h][j], __fadd2_rn(__fadd2_rn(sx, sy), __fadd2_rn(zd, zu)));
+            };
+            auto keep_max = [&](unsigned c, int h, float r0, float r1) {
+                if ((c & PAIR_C0) && in[2 * h]) rmax = max(rmax, __float_as_uint(fabsf(r0)));
+                if ((c & PAIR_C1) && in[2 * h + 1]) rmax = max(rmax, __float_as_uint(fabsf(r1)));
+            };
+            const int zr = q - 1;  // the plane of stage 1
+            const bool own_zr = zr >= za && zr < zb;
+
+            // ---- residual, at time 0, of the cells of plane q - 1 that stage 1 does not update
+            if (chk) {
+                const int j = (k - 1 + R) % R, o = e ^ 1;
+                float2 n[H];
+#pragma unroll
+                for (int h = 0; h < H; ++h) n[h] = P[e][h][j];
+                const float above = prv[(2 * T + 1) * PROW + me0 - TB_TX], below = prv[2 * T * PROW + me0 + TB_TX];
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const float2 s2 = rhs_sum(o, h, j, n, above, below, prev[h], P[o][h][k]);
+                    const unsigned c = C[j] >> (12 * h + 6 * o);
+                    if (own_zr)
+                        keep_max(c, h, fmaf(pair_nacc0(c), P[o][h][j].x, s2.x), fmaf(pair_nacc1(c), P[o][h][j].y, s2.y));
+                    prev[h] = P[e][h][j];
+                }
+            }
+
+            // ---- stages 1..T: plane q - t (slot j) from time t - 1 to time t
+#pragma unroll
+            for (int t = 1; t <= T; ++t) {
+                if (!(FULL || t <= nhalf)) continue;
+                const int j = (k - t + 2 * R) % R;
+                const int ju = (k - t + 1 + 2 * R) % R;
+                const int jd = (k - t - 1 + 2 * R) % R;
+                // row y0 - 1 of the column the first row updates (the thread above's last row), row y0 + PY
+                // of the column the last row updates (the thread below's first): the other pair, as the
+                // stage before published it at the last iteration
+                const float above = prv[(2 * t - 1) * PROW + me0 - TB_TX];
+                const float below = prv[(2 * t - 2) * PROW + me0 + TB_TX];
+                float2 n[H];
+#pragma unroll
+                for (int h = 0; h < H; ++h) n[h] = P[e ^ 1][h][j];
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const unsigned c = C[j] >> (12 * h + 6 * e);
+                    const float2 w = *reinterpret_cast<const float2*>(table + ((c & (PAIR_C0 | PAIR_C1)) | lane8));
+                    const float2 s2 = rhs_sum(e, h, j, n, above, below, P[e][h][jd], P[e][h][ju]);
+                    const float2 p = P[e][h][j];
+                    const float r0 = fmaf(pair_nacc0(c), p.x, s2.x), r1 = fmaf(pair_nacc1(c), p.y, s2.y);
+                    if (t == 1 && chk && own_zr) keep_max(c, h, r0, r1);
+                    // a cell that is not projectable keeps its value, whatever its neighbours hold
+                    if (c & PAIR_C0) P[e][h][j].x = fmaf(w.x, r0, p.x);
+                    if (c & PAIR_C1) P[e][h][j].y = fmaf(w.y, r1, p.y);
+                }
+                if (t < T) {
+                    cur[(2 * t) * PROW + me0] = P[e][0][j].x;
+                    cur[(2 * t + 1) * PROW + me0] = P[e][H - 1][j].y;
+                }
+            }
+
+            // ---- plane q - T is finished
+            const int zo = q - T;
+            if (zo >= za) {
+                const int j = (k - T + R) % R;
+                float* o = out0 + g.XY * zo;
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    if (in[2 * h])
+                        *reinterpret_cast<float2*>(o + 2 * h * g.X) = make_float2(P[0][h][j].x, P[1][h][j].x);
+                    if (in[2 * h + 1])
+                        *reinterpret_cast<float2*>(o + (2 * h + 1) * g.X) = make_float2(P[1][h][j].y, P[0][h][j].y);
+                }
+            }
+            par ^= 1;
+        }
+    }
+
+    if (chk) {
+        // the residual of this launch's input; if it is within tolerance the solve ends on that
+        // input and this launch's passes are dropped
+        block_max_to(rmax, &status->rmax_bits[group]);
+        if (tid == 0) check_decide(status, group, tol, ntiles, pcur, 1 - out_idx);
+    }
+}
+
+template <int T, bool FULL, int CHK>
+__global__ void __launch_bounds__(PairGeom<T>::THREADS, 1)
+k_sweep_pair(const __grid_constant__ PairMaps maps, Grid g, float* __restrict__ Pout, int nhalf, int colour0, int zchunk,
+             const __grid_constant__ WAcc8 wa, StepStatus* status, int check, int group, float tol,
+             int* __restrict__ pcur, int out_idx, int* __restrict__ kerr, const int* __restrict__ group_base) {
+    // inside a graph's device-side group loop the group index is relative to the loop counter
+    if (group_base != nullptr) group += *group_base;
+    sweep_pair_tile<T, false, FULL, CHK>(maps, g, Pout, nhalf, colour0, zchunk, wa, status, check, group, tol, pcur,
+                                         out_idx, kerr, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z,
+                                         gridDim.x * gridDim.y * gridDim.z);
+}
+
 template <int T, int PY, bool FULL, int CHK>
 __global__ void __launch_bounds__(TBGeom<PY>::THREADS, 1)
 k_sweep_tb(const __grid_constant__ TBMaps maps, Grid g, float* __restrict__ Pout, int nhalf,
@@ -666,7 +1008,7 @@ k_sweep_tb_ycl(const __grid_constant__ TBMaps maps, Grid g, float* __restrict__ 
 // One grid of a grouped blocked launch.  The tensor maps live in global memory (64-byte
 // aligned records), one set per input buffer: maps[0] reads P, maps[1] reads P2.
 struct GroupTBGrid {
-    TBMaps maps[2];
+    PairMaps maps[2];
     Grid g;
     float* P;
     float* P2;
@@ -681,7 +1023,7 @@ struct GroupTBGrid {
 // CTA b of the launch takes tile b of the flat index space (the tiles of one grid are
 // contiguous; `starts` holds n + 1 prefix sums).  in_a: read P and write P2, else the reverse.
 template <int T, bool FULL, int CHK>
-__global__ void __launch_bounds__(TBGeom<2>::THREADS, 1)
+__global__ void __launch_bounds__(PairGeom<T>::THREADS, 1)
 k_group_sweep_tb(const GroupTBGrid* __restrict__ grids, const int* __restrict__ starts, int n, int in_a,
                  int nhalf, int colour0, int zchunk, int check, int group, const int* __restrict__ group_base) {
     const int t = (int)blockIdx.x;
@@ -703,9 +1045,8 @@ k_group_sweep_tb(const GroupTBGrid* __restrict__ grids, const int* __restrict__ 
     int* const pcur = d.pcur;
     int* const kerr = d.kerr;
     const float tol = d.tol;
-    sweep_tile<T, 2, true, false, FULL, CHK>(d.maps[in_a ? 0 : 1], g, Pout, nhalf, colour0, zchunk, d.wa, status,
-                                             check, group, tol, pcur, in_a ? 1 : 0, kerr, bx, by, bz,
-                                             (unsigned)(per * d.zchunks));
+    sweep_pair_tile<T, true, FULL, CHK>(d.maps[in_a ? 0 : 1], g, Pout, nhalf, colour0, zchunk, d.wa, status, check,
+                                        group, tol, pcur, in_a ? 1 : 0, kerr, bx, by, bz, (unsigned)(per * d.zchunks));
 }
 
 // End of one iteration of a grouped step's device-side loop over tolerance groups: advance
@@ -804,6 +1145,42 @@ int launch_tb(const TBMaps& maps, const Grid& g, float* Pout, int nhalf, int col
     return 0;
 }
 
+template <int T>
+int configure_pair() {
+    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    static_assert(pair_smem_bytes<T>() + 256 <= 227 * 1024, "shared memory of the pair form");
+    const int bytes = (int)pair_smem_bytes<T>();
+    const bool ok = cudaFuncSetAttribute(k_sweep_pair<T, false, -1>, attr, bytes) == cudaSuccess &&
+                    cudaFuncSetAttribute(k_sweep_pair<T, true, 0>, attr, bytes) == cudaSuccess &&
+                    cudaFuncSetAttribute(k_sweep_pair<T, true, 1>, attr, bytes) == cudaSuccess &&
+                    cudaFuncSetAttribute(k_sweep_tb_fused<T, 2>, attr, (int)tb_smem_bytes_fused<T, 2>()) == cudaSuccess;
+    return ok ? 0 : -1;
+}
+
+template <int T>
+int launch_pair(const PairMaps& maps, const TBMaps& maps32, const Grid& g, float* Pout, int nhalf, int colour0, int zchunk,
+                const float* wacc7, StepStatus* status, int check, int group, float tol, int* pcur, int out_idx,
+                int* kerr, const int* group_base, cudaStream_t st, const SweepFuse* fuse) {
+    using G = PairGeom<T>;
+    WAcc8 wa;
+    for (int k = 0; k < 7; ++k) wa.w[k] = wacc7[k];
+    wa.w[7] = 0.0f;
+    const unsigned nz = (unsigned)((g.nz + zchunk - 1) / zchunk), nx = (unsigned)sweep_windows(g.nx, 2 * TB_TX, T);
+    const dim3 grid(nx, (unsigned)sweep_windows(g.ny, G::ROWS, T), nz), block(TB_TX, G::TY);
+#define SMK_PAIR_LAUNCH(FULL, CHK)                                                                             \
+    k_sweep_pair<T, FULL, CHK><<<grid, block, pair_smem_bytes<T>(), st>>>(                                     \
+        maps, g, Pout, nhalf, colour0, zchunk, wa, status, check, group, tol, pcur, out_idx, kerr, group_base)
+    if (nhalf == T && check) SMK_PAIR_LAUNCH(true, 1);
+    else if (nhalf == T && fuse != nullptr && fuse->mode == 1)
+        k_sweep_tb_fused<T, 2><<<dim3(nx, (unsigned)sweep_windows(g.ny, TBGeom<2>::ROWS, T), nz),
+                                 dim3(TB_TX, TBGeom<2>::TY), tb_smem_bytes_fused<T, 2>(), st>>>(
+            maps32, g, Pout, colour0, zchunk, wa, status, group, tol, pcur, out_idx, kerr, group_base, *fuse);
+    else if (nhalf == T) SMK_PAIR_LAUNCH(true, 0);
+    else SMK_PAIR_LAUNCH(false, -1);
+#undef SMK_PAIR_LAUNCH
+    return 0;
+}
+
 constexpr int YCL_DEPTH = 6;  // the y-cluster form's depth
 
 // Cluster geometry of a y-cluster shape: `n` CTAs per cluster, `hy` halo rows at each end of a
@@ -859,6 +1236,22 @@ int launch_tb_ycl(int n_req, const TBMaps& maps, const Grid& g, float* Pout, int
     return e == cudaSuccess ? 0 : -1;
 }
 
+// The sweep codes from the flags: patch (i, j) of plane z covers cells (2i, 2j) .. (2i + 1, 2j + 1);
+// a cell's three bits are its number of fluid neighbours, 0 where it is not projectable (every
+// projectable cell has at least one), in the order A0, B1, B0, A1 (A = column 2i, 0 = row 2j).
+__global__ void k_build_codes(Grid g, const uint8_t* __restrict__ flags, uint16_t* __restrict__ codes, int rows) {
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x), j = (int)blockIdx.y, z = (int)blockIdx.z;
+    if (i >= g.X / 2) return;
+    auto acc = [&](int x, int y) -> unsigned {
+        if (x >= g.nx || y >= g.ny || z >= g.nz) return 0u;
+        const unsigned f = flags[g.idx(x, y, z)];
+        return (f & F_PROJ) ? (unsigned)__popc(f & F_NBRS) : 0u;
+    };
+    const int x = 2 * i, y = 2 * j;
+    codes[(size_t)i + (size_t)(g.X / 2) * ((size_t)j + (size_t)rows * (size_t)z)] =
+        (uint16_t)(acc(x, y) | (acc(x + 1, y + 1) << 3) | (acc(x + 1, y) << 6) | (acc(x, y + 1) << 9));
+}
+
 // End of one iteration of a graph's device-side loop over tolerance groups: advance the group
 // counter and keep looping while the solve is not done and full groups remain.  One thread.
 __global__ void k_group_loop_next(const StepStatus* status, int* counter, int step, int limit,
@@ -893,11 +1286,26 @@ bool encode_3d_box(CUtensorMap* m, const void* base, bool is_u8, const Grid& g, 
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
+
+bool encode_codes(CUtensorMap* m, const void* base, const Grid& g, int box_w, int box_h) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn || base == nullptr || (reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (box_w * 2) % 16 != 0) return false;
+    // rows of X/2 patches (X is a multiple of 16: 16-byte strides)
+    cuuint64_t dims[3] = {(cuuint64_t)(g.X / 2), (cuuint64_t)sweep_code_rows(g), (cuuint64_t)(g.nz + 1)};
+    cuuint64_t strides[2] = {(cuuint64_t)g.X, (cuuint64_t)g.X * (cuuint64_t)sweep_code_rows(g)};
+    cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, 1u};
+    cuuint32_t estr[3] = {1u, 1u, 1u};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 }  // namespace tb
 
 bool sweep_tb_fusable(int T, int rows, int nhalf, int check) {
     return (rows == 2 || rows == 4) && sweep_tb_shape_supported(T, rows) && nhalf == T && !check;
 }
+
+int sweep_tile_rows(int T) { return T == 6 ? PairGeom<6>::ROWS : T == 4 ? PairGeom<4>::ROWS : PairGeom<2>::ROWS; }
 
 int sweep_tb_shape_supported(int T, int rows) {
     if (rows & SWEEP_YCLUSTER) {
@@ -925,33 +1333,36 @@ int sweep_ycluster_usable(const Grid& g, int n_req) {
 }
 
 int prepare_sweep_kernels() {
-    const int gbytes = (int)tb_smem_bytes<GROUP_TB_DEPTH, 2>();
     const cudaFuncAttribute gattr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    const int grouped = (cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, false, -1>, gattr, gbytes) == cudaSuccess &&
-                         cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, true, 0>, gattr, gbytes) == cudaSuccess &&
-                         cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, true, 1>, gattr, gbytes) == cudaSuccess)
+    const int gb = (int)pair_smem_bytes<GROUP_TB_DEPTH>();
+    const int grouped = (cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, false, -1>, gattr, gb) == cudaSuccess &&
+                         cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, true, 0>, gattr, gb) == cudaSuccess &&
+                         cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, true, 1>, gattr, gb) == cudaSuccess)
                             ? 0 : -1;
     const int ycl = cudaFuncSetAttribute(k_sweep_tb_ycl<YCL_DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tb_smem_bytes<YCL_DEPTH, 2>()) == cudaSuccess ? 0 : -1;
-    return configure_tb<2, 2>() | configure_tb<4, 2>() | configure_tb<6, 2>() | configure_tb<4, 4>() | grouped | ycl;
+    return configure_pair<2>() | configure_pair<4>() | configure_pair<6>() | configure_tb<4, 4>() | grouped | ycl;
 }
 
-// Tensor maps for the sweep's TMA loads: P_a, P_b, b (float) and flags (u8), for the box
-// heights of the 2-row ([0]) and 4-row ([1]) patch kernels.
+// Tensor maps for the sweep's TMA loads: P_a, P_b, b (float) for boxes of 32, 48 and 64 rows, the
+// sweep codes of those boxes, and the flags (u8) for boxes of 32 rows.
 struct SweepMaps {
-    CUtensorMap pa[2], pb[2], b[2], f[2];
+    CUtensorMap pa[3], pb[3], b[3], c[3], f;
 };
 
 SweepMaps* create_sweep_maps(const Grid& g, const float* Pa, const float* Pb, const float* b,
-                             const uint8_t* flags) {
+                             const uint8_t* flags, const uint16_t* codes) {
+    static_assert(TBGeom<2>::ROWS == 32 && TBGeom<4>::ROWS == 32 && PairGeom<6>::ROWS == 32 && PairGeom<4>::ROWS == 48 &&
+                      PairGeom<2>::ROWS == 64, "box heights");
     SweepMaps* m = new SweepMaps();
-    const int rows[2] = {TBGeom<2>::ROWS, TBGeom<4>::ROWS};
-    for (int v = 0; v < 2; ++v) {
-        if (!encode_3d(&m->pa[v], Pa, false, g, rows[v]) || !encode_3d(&m->pb[v], Pb, false, g, rows[v]) ||
-            !encode_3d(&m->b[v], b, false, g, rows[v]) || !encode_3d(&m->f[v], flags, true, g, rows[v])) {
-            delete m;
-            return nullptr;
-        }
+    const int rows[3] = {32, 48, 64};
+    bool ok = encode_3d(&m->f, flags, true, g, 32);
+    for (int v = 0; v < 3 && ok; ++v)
+        ok = encode_3d(&m->pa[v], Pa, false, g, rows[v]) && encode_3d(&m->pb[v], Pb, false, g, rows[v]) &&
+             encode_3d(&m->b[v], b, false, g, rows[v]) && tb::encode_codes(&m->c[v], codes, g, CODE_BOX, rows[v] / 2);
+    if (!ok) {
+        delete m;
+        return nullptr;
     }
     return m;
 }
@@ -964,22 +1375,32 @@ int launch_sweep_tb(const SweepMaps* m, const Grid& g, bool in_is_a, float* Pout
                     const int* group_base, cudaStream_t st, const SweepFuse* fuse) {
     if (!sweep_tb_shape_supported(T, rows)) return -1;
     if (fuse != nullptr && (fuse->mode == 0 || !sweep_tb_fusable(T, rows, nhalf, check))) fuse = nullptr;
-    const int v = rows == 4 ? 1 : 0;
-    TBMaps maps;
-    maps.pin = in_is_a ? m->pa[v] : m->pb[v];
-    maps.b = m->b[v];
-    maps.f = m->f[v];
-#define SMK_TB_ARGS maps, g, Pout, nhalf, colour0, zchunk, wacc7, status, check, group, tol, pcur, out_idx, kerr, group_base, st
-    if (rows & SWEEP_YCLUSTER) return launch_tb_ycl(sweep_ycluster_n(rows), SMK_TB_ARGS);
-#undef SMK_TB_ARGS
-#define SMK_TB_ARGS maps, g, Pout, nhalf, colour0, zchunk, wacc7, status, check, group, tol, pcur, out_idx, kerr, group_base, st, fuse
-    if (rows == 4) return launch_tb<4, 4>(SMK_TB_ARGS);
+    auto set = [&](int v) {
+        PairMaps maps;
+        maps.pin = in_is_a ? m->pa[v] : m->pb[v];
+        maps.b = m->b[v];
+        maps.c = m->c[v];
+        return maps;
+    };
+    TBMaps maps32;
+    maps32.pin = in_is_a ? m->pa[0] : m->pb[0];
+    maps32.b = m->b[0];
+    maps32.f = m->f;
+#define SMK_TB_ARGS g, Pout, nhalf, colour0, zchunk, wacc7, status, check, group, tol, pcur, out_idx, kerr, group_base, st
+    if (rows & SWEEP_YCLUSTER) return launch_tb_ycl(sweep_ycluster_n(rows), maps32, SMK_TB_ARGS);
+    if (rows == 4) return launch_tb<4, 4>(maps32, SMK_TB_ARGS, fuse);
     switch (T) {
-        case 2: return launch_tb<2, 2>(SMK_TB_ARGS);
-        case 4: return launch_tb<4, 2>(SMK_TB_ARGS);
-        default: return launch_tb<6, 2>(SMK_TB_ARGS);
+        case 2: return launch_pair<2>(set(PairGeom<2>::MAPS), maps32, SMK_TB_ARGS, fuse);
+        case 4: return launch_pair<4>(set(PairGeom<4>::MAPS), maps32, SMK_TB_ARGS, fuse);
+        default: return launch_pair<6>(set(PairGeom<6>::MAPS), maps32, SMK_TB_ARGS, fuse);
     }
 #undef SMK_TB_ARGS
+}
+
+void launch_build_codes(const Grid& g, const uint8_t* flags, uint16_t* codes, cudaStream_t st) {
+    const int rows = sweep_code_rows(g);
+    k_build_codes<<<dim3((unsigned)((g.X / 2 + 127) / 128), (unsigned)rows, (unsigned)(g.nz + 1)), 128, 0, st>>>(g, flags, codes,
+                                                                                                         rows);
 }
 
 size_t group_tb_record_bytes() { return sizeof(GroupTBGrid); }
@@ -989,10 +1410,11 @@ int group_tb_fill(void* rec, const SweepMaps* m, const Grid& g, float* P, float*
     constexpr int T = GROUP_TB_DEPTH;
     GroupTBGrid d;
     memset(&d, 0, sizeof(d));
-    d.maps[0].pin = m->pa[0];
-    d.maps[1].pin = m->pb[0];
-    d.maps[0].b = d.maps[1].b = m->b[0];
-    d.maps[0].f = d.maps[1].f = m->f[0];
+    constexpr int v = PairGeom<T>::MAPS;
+    d.maps[0].pin = m->pa[v];
+    d.maps[1].pin = m->pb[v];
+    d.maps[0].b = d.maps[1].b = m->b[v];
+    d.maps[0].c = d.maps[1].c = m->c[v];
     d.g = g;
     d.P = P;
     d.P2 = P2;
@@ -1003,7 +1425,7 @@ int group_tb_fill(void* rec, const SweepMaps* m, const Grid& g, float* P, float*
     d.wa.w[7] = 0.0f;
     d.tol = tol;
     d.tiles_x = sweep_windows(g.nx, 2 * TB_TX, T);
-    d.tiles_y = sweep_windows(g.ny, TBGeom<2>::ROWS, T);
+    d.tiles_y = sweep_windows(g.ny, PairGeom<T>::ROWS, T);
     d.zchunks = (g.nz + zchunk - 1) / zchunk;
     memcpy(rec, &d, sizeof(d));
     return d.tiles_x * d.tiles_y * d.zchunks;
@@ -1014,8 +1436,9 @@ int launch_group_sweep_tb(const void* grids, const int* starts, int n, int total
     if (total_tiles <= 0) return 0;
     // as launch_tb: full launches without per-stage tests, check code present only where needed
 #define SMK_GTB_LAUNCH(FULL, CHK)                                                                             \
-    k_group_sweep_tb<GROUP_TB_DEPTH, FULL, CHK><<<(unsigned)total_tiles, dim3(TB_TX, TBGeom<2>::TY),          \
-                                                 tb_smem_bytes<GROUP_TB_DEPTH, 2>(), st>>>(                  \
+    k_group_sweep_tb<GROUP_TB_DEPTH, FULL, CHK><<<(unsigned)total_tiles,                                      \
+                                                 dim3(TB_TX, PairGeom<GROUP_TB_DEPTH>::TY),                   \
+                                                 pair_smem_bytes<GROUP_TB_DEPTH>(), st>>>(                    \
         static_cast<const GroupTBGrid*>(grids), starts, n, in_a ? 1 : 0, nhalf, colour0, zchunk, check, group, \
         group_base)
     if (nhalf == GROUP_TB_DEPTH && check) SMK_GTB_LAUNCH(true, 1);

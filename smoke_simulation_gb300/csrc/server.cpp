@@ -80,7 +80,8 @@ struct TickRec {
 size_t footprint(int nx, int ny, int nz) {
     const size_t X = ((size_t)nx + 1 + 15) / 16 * 16;
     const size_t elems = X * (size_t)(ny + 1) * (size_t)(nz + 1);
-    return elems * (11 * sizeof(float) + 2) + (1u << 20);
+    // 11 float fields, mask and flags, half a byte of sweep code (a 16-bit code per 2 x 2 patch)
+    return elems * (11 * sizeof(float) + 3) + (1u << 20);
 }
 
 }  // namespace
@@ -307,6 +308,13 @@ static void note_admission(smk_server* s, Request* r) {
 
 static int admit(smk_server* s, Request* r) {
     int rc = smk_create(r->nx, r->ny, r->nz, &r->params, &r->sim);
+    if (rc == SMK_OK && s->mode == SMK_SERVE_STREAMS) {
+        // its steps run next to those of the requests that are active or waiting
+        double total = (double)r->nx * r->ny * r->nz;
+        for (const Request* q : s->active) total += (double)q->nx * q->ny * q->nz;
+        for (const Request* q : s->queue) total += (double)q->nx * q->ny * q->nz;
+        r->sim->choose_sweep(r->sim->sweep_share(total));
+    }
     if (rc == SMK_OK) rc = smk_set_graph_loops(r->sim, s->graph_loops);
     if (rc == SMK_OK && !r->mask.empty()) rc = smk_set_solid_mask(r->sim, r->mask.data());
     for (size_t k = 0; rc == SMK_OK && k < r->boxes.size() / 9; ++k) {

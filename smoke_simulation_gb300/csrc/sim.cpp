@@ -98,6 +98,15 @@ int default_vsweep_zchunk(const Grid& g, int T) {
     return best;
 }
 
+// The same of the blocked pressure sweep: a march iteration takes 0.92 us with T = 4 and 0.87 with
+// T = 6 (measured at 256^3: 67 us in one wave of 72 iterations, 113 us in 130).
+float sweep_launch_us(const Grid& g, int T, int zchunk, int sms) {
+    const int tiles = tb::sweep_windows(g.nx, 2 * tb::TX, T) * tb::sweep_windows(g.ny, sweep_tile_rows(T), T);
+    const int chunks = (g.nz + zchunk - 1) / zchunk;
+    const int waves = (tiles * chunks + sms - 1) / sms;
+    return 3.0f + (T == 4 ? 0.92f : 0.87f) * (float)waves * (float)(std::min(zchunk, g.nz) + 2 * T + 1);
+}
+
 // One colour pass per launch: 25 bytes a cell at 5.3 TB/s (measured: 86.7 us at 256^3, 18.5 at
 // 160^3) and 2 us (4.3 us at 80^3).
 float one_pass_us(const Grid& g) { return 2.0f + 25.0f * (float)g.nx * (float)g.ny * (float)g.nz / 5.3e6f; }
@@ -178,8 +187,10 @@ int smk_sim::alloc() {
     SMK_CUDA(cudaMalloc((void**)&s, n));
     SMK_CUDA(cudaMalloc((void**)&flags, n));
     SMK_CUDA(cudaMemset(flags, 0, n));
+    SMK_CUDA(cudaMalloc((void**)&codes, sweep_code_count(g) * sizeof(uint16_t)));
+    SMK_CUDA(cudaMemset(codes, 0, sweep_code_count(g) * sizeof(uint16_t)));
     // the tensor maps capture the buffer addresses: every buffer must exist first
-    maps = create_sweep_maps(g, P, P2, b, flags);
+    maps = create_sweep_maps(g, P, P2, b, flags, codes);
     if (!maps) return fail(SMK_ERR_CUDA, "could not encode the TMA tensor maps of the sweep kernel");
     if (!bf16) {
         vmaps = create_vsweep_maps(g, u, v, w, P, P2, b, flags);
@@ -201,6 +212,7 @@ int smk_sim::alloc() {
         amaps = create_advect_maps(g, au, av, aw, 1);
     }
     if (!amaps) return fail(SMK_ERR_CUDA, "could not encode the TMA tensor maps of the velocity advection");
+    choose_sweep(device_sms());
     status_groups = 4096;
     SMK_CUDA(cudaMalloc((void**)&status, sizeof(StepStatus) + sizeof(unsigned) * status_groups));
     SMK_CUDA(cudaMemset(status, 0, sizeof(StepStatus) + sizeof(unsigned) * status_groups));
@@ -234,6 +246,7 @@ void smk_sim::release() {
     if (amaps) destroy_advect_maps(amaps);
     if (s) cudaFree(s);
     if (flags) cudaFree(flags);
+    if (codes) cudaFree(codes);
     if (status) cudaFree(status);
     if (tune_status) cudaFree(tune_status);
     for (auto& e : ev)
@@ -298,7 +311,8 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     obstacles_dirty = false;
     if (mask_dirty) {
         launch_build_flags(g, s, flags, st);
-        ++launches;
+        launch_build_codes(g, flags, codes, st);
+        launches += 2;
         mask_dirty = false;
     }
     if (timed) SMK_CUDA(rec(ev[1]));
@@ -612,6 +626,40 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     return SMK_OK;
 }
 
+// The blocked sweep's depth and z-chunk with the least device time per sweep on `sms` SMs: short
+// chunks fill the chip on small grids, long ones recompute fewer halo planes on large ones, and the
+// CTAs should come out as whole waves.  256^3: depth 4, 64 planes (140 CTAs, 33 us a sweep; 37 planes,
+// the same kernel in two uneven waves, 45); 128^3: 8 planes (10 us a sweep; 47 planes, 34).
+void smk_sim::choose_sweep(int sms) {
+    const bool tol = p.projection == SMK_PROJECT_PRESSURE && p.tol > 0.0f;
+    const int passes = 2 * (tol ? p.check_every : std::max(1, std::min(p.max_sweeps, 60)));
+    float best = 1e30f;
+    for (int T = 4; T <= 6; T += 2) {
+        const int launches = (passes + T - 1) / T;
+        for (int n = 1; n <= g.nz; ++n) {
+            const int zc = (g.nz + n - 1) / n;
+            const float us = (float)launches * sweep_launch_us(g, T, zc, sms);
+            if (us < best) {
+                best = us;
+                sweep_depth = T;
+                sweep_zchunk = zc;
+            }
+            if (zc <= 4) break;
+        }
+    }
+    sweep_rows = 2;
+}
+
+// In proportion to its cells, and at least one SM per 40,000: with more concurrent grids than that,
+// chunks longer than its march needs would only keep its own chain of launches waiting (48-request
+// stream: 40,000 cells an SM 688 ms, 80,000 695, 160,000 783, 20,000 790, the whole chip for every
+// grid 958).
+int smk_sim::sweep_share(double total) const {
+    const double cells = (double)g.nx * g.ny * g.nz, sms = device_sms();
+    const double per_sm = std::min(40000.0, std::max(total, cells) / sms);
+    return (int)std::max(1.0, std::min(sms, std::floor(cells / per_sm)));
+}
+
 void smk_sim::set_velocity_sweep(int depth, int zchunk) {
     vsweep_set = true;
     vsweep_chosen = VelocitySweep{depth, 0, 0};
@@ -644,7 +692,8 @@ int smk_sim::prepare_mask(cudaStream_t st) {
     obstacles_dirty = false;
     if (mask_dirty) {
         launch_build_flags(g, s, flags, st);
-        ++n;
+        launch_build_codes(g, flags, codes, st);
+        n += 2;
         mask_dirty = false;
     }
     launches += n;
@@ -1204,6 +1253,7 @@ int smk_set_sweep_shape(smk_sim* sim, int depth, int rows, int zchunk) {
                                          "cluster spans y)");
     }
     if (zchunk < 1) return fail(SMK_ERR_INVALID, "zchunk must be >= 1");
+    sim->sweep_set = true;
     sim->sweep_depth = depth;
     sim->sweep_rows = depth != 0 ? rows : 2;
     sim->sweep_zchunk = zchunk;
@@ -1282,8 +1332,8 @@ int smk_get_sweep_shape(const smk_sim* sim, int* depth, int* rows, int* zchunk) 
 // The blocked sweep kernel has two free parameters: the depth T (colour passes per HBM pass)
 // and the z-chunk (planes per CTA).  Larger T moves fewer bytes per sweep but recomputes a
 // wider halo; the z-chunk trades the pipeline's start-up planes against wave quantisation on
-// the SM count.  Candidates are chunks with no unroll padding ((chunk + 2T + 1) a multiple of
-// the ring length T + 4); each is timed on the simulation's own buffers with CUDA events and
+// the SM count.  Candidates are equal chunks (y-cluster and 4-row forms: chunks with no unroll
+// padding, (chunk + 2T + 1) a multiple of the ring length T + 4); each is timed on the simulation's own buffers with CUDA events and
 // the fastest is kept.  Results are cached per grid shape for the process.  Tuning reads P, b
 // and the flags and writes only the second pressure buffer, after moving a live pressure out
 // of it, so the simulation's results do not depend on whether or when tuning ran.
@@ -1425,6 +1475,7 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
+            sim->sweep_set = true;
             sim->sweep_depth = it->second.depth;
             sim->sweep_rows = it->second.rows;
             sim->sweep_zchunk = it->second.zchunk;
@@ -1513,7 +1564,16 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
     for (const auto& shape : shapes) {
         const int d = shape[0], rows = shape[1];
         if (d == 0) continue;
-        const int R = d + 4;
+        if (rows == 2) {  // the pair form: equal chunks
+            for (int n = 1, last = 0; n <= 32; ++n) {
+                const int zc = (g.nz + n - 1) / n;
+                if (zc < 4) break;
+                if (zc != last) cands.push_back(Cand{d, rows, zc, 1e30f});
+                last = zc;
+            }
+            continue;
+        }
+        const int R = d + 4;  // the other forms: no padding of the march's unroll
         for (int m = 2; m <= 16; ++m) {
             const int zc = R * m - 2 * d - 1;
             if (zc < 8) continue;
@@ -1551,6 +1611,7 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
     SMK_CUDA(cudaGetLastError());
     int krc = check_kernel_error(sim);
     if (krc) return krc;
+    sim->sweep_set = true;
     sim->sweep_depth = best_d;
     sim->sweep_rows = best_r;
     sim->sweep_zchunk = best_z;

@@ -77,6 +77,7 @@ struct smk_sim {
     smk::VSweepMaps* vmaps = nullptr;  // TMA tensor maps of u, v, w (both buffers), P, P2, b, flags
     uint8_t* s = nullptr;
     uint8_t* flags = nullptr;
+    uint16_t* codes = nullptr;  // sweep codes (launch_build_codes), rebuilt with the flags
     smk::StepStatus* status = nullptr;
     smk::StepStatus* tune_status = nullptr;  // status of the autotuner's timing launches
     int status_groups = 0;
@@ -87,9 +88,14 @@ struct smk_sim {
     bool obstacles_dirty = false;
 
     // sweep kernel: 0 = one colour pass per launch; T > 0 = temporally blocked, T passes per
-    // launch over z-chunks of sweep_zchunk planes (chosen by smk_set_sweep_kernel / autotune)
+    // launch over z-chunks of sweep_zchunk planes (from the grid at creation, choose_sweep;
+    // smk_set_sweep_kernel / autotune)
+    bool sweep_set = false;
     int sweep_depth = 4;
     int sweep_zchunk = 47;
+    void choose_sweep(int sms);
+    // The share of the SMs (1..all) of a grid stepped next to others of `total` cells in all
+    int sweep_share(double total) const;
     int sweep_rows = 2;  // cell rows of a thread's patch in the blocked kernel (2 or 4)
     // reference scheme: 0 = one colour pass per launch (k_project_velocity); T = 2 or 4 = the
     // temporally blocked velocity sweep, T passes per launch over z-chunks of vsweep_zchunk planes

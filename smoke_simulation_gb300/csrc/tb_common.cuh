@@ -108,6 +108,8 @@ __host__ __device__ inline void sweep_window(int n, int W, int T, int k, int& st
 bool encode_3d(CUtensorMap* m, const void* base, bool is_u8, const Grid& g, int rows);
 // The same with a box box_w elements wide (box_w x element size a multiple of 16 bytes).
 bool encode_3d_box(CUtensorMap* m, const void* base, bool is_u8, const Grid& g, int box_w, int rows);
+// A map over the sweep codes (16 bits per 2 x 2 patch), boxes of box_w x box_h x 1 patches.
+bool encode_codes(CUtensorMap* m, const void* base, const Grid& g, int box_w, int box_h);
 
 }  // namespace tb
 }  // namespace smk
