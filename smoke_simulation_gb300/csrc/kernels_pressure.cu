@@ -224,24 +224,59 @@ __device__ __forceinline__ uint3 vblock(int vb, int nbx, int nby) {
 
 // FP64 |div u| per projectable cell (read only): the max (as IEEE bits) and whether any cell
 // exceeds tol.
+//
+// A cell's FP64 sum costs five passes through a pipe that takes a few lanes per clock and SM, and
+// bound this kernel (3.4 ms at 512^3, where its 13 bytes a cell take 0.26 ms).  Its FP32 sum d is off
+// by at most 5 * 2^-24 of the sum of the six magnitudes (five roundings, each of a partial sum no
+// larger), so a cell whose |d| + 2^-21 * that sum stays below a maximum already found cannot raise
+// it: only the others (a NaN among them) are summed in FP64.  The CTA's threads share the maximum
+// they found, which starts from the other CTAs'.  Four cells of a row per thread where the rows allow.
+__device__ __forceinline__ double div64(float u0, float u1, float v0, float v1, float w0, float w1) {
+    return ((((-(double)u0 + (double)u1) + -(double)v0) + (double)v1) + -(double)w0) + (double)w1;
+}
+
+__device__ __forceinline__ void measure_cell(float u0, float u1, float v0, float v1, float w0, float w1, double& m,
+                                             unsigned long long* shared_max) {
+    const float d = ((((-u0 + u1) + -v0) + v1) + -w0) + w1;
+    const float mag = ((fabsf(u0) + fabsf(u1)) + (fabsf(v0) + fabsf(v1))) + (fabsf(w0) + fabsf(w1));
+    const float found = __double2float_rd(__longlong_as_double((long long)*(volatile unsigned long long*)shared_max));
+    if (fmaf(mag, 0x1p-21f, fabsf(d)) < found) return;
+    const double a = fabs(div64(u0, u1, v0, v1, w0, w1));
+    if (!(a <= m)) {
+        m = a;  // NaN propagates as the largest value
+        atomicMax(shared_max, (unsigned long long)__double_as_longlong(a));
+    }
+}
+
+template <bool VEC>
 __global__ void k_refine_measure(Grid g, const float* u, const float* v, const float* w,
                                  const uint8_t* __restrict__ flags, RefineStatus* rs, double tol, int nbx,
                                  int nby, int nvb) {
+    __shared__ unsigned long long found;
     if (*(volatile int*)&rs->stop) return;
+    if (threadIdx.x == 0 && threadIdx.y == 0) found = *(volatile unsigned long long*)&rs->div_bits;
+    __syncthreads();
     double m = 0.0;
     for (int vb = (int)blockIdx.x; vb < nvb; vb += (int)gridDim.x) {
         const uint3 bid = vblock(vb, nbx, nby);
-        const int x = (int)bid.x * BX + (int)threadIdx.x;
+        const int x = ((int)bid.x * BX + (int)threadIdx.x) * (VEC ? 4 : 1);
         const int y = (int)bid.y * BY + (int)threadIdx.y;
         const int z = (int)bid.z;
-        if (x < g.nx && y < g.ny && z < g.nz) {
-            const int i = g.idx(x, y, z);
-            if (flags[i] & F_PROJ) {
-                const double d = ((((-(double)u[i] + (double)u[i + 1]) + -(double)v[i]) + (double)v[i + g.X]) +
-                                  -(double)w[i]) + (double)w[i + g.XY];
-                const double a = fabs(d);
-                if (!(a <= m)) m = a;  // NaN propagates as the largest value
-            }
+        if (x >= g.nx || y >= g.ny || z >= g.nz) continue;
+        const int i = g.idx(x, y, z);
+        if (VEC) {
+            // a row holds at least nx + 1 elements and starts on 16 bytes: the group's loads stay in it
+            const uchar4 f = *reinterpret_cast<const uchar4*>(flags + i);
+            if (!((f.x | f.y | f.z | f.w) & F_PROJ)) continue;
+            const float4 ua = *reinterpret_cast<const float4*>(u + i);
+            const float4 va = *reinterpret_cast<const float4*>(v + i), vb4 = *reinterpret_cast<const float4*>(v + i + g.X);
+            const float4 wa = *reinterpret_cast<const float4*>(w + i), wb = *reinterpret_cast<const float4*>(w + i + g.XY);
+            if (f.x & F_PROJ) measure_cell(ua.x, ua.y, va.x, vb4.x, wa.x, wb.x, m, &found);
+            if (f.y & F_PROJ) measure_cell(ua.y, ua.z, va.y, vb4.y, wa.y, wb.y, m, &found);
+            if (f.z & F_PROJ) measure_cell(ua.z, ua.w, va.z, vb4.z, wa.z, wb.z, m, &found);
+            if (f.w & F_PROJ) measure_cell(ua.w, u[i + 4], va.w, vb4.w, wa.w, wb.w, m, &found);
+        } else if (flags[i] & F_PROJ) {
+            measure_cell(u[i], u[i + 1], v[i], v[i + g.X], w[i], w[i + g.XY], m, &found);
         }
     }
     // one flag store and at most one atomic per CTA, each only when it changes the stored value
@@ -358,8 +393,19 @@ void launch_refine(const Grid& g, float* u, float* v, float* w, Tv* us, Tv* vs, 
     const int sbx = (int)sw.x, sby = (int)sw.y, snv = sbx * sby * (int)sw.z;
     const dim3 fc = grid3(g.nx - 1, g.ny - 1, g.nz - 1);
     const int fbx = (int)fc.x, fby = (int)fc.y, fnv = fbx * fby * (int)fc.z;
+    // the groups of four cells of a row's end read u up to x = nx + 3 at most: inside the pitch of
+    // every grid of the library's own layout (vec4_layout), whose rows are a multiple of 16
+    const bool vec = vec4_layout(g, {u, v, w}, flags);
+    const dim3 quads = grid3((g.nx + 3) / 4, g.ny, g.nz);
+    const int qnv = (int)(quads.x * quads.y * quads.z);
+    auto measure = [&] {
+        if (vec)
+            k_refine_measure<true><<<grid_of(qnv), blk, 0, st>>>(g, u, v, w, flags, rs, tol, (int)quads.x, (int)quads.y, qnv);
+        else
+            k_refine_measure<false><<<grid_of(cnv), blk, 0, st>>>(g, u, v, w, flags, rs, tol, cbx, cby, cnv);
+    };
     k_refine_reset<<<1, 1, 0, st>>>(rs, 1);
-    k_refine_measure<<<grid_of(cnv), blk, 0, st>>>(g, u, v, w, flags, rs, tol, cbx, cby, cnv);
+    measure();
     k_refine_decide<<<1, 1, 0, st>>>(rs);
     *launches += 3;
     for (int r = 0; r < rounds; ++r) {
@@ -370,7 +416,7 @@ void launch_refine(const Grid& g, float* u, float* v, float* w, Tv* us, Tv* vs, 
         k_refine_apply<Tv><<<grid_of(fnv), blk, 0, st>>>(g, u, v, w, us, vs, ws, P0, P1, pcur, flags, rs, fbx, fby,
                                                          fnv);
         k_refine_reset<<<1, 1, 0, st>>>(rs, 0);
-        k_refine_measure<<<grid_of(cnv), blk, 0, st>>>(g, u, v, w, flags, rs, tol, cbx, cby, cnv);
+        measure();
         k_refine_decide<<<1, 1, 0, st>>>(rs);
         *launches += 2 * sweeps + 5;
     }
