@@ -383,7 +383,7 @@ const char* smk_server_last_error(void);
  * solver SMK_SOLVER_RBSOR, refine 0; warm_start is ignored) with params->max_sweeps, omega
  * (0 < omega < 2), tol and check_every; the result equals, bit for bit, the projection that
  * smk_step's PRESSURE scheme applies to the same field and mask from a zero pressure.  Scratch comes from one fixed device array inside the
- * library (about 19 MB, held by every GPU that loads the library until exit): grids with
+ * library (about 28 MB, held by every GPU that loads the library until exit): grids with
  * (nx+1)(ny+1)(nz+1) > 2,097,152 or nz > 65535 are rejected with SMK_ERR_INVALID.  All calls
  * share that array and find the previous call's contents in it (each call rewrites what it
  * reads): calls that overlap on the GPU race; order them on one stream.  The first call on a

@@ -485,10 +485,16 @@ int grouped_step(smk_batch* b, const float* dts, float dt_all, cudaStream_t st) 
 struct BranchShapes {
     std::vector<smk_sim*> sims;
     std::vector<std::pair<int, int>> kept;  // depth, z-chunk
+    std::vector<smk_sim*> resident;
     explicit BranchShapes(const smk_batch* b) {
         for (size_t i = 0; i < b->sims.size(); ++i) {
             smk_sim* s = b->sims[i];
-            if (s->sweep_set || b->sims.size() < 2) continue;
+            if (b->sims.size() < 2) continue;
+            if (s->resident_ok) {
+                resident.push_back(s);
+                s->resident_ok = false;
+            }
+            if (s->sweep_set) continue;
             sims.push_back(s);
             kept.emplace_back(s->sweep_depth, s->sweep_zchunk);
             s->sweep_depth = b->branch_shape[i].first;
@@ -500,6 +506,7 @@ struct BranchShapes {
             sims[i]->sweep_depth = kept[i].first;
             sims[i]->sweep_zchunk = kept[i].second;
         }
+        for (smk_sim* s : resident) s->resident_ok = true;
     }
 };
 

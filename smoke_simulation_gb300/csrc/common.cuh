@@ -78,6 +78,14 @@ struct RefineStatus {
     int pad;
 };
 
+// Whole solves with the iterate resident in shared memory (kernels_resident.cu): boxes of by x bz rows of
+// the interior, cy x cz of them, one CTA each, all resident.
+struct ResidentPlan {
+    int by, bz, cy, cz;
+    int hx, hp;  // cells of one colour in a row; elements of a colour row
+    int rt, ns;  // threads, and cells of one colour per thread
+};
+
 // Object records (the reference's packing, smokeSimulation.cu:719-725, :750-758).
 struct SphereObj { float x, y, z, r; };
 struct ObstacleObj { float x, y, z, vx, vy, vz, r; };
@@ -106,6 +114,17 @@ __device__ __forceinline__ void block_max_to(unsigned v, unsigned* dst) {
         if (lane == 0 && w > *(volatile unsigned*)dst) atomicMax(dst, w);
     }
     __syncthreads();
+}
+
+// Whether `kernel` already has `bytes` of dynamic shared memory on this device (the attribute belongs to
+// the context: a reset takes it away): the last of a family of kernels that are set together.
+inline bool smem_attribute_set(const void* kernel, int bytes) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.maxDynamicSharedSizeBytes >= bytes;
 }
 
 // ---- storage types ----------------------------------------------------------------------------

@@ -130,4 +130,56 @@ __host__ __device__ __forceinline__ float pt_grid(float x, int d, float zh, floa
 
 __host__ __device__ __forceinline__ float scale_exact(float q, double omega) { return (float)((double)q * omega); }
 
+#ifdef __CUDACC__
+// A cell that the common path does not decide (es_rare, or the rounding test): zh, zl as in its table
+// entry, pt the common path's value, kept where `rare` is not set; ofs holds the cell's six neighbour bits
+// (8..13) and its projectable bit (14).  pt_scaled, pt_grid, then FP64
+// (exact_scale.cuh; zh + zl stands for 1/acc, whose 2^-48 the correction by the exact remainder makes up
+// for).  The FP64 part is one block of PTX: as plain code the compiler evaluates it for every lane
+// and selects, which puts the FP64 instructions on every cell.
+constexpr unsigned ES_ENTRY_PROJ = 1u << 14;
+static __device__ __noinline__ float cell_pt_rare(float pt, bool rare, float x, unsigned ofs, float zh, float zl,
+                                             const OmegaSplit& os, double omega) {
+    rare = rare && (ofs & ES_ENTRY_PROJ);
+    const int acc = max(__popc((ofs >> 8) & 63u), 1);
+    bool ok;
+    const bool tiny = rare && fabsf(x) < ES_TINY;
+    const float ps = pt_scaled(x, zh, zl, os, ok);
+    if (tiny && ok) pt = ps;
+    rare = rare && !(tiny && ok);
+    if (!__any_sync(0xffffffffu, rare)) return pt;
+    const float pg = pt_grid(x, acc, zh, zl, os, ok);
+    if (rare && ok) pt = pg;
+    const bool left = rare && !ok;
+    if (!__any_sync(0xffffffffu, left)) return pt;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred mine, fin;\n\t"
+        ".reg .f32 ax, r;\n\t"
+        ".reg .f64 X, d, i, y, c, e;\n\t"
+        "setp.ne.u32 mine, %1, 0;\n\t"
+        "cvt.rn.f64.u32 d, %3;\n\t"
+        "cvt.f64.f32 i, %5;\n\t"
+        "cvt.f64.f32 e, %6;\n\t"
+        "add.rn.f64 i, i, e;\n\t"
+        "cvt.f64.f32 X, %2;\n\t"
+        "mul.rn.f64 y, X, i;\n\t"
+        "neg.f64 c, y;\n\t"
+        "fma.rn.f64 e, c, d, X;\n\t"
+        "fma.rn.f64 c, e, i, y;\n\t"
+        "abs.f32 ax, %2;\n\t"
+        "setp.lt.f32 fin, ax, 0f7f800000;\n\t"
+        "selp.f64 y, c, y, fin;\n\t"
+        "cvt.rn.f32.f64 r, y;\n\t"
+        "cvt.f64.f32 y, r;\n\t"
+        "mul.rn.f64 y, y, %4;\n\t"
+        "cvt.rn.f32.f64 r, y;\n\t"
+        "selp.f32 %0, r, %0, mine;\n\t"
+        "}"
+        : "+f"(pt)
+        : "r"((unsigned)left), "f"(x), "r"(acc), "d"(omega), "f"(zh), "f"(zl));
+    return pt;
+}
+#endif
+
 }  // namespace smk

@@ -177,6 +177,19 @@ void destroy_vsweep_maps(VSweepMaps* m);
 int launch_vsweep_tb(const VSweepMaps* m, const Grid& g, int buf, bool from_state, float* uo, float* vo, float* wo,
                      int T, int nhalf, int colour0, int zchunk, double omega, const OmegaSplit& os, int* kerr,
                      cudaStream_t st);
+// Whole solves with the iterate resident in shared memory (kernels_resident.cu; ResidentPlan).
+// The plan of a grid for at most `sms` CTAs; false when it does not fit.
+bool resident_plan(const Grid& g, bool velocity, int sms, ResidentPlan* out);
+// The exchange buffer (device, 8-byte aligned), all zero before every launch.
+size_t resident_exchange_bytes(const ResidentPlan& p);
+int prepare_resident_kernels();
+// Red-black SOR on P in place, max_sweeps sweeps or until the tolerance rule ends it (tol > 0).
+int launch_resident_sor(const Grid& g, const ResidentPlan& p, void* ex, int* kerr, float* P, const float* b,
+                        const uint8_t* flags, const float* wacc7, int max_sweeps, int check_every, float tol,
+                        StepStatus* status, cudaStream_t st);
+// The reference scheme's red-black passes on u, v, w in place.
+int launch_resident_vel(const Grid& g, const ResidentPlan& p, void* ex, int* kerr, float* u, float* v, float* w,
+                        const uint8_t* flags, int iterations, double omega, cudaStream_t st);
 void launch_div_max(const Grid& g, const float* u, const float* v, const float* w,
                     const uint8_t* flags, StepStatus* status, cudaStream_t st);
 // FP64-checked refinement rounds after the projection (u, v, w: the FP32 projected velocity;

@@ -1333,15 +1333,17 @@ int sweep_ycluster_usable(const Grid& g, int n_req) {
 }
 
 int prepare_sweep_kernels() {
+    if (smem_attribute_set((const void*)k_sweep_tb_ycl<YCL_DEPTH>, (int)tb_smem_bytes<YCL_DEPTH, 2>())) return 0;
     const cudaFuncAttribute gattr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const int gb = (int)pair_smem_bytes<GROUP_TB_DEPTH>();
     const int grouped = (cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, false, -1>, gattr, gb) == cudaSuccess &&
                          cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, true, 0>, gattr, gb) == cudaSuccess &&
                          cudaFuncSetAttribute(k_group_sweep_tb<GROUP_TB_DEPTH, true, 1>, gattr, gb) == cudaSuccess)
                             ? 0 : -1;
+    const int others = configure_pair<2>() | configure_pair<4>() | configure_pair<6>() | configure_tb<4, 4>() | grouped;
     const int ycl = cudaFuncSetAttribute(k_sweep_tb_ycl<YCL_DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tb_smem_bytes<YCL_DEPTH, 2>()) == cudaSuccess ? 0 : -1;
-    return configure_pair<2>() | configure_pair<4>() | configure_pair<6>() | configure_tb<4, 4>() | grouped | ycl;
+    return others | ycl;
 }
 
 // Tensor maps for the sweep's TMA loads: P_a, P_b, b (float) for boxes of 32, 48 and 64 rows, the

@@ -123,54 +123,6 @@ __device__ __forceinline__ void closed_upper(unsigned c, unsigned bit, float p, 
 // What an upper face held by another thread receives: p_t * s, or -0 from a cell that is not projectable.
 __device__ __forceinline__ float face_sent(unsigned c, unsigned bit, float pu) { return (c & bit) ? pu : pu * 0.0f; }
 
-// A cell that the common path does not decide (es_rare, or the rounding test): zh, zl as in its table
-// entry, pt the common path's value, kept where `rare` is not set.  pt_scaled, pt_grid, then FP64
-// (exact_scale.cuh; zh + zl stands for 1/acc, whose 2^-48 the correction by the exact remainder makes up
-// for).  The FP64 part is one block of PTX: as plain code the compiler evaluates it for every lane
-// and selects, which puts the FP64 instructions on every cell.
-__device__ __noinline__ float cell_pt_rare(float pt, bool rare, float x, unsigned ofs, float zh, float zl,
-                                             const OmegaSplit& os, double omega) {
-    rare = rare && (ofs & C_PROJ);
-    const int acc = max(__popc((ofs >> 8) & 63u), 1);
-    bool ok;
-    const bool tiny = rare && fabsf(x) < ES_TINY;
-    const float ps = pt_scaled(x, zh, zl, os, ok);
-    if (tiny && ok) pt = ps;
-    rare = rare && !(tiny && ok);
-    if (!__any_sync(0xffffffffu, rare)) return pt;
-    const float pg = pt_grid(x, acc, zh, zl, os, ok);
-    if (rare && ok) pt = pg;
-    const bool left = rare && !ok;
-    if (!__any_sync(0xffffffffu, left)) return pt;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred mine, fin;\n\t"
-        ".reg .f32 ax, r;\n\t"
-        ".reg .f64 X, d, i, y, c, e;\n\t"
-        "setp.ne.u32 mine, %1, 0;\n\t"
-        "cvt.rn.f64.u32 d, %3;\n\t"
-        "cvt.f64.f32 i, %5;\n\t"
-        "cvt.f64.f32 e, %6;\n\t"
-        "add.rn.f64 i, i, e;\n\t"
-        "cvt.f64.f32 X, %2;\n\t"
-        "mul.rn.f64 y, X, i;\n\t"
-        "neg.f64 c, y;\n\t"
-        "fma.rn.f64 e, c, d, X;\n\t"
-        "fma.rn.f64 c, e, i, y;\n\t"
-        "abs.f32 ax, %2;\n\t"
-        "setp.lt.f32 fin, ax, 0f7f800000;\n\t"
-        "selp.f64 y, c, y, fin;\n\t"
-        "cvt.rn.f32.f64 r, y;\n\t"
-        "cvt.f64.f32 y, r;\n\t"
-        "mul.rn.f64 y, y, %4;\n\t"
-        "cvt.rn.f32.f64 r, y;\n\t"
-        "selp.f32 %0, r, %0, mine;\n\t"
-        "}"
-        : "+f"(pt)
-        : "r"((unsigned)left), "f"(x), "r"(acc), "d"(omega), "f"(zh), "f"(zl));
-    return pt;
-}
-
 // One tile of a launch: T colour passes (nhalf of them when not FULL) starting at colour0.
 //
 // A thread's 2 x 2 patch is held as two pairs per field, E = (A0, B1) and O = (B0, A1): one
@@ -494,6 +446,7 @@ int vsweep_depth_supported(int T) { return T == 2 || T == 4; }
 int vsweep_tile_rows(int T) { return 2 * vt_ty(T); }
 
 int prepare_vsweep_kernels() {
+    if (smem_attribute_set((const void*)k_vsweep_tb<4, 16, true>, (int)vt_smem_bytes<4, 16>())) return 0;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const bool ok =
         cudaFuncSetAttribute(k_vsweep_tb<2, 24, true>, a, (int)vt_smem_bytes<2, 24>()) == cudaSuccess &&

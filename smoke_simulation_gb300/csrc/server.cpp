@@ -80,8 +80,10 @@ struct TickRec {
 size_t footprint(int nx, int ny, int nz) {
     const size_t X = ((size_t)nx + 1 + 15) / 16 * 16;
     const size_t elems = X * (size_t)(ny + 1) * (size_t)(nz + 1);
-    // 11 float fields, mask and flags, half a byte of sweep code (a 16-bit code per 2 x 2 patch)
-    return elems * (11 * sizeof(float) + 3) + (1u << 20);
+    // 11 float fields, mask and flags, half a byte of sweep code (a 16-bit code per 2 x 2 patch), the
+    // resident solves' exchange buffer
+    const smk::Grid g{nx, ny, nz, (int)X, (int)(X * (size_t)(ny + 1))};
+    return elems * (11 * sizeof(float) + 3) + smk_sim::exchange_bytes_of(g) + (1u << 20);
 }
 
 }  // namespace
@@ -314,6 +316,7 @@ static int admit(smk_server* s, Request* r) {
         for (const Request* q : s->active) total += (double)q->nx * q->ny * q->nz;
         for (const Request* q : s->queue) total += (double)q->nx * q->ny * q->nz;
         r->sim->choose_sweep(r->sim->sweep_share(total));
+        r->sim->resident_ok = false;
     }
     if (rc == SMK_OK) rc = smk_set_graph_loops(r->sim, s->graph_loops);
     if (rc == SMK_OK && !r->mask.empty()) rc = smk_set_solid_mask(r->sim, r->mask.data());

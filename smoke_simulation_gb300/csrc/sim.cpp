@@ -185,10 +185,11 @@ int smk_sim::alloc() {
     SMK_CUDA(cudaMalloc((void**)&refine, sizeof(RefineStatus)));
     SMK_CUDA(cudaMemset(refine, 0, sizeof(RefineStatus)));
     SMK_CUDA(cudaMalloc((void**)&s, n));
-    SMK_CUDA(cudaMalloc((void**)&flags, n));
-    SMK_CUDA(cudaMemset(flags, 0, n));
-    SMK_CUDA(cudaMalloc((void**)&codes, sweep_code_count(g) * sizeof(uint16_t)));
-    SMK_CUDA(cudaMemset(codes, 0, sweep_code_count(g) * sizeof(uint16_t)));
+    // flags and sweep codes in one allocation
+    const size_t flag_bytes = (n + 255) / 256 * 256, code_bytes = sweep_code_count(g) * sizeof(uint16_t);
+    SMK_CUDA(cudaMalloc((void**)&flags, flag_bytes + code_bytes));
+    SMK_CUDA(cudaMemset(flags, 0, flag_bytes + code_bytes));
+    codes = reinterpret_cast<uint16_t*>(flags + flag_bytes);
     // the tensor maps capture the buffer addresses: every buffer must exist first
     maps = create_sweep_maps(g, P, P2, b, flags, codes);
     if (!maps) return fail(SMK_ERR_CUDA, "could not encode the TMA tensor maps of the sweep kernel");
@@ -214,8 +215,11 @@ int smk_sim::alloc() {
     if (!amaps) return fail(SMK_ERR_CUDA, "could not encode the TMA tensor maps of the velocity advection");
     choose_sweep(device_sms());
     status_groups = 4096;
-    SMK_CUDA(cudaMalloc((void**)&status, sizeof(StepStatus) + sizeof(unsigned) * status_groups));
-    SMK_CUDA(cudaMemset(status, 0, sizeof(StepStatus) + sizeof(unsigned) * status_groups));
+    choose_resident();
+    const size_t status_bytes = (sizeof(StepStatus) + sizeof(unsigned) * status_groups + 255) / 256 * 256;
+    SMK_CUDA(cudaMalloc((void**)&status, status_bytes + exchange_bytes));
+    SMK_CUDA(cudaMemset(status, 0, status_bytes + exchange_bytes));
+    exchange = reinterpret_cast<unsigned char*>(status) + status_bytes;
     SMK_CUDA(cudaMalloc((void**)&tune_status, sizeof(StepStatus) + sizeof(unsigned)));
     for (auto& e : ev) SMK_CUDA(cudaEventCreate(&e));
     SMK_CUDA(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
@@ -223,7 +227,7 @@ int smk_sim::alloc() {
     SMK_CUDA(cudaStreamCreateWithFlags(&rb_stream, cudaStreamNonBlocking));
     SMK_CUDA(cudaEventCreateWithFlags(&rb_fork, cudaEventDisableTiming));
     SMK_CUDA(cudaEventCreateWithFlags(&rb_join, cudaEventDisableTiming));
-    if (prepare_sweep_kernels() != 0 || prepare_vsweep_kernels() != 0)
+    if (prepare_sweep_kernels() != 0 || prepare_vsweep_kernels() != 0 || prepare_resident_kernels() != 0)
         return fail(SMK_ERR_CUDA, "sweep kernel configuration failed");
     // initializeVolume's mask: fluid except the y = 0 floor (smokeSimulation.cu:200-207)
     std::vector<uint8_t> host((size_t)g.nx * g.ny * g.nz, 1);
@@ -246,7 +250,6 @@ void smk_sim::release() {
     if (amaps) destroy_advect_maps(amaps);
     if (s) cudaFree(s);
     if (flags) cudaFree(flags);
-    if (codes) cudaFree(codes);
     if (status) cudaFree(status);
     if (tune_status) cudaFree(tune_status);
     for (auto& e : ev)
@@ -336,12 +339,19 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     if (timed) SMK_CUDA(rec(ev[2]));
 
     // c/d: projection (:795-801)
+    const bool resident = p.projection == SMK_PROJECT_REFERENCE ? resident_velocity() : resident_pressure();
     const size_t status_bytes = sizeof(StepStatus) + sizeof(unsigned) * status_groups;
-    SMK_CUDA(cudaMemsetAsync(status, 0, status_bytes, st));
+    SMK_CUDA(cudaMemsetAsync(status, 0,
+                             resident ? (size_t)(exchange - reinterpret_cast<unsigned char*>(status)) + exchange_bytes
+                                      : status_bytes, st));
     last_groups = 0;
     if (p.projection == SMK_PROJECT_REFERENCE) {
         const VelocitySweep vs = velocity_sweep();
-        if (vs.depth > 0) {
+        if (resident) {
+            if (launch_resident_vel(g, res_v, exchange, kerr, u[now], v[now], w[now], flags, p.max_sweeps, p.omega, st) != 0)
+                return fail(SMK_ERR_CUDA, "resident projection launch failed");
+            ++launches;
+        } else if (vs.depth > 0) {
             // temporally blocked: launches of up to T colour passes alternating between the state
             // (u, v, w)[now] and the scratch arrays (P, P2, b), an even number of them so that the
             // result ends in the state; the passes are those of the loop below, in the same order
@@ -422,6 +432,12 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
                 }
                 ++group;
             }
+        } else if (resident) {
+            if (launch_resident_sor(g, res_p, exchange, kerr, P, b, flags, wacc, p.max_sweeps, G, use_tol ? p.tol : 0.0f,
+                                    status, st) != 0)
+                return fail(SMK_ERR_CUDA, "resident solve launch failed");
+            ++launches;
+            group = use_tol ? (p.max_sweeps + G - 1) / G : 1;
         } else if (sweep_depth > 0) {
             // temporally blocked: each launch applies up to sweep_depth colour passes,
             // ping-ponging P <-> P2; group starts are the check launches, and a launch of fewer
@@ -531,7 +547,7 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
         last_groups = group;
         if (timed) SMK_CUDA(rec(ev[6]));
         // the blocked and Jacobi solves record where the pressure is; the colour passes keep it in P
-        const bool pcur_set = (sweep_depth > 0 || p.solver == SMK_SOLVER_JACOBI) && p.max_sweeps > 0;
+        const bool pcur_set = !resident && (sweep_depth > 0 || p.solver == SMK_SOLVER_JACOBI) && p.max_sweeps > 0;
         if (!pcur_set) SMK_CUDA(cudaMemsetAsync(pcur, 0, sizeof(int), st));
         if (bf16) {
             launch_project_bf16(g, bf(u[now]), bf(v[now]), bf(w[now]), P, P2, pcur, flags, proj[0], proj[1],
@@ -650,6 +666,25 @@ void smk_sim::choose_sweep(int sms) {
     sweep_rows = 2;
 }
 
+// Every grid with a plan takes it (up to about 128^3; us per 30 sweeps or iterations, one pass per launch /
+// blocked / resident).  Velocity form: 32^3 113 / - / 66, 64^3 155 / - / 82, 80^3 261 / - / 129, 100^3 380 /
+// 369 / 234, 127^3 552 / 592 / 369.  Pressure form with a check every 6 sweeps: 32^3 155 / 208 / 87, 64^3
+// 275 / 205 / 96, 100^3 648 / 238 / 162, 127^3 978 / 286 / 265; without checks 127^3 308 / 242 / 228.
+void smk_sim::choose_resident() {
+    const int sms = device_sms();
+    res_p_fits = resident_plan(g, false, sms, &res_p);
+    res_v_fits = !bf16 && resident_plan(g, true, sms, &res_v);
+    exchange_bytes = std::max(res_p_fits ? resident_exchange_bytes(res_p) : 0, res_v_fits ? resident_exchange_bytes(res_v) : 0);
+}
+
+size_t smk_sim::exchange_bytes_of(const Grid& g) {
+    ResidentPlan a;
+    size_t n = 0;
+    for (bool velocity : {false, true})
+        if (resident_plan(g, velocity, device_sms(), &a)) n = std::max(n, resident_exchange_bytes(a));
+    return n;
+}
+
 // In proportion to its cells, and at least one SM per 40,000: with more concurrent grids than that,
 // chunks longer than its march needs would only keep its own chain of launches waiting (48-request
 // stream: 40,000 cells an SM 688 ms, 80,000 695, 160,000 783, 20,000 790, the whole chip for every
@@ -713,6 +748,8 @@ std::string smk_sim::graph_signature(float dt) const {
     const char kh = keeps_history() ? 1 : 0;
     put(&ea, sizeof(ea));
     put(&kh, 1);
+    const char res = (p.projection == SMK_PROJECT_REFERENCE ? resident_velocity() : resident_pressure()) ? 1 : 0;
+    put(&res, 1);
     put(&sweep_depth, sizeof(sweep_depth));
     put(&sweep_zchunk, sizeof(sweep_zchunk));
     put(&sweep_rows, sizeof(sweep_rows));
@@ -1345,7 +1382,7 @@ int smk_get_sweep_shape(const smk_sim* sim, int* depth, int* rows, int* zchunk) 
 namespace {
 std::mutex g_tune_mutex;
 // key: device, grid shape, tolerance group size (0 = no tolerance)
-struct TunedShape { int depth, rows, zchunk; };
+struct TunedShape { int depth, rows, zchunk; bool resident; };
 std::map<std::tuple<int, int, int, int, int>, TunedShape> g_tune_cache;
 }  // namespace
 
@@ -1366,6 +1403,7 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
             sim->set_velocity_sweep(sim->vmaps ? it->second.depth : 0, it->second.zchunk);
+            sim->vsweep_set = !it->second.resident;
             if (depth_out) *depth_out = sim->vsweep_chosen.depth;
             if (zchunk_out) *zchunk_out = it->second.zchunk;
             if (us_out) *us_out = -1.0f;
@@ -1380,10 +1418,18 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
     SMK_CUDA(cudaEventCreate(&e1));
     const int now = sim->index_now;
     const OmegaSplit os = omega_split(sim->p.omega);
+    constexpr int RESIDENT = -1;  // the resident solve, where the grid has one
     // microseconds per iteration of one candidate, issued as a step issues it
     auto time_it = [&](int depth, int zc, float* us) -> int {
         const int iters = 4;
         auto run = [&]() -> int {
+            if (depth == RESIDENT) {
+                SMK_CUDA(cudaMemsetAsync(sim->exchange, 0, sim->exchange_bytes, st));
+                if (launch_resident_vel(g, sim->res_v, sim->exchange, sim->kerr, sim->P, sim->P2, sim->b, sim->flags, iters,
+                                        sim->p.omega, st) != 0)
+                    return fail(SMK_ERR_CUDA, "resident projection launch failed");
+                return SMK_OK;
+            }
             if (depth == 0) {
                 for (int it = 0; it < iters; ++it) {
                     launch_project_velocity(g, sim->P, sim->P2, sim->b, sim->flags, 0, sim->p.omega, st);
@@ -1416,6 +1462,7 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
         float us;
     };
     std::vector<Cand> cands{Cand{0, 0, 1e30f}};
+    if (sim->res_v_fits) cands.push_back(Cand{RESIDENT, 0, 1e30f});
     const int depths[2] = {2, 4};
     for (int di = 0; di < 2 && sim->vmaps != nullptr; ++di) {
         const int T = depths[di], planes = g.nz + 1;
@@ -1450,10 +1497,13 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
     sim->pressure_clobbered = true;
     int krc = check_kernel_error(sim);
     if (krc) return krc;
+    const bool resident = best_d == RESIDENT;
+    if (resident) best_d = best_z = 0;
     sim->set_velocity_sweep(best_d, best_z);
+    sim->vsweep_set = !resident;
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
-        g_tune_cache[key] = TunedShape{best_d, 2, best_z};
+        g_tune_cache[key] = TunedShape{best_d, 2, best_z, resident};
     }
     if (depth_out) *depth_out = best_d;
     if (zchunk_out) *zchunk_out = best_z;
@@ -1475,7 +1525,7 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
-            sim->sweep_set = true;
+            sim->sweep_set = !it->second.resident;
             sim->sweep_depth = it->second.depth;
             sim->sweep_rows = it->second.rows;
             sim->sweep_zchunk = it->second.zchunk;
@@ -1605,19 +1655,45 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
             best_z = c.zc;
         }
     }
+    // the resident solve, where the grid has one: a group of sweeps as one launch
+    bool resident = false;
+    if (sim->res_p_fits && sim->p.solver == SMK_SOLVER_RBSOR) {
+        float us = 1e30f;
+        for (int round = 0; round < 4; ++round) {  // the first one warms up
+            SMK_CUDA(cudaMemsetAsync(sim->exchange, 0, sim->exchange_bytes, st));
+            SMK_CUDA(cudaMemsetAsync(sim->tune_status, 0, sizeof(StepStatus) + sizeof(unsigned), st));
+            SMK_CUDA(cudaEventRecord(e0, st));
+            // a tolerance no residual meets but zero: the check runs, the sweeps go on
+            if (launch_resident_sor(g, sim->res_p, sim->exchange, sim->kerr, sim->P, sim->b, sim->flags, wacc, G, G,
+                                    use_tol ? 1e-38f : 0.0f, sim->tune_status, st) != 0)
+                return fail(SMK_ERR_CUDA, "resident solve launch failed");
+            SMK_CUDA(cudaEventRecord(e1, st));
+            SMK_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.0f;
+            SMK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            if (round > 0) us = std::min(us, 1e3f * ms / G);
+        }
+        resident = us < best;
+        if (resident) best = us;
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaStreamDestroy(st);
     SMK_CUDA(cudaGetLastError());
     int krc = check_kernel_error(sim);
     if (krc) return krc;
-    sim->sweep_set = true;
+    if (resident) {  // the shape that a server or a batch's branches would use stays the grid's
+        best_d = sim->sweep_depth;
+        best_r = sim->sweep_rows;
+        best_z = sim->sweep_zchunk;
+    }
+    sim->sweep_set = !resident;
     sim->sweep_depth = best_d;
     sim->sweep_rows = best_r;
     sim->sweep_zchunk = best_z;
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
-        g_tune_cache[key] = TunedShape{best_d, best_r, best_z};
+        g_tune_cache[key] = TunedShape{best_d, best_r, best_z, resident};
     }
     if (depth_out) *depth_out = best_d;
     if (zchunk_out) *zchunk_out = best_z;

@@ -79,6 +79,19 @@ struct smk_sim {
     uint8_t* flags = nullptr;
     uint16_t* codes = nullptr;  // sweep codes (launch_build_codes), rebuilt with the flags
     smk::StepStatus* status = nullptr;
+    // Solves resident in shared memory (kernels_resident.cu) of grids where that is the fastest form, while
+    // no sweep was set and the grid is stepped by itself (resident_ok: not by a server or as a batch's
+    // branch, where its CTAs would hold every SM for the whole solve).  Their exchange buffer follows
+    // the status words, so that one memset clears both.
+    smk::ResidentPlan res_p, res_v;
+    bool res_p_fits = false, res_v_fits = false;
+    bool resident_ok = true;
+    unsigned char* exchange = nullptr;
+    size_t exchange_bytes = 0;
+    bool resident_pressure() const {
+        return res_p_fits && resident_ok && !sweep_set && !fuse_subtract && p.solver == SMK_SOLVER_RBSOR && p.max_sweeps > 0;
+    }
+    bool resident_velocity() const { return res_v_fits && resident_ok && !vsweep_set && p.max_sweeps > 0; }
     smk::StepStatus* tune_status = nullptr;  // status of the autotuner's timing launches
     int status_groups = 0;
 
@@ -94,6 +107,8 @@ struct smk_sim {
     int sweep_depth = 4;
     int sweep_zchunk = 47;
     void choose_sweep(int sms);
+    void choose_resident();
+    static size_t exchange_bytes_of(const smk::Grid& g);
     // The share of the SMs (1..all) of a grid stepped next to others of `total` cells in all
     int sweep_share(double total) const;
     int sweep_rows = 2;  // cell rows of a thread's patch in the blocked kernel (2 or 4)
@@ -110,7 +125,7 @@ struct smk_sim {
     VelocitySweep velocity_sweep() const {
         if (vmaps == nullptr || p.max_sweeps <= 0) return VelocitySweep{0, 0, 0};
         if (vsweep_set) return vsweep_chosen;
-        return pressure_used || p.max_sweeps < 4 ? VelocitySweep{0, 0, 0} : vsweep_auto;
+        return pressure_used || p.max_sweeps < 4 || resident_velocity() ? VelocitySweep{0, 0, 0} : vsweep_auto;
     }
     void set_velocity_sweep(int depth, int zchunk);
     // P or P2 may hold a pressure history (a PRESSURE step ran): the sweep picked from the grid then

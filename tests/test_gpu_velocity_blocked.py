@@ -31,19 +31,20 @@ def _special(sc, seed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims,iterations,omega,special", [
-    ((130, 118, 141), 30, 1.9, False),   # 60 passes: fourteen launches of 4 and two of 2
-    ((130, 118, 141), 7, 1.9, True),     # 14 passes: 4, 4, 4, 2
-    ((257, 97, 115), 6, 1.9, True),      # windows along x that end one column past a tile
-    ((113, 145, 121), 5, 1.37123456789, False),  # an over-relaxation without a small denominator
+@pytest.mark.parametrize("dims,iterations,omega,special,depth", [
+    ((130, 118, 141), 30, 1.9, False, 4),   # 60 passes: fourteen launches of 4 and two of 2
+    ((130, 118, 141), 7, 1.9, True, 4),     # 14 passes: 4, 4, 4, 2
+    ((257, 97, 115), 6, 1.9, True, 4),      # windows along x that end one column past a tile
+    ((143, 145, 121), 5, 1.37123456789, False, 4),  # an over-relaxation without a small denominator
+    ((113, 145, 121), 5, 1.37123456789, False, 0),  # resident in shared memory
 ])
-def test_grid_choice_equals_one_pass_per_launch(gpu, dims, iterations, omega, special):
+def test_grid_choice_equals_one_pass_per_launch(gpu, dims, iterations, omega, special, depth):
     sc = S.small_scene(*dims, steps=2, seed=5, iterations=iterations, obstacles=2, omega=omega)
     if special:
         sc.u0, sc.v0, sc.w0 = _special(sc, 8)
     a, b = smk.from_scene(sc), smk.from_scene(sc)
     b.set_velocity_sweep(0)
-    assert a.velocity_sweep()[0] == 4 and b.velocity_sweep()[0] == 0
+    assert a.velocity_sweep()[0] == depth and b.velocity_sweep()[0] == 0
     for k in range(sc.steps):
         a.step(sc.dt)
         b.step(sc.dt)
