@@ -207,7 +207,7 @@ AdvectMaps* create_advect_maps(const Grid& g, const float* const* u, const float
                                int n);
 void destroy_advect_maps(AdvectMaps* m);
 // The velocity advection walks the face planes 1 .. nz - 1 in chunks of
-// advect_velocity_chunk_planes() planes (chunk c: planes 1 + c * that .. ); a launch advects the
+// advect_velocity_chunk_planes(g) planes (chunk c: planes 1 + c * that .. ); a launch advects the
 // chunks [c0, c1) (c1 < 0: through the last).  The density advection's launch covers cells
 // z = 1 + zz for zz in [z0, z1) (z1 < 0: through nz - 2); cell z reads the advected faces of
 // planes z and z + 1.
@@ -215,7 +215,7 @@ template <typename To>
 int launch_advect_velocity_tile(const AdvectMaps* m, int set, const Grid& g, const float* u0, const float* v0,
                                 const float* w0, To* u1, To* v1, To* w1, const uint8_t* flags, float dt, int* kerr,
                                 cudaStream_t st, int c0 = 0, int c1 = -1);
-int advect_velocity_chunk_planes();
+int advect_velocity_chunk_planes(const Grid& g);
 int advect_velocity_chunks(const Grid& g);
 template <typename T, typename Tv>
 void launch_advect_density(const Grid& g, const T* r0, T* r1, const Tv* u1, const Tv* v1, const Tv* w1,

@@ -1,16 +1,21 @@
 // Velocity advection (velocityAdvectionU/V/W, smokeSimulation.cu:527-615) with the velocity
 // planes staged in shared memory by TMA.
 //
-// A CTA of 32 x 8 threads owns a 32 x 8 tile of cells in x-y and a run of AT_ZC consecutive
-// planes, and walks them in ascending z, one cell per thread and plane.  Each plane of u, v
-// and w arrives as a 40 x 10 box (the tile plus one cell on every side, the x origin rounded
+// A CTA of 32 x 8 threads owns a 32 x 16 tile of cells in x-y and a run of consecutive planes, and
+// walks them in ascending z, a thread computing the cells of two rows y and y + 1.  Each plane of u, v
+// and w arrives as a 40 x 18 box (the tile plus one cell on every side, the x origin rounded
 // down to a 16-byte boundary) in a four-slot ring: while plane z is computed, planes z - 1,
 // z and z + 1 are resident and plane z + 2 is in flight.  The three 8-point averages of a cell
-// read planes z - 1 and z at fixed offsets from one shared-memory address; a trilinear sample
-// reads the window when its eight corners lie in planes z - 1 .. z + 1 of the window (every
-// backtrace shorter than one cell does) and global memory otherwise.  The arithmetic is the
-// reference's, term for term (avgU/V/W, sample_ref), so the results are the bits of the
-// per-cell kernel.
+// read planes z - 1 and z at fixed offsets from one shared-memory address.  Where every backtrace of
+// the two cells is shorter than REACH, the eight corners of each sample lie in the window and both
+// cells go through packed arithmetic (sample_pair; without the clamps in tiles that cannot need them);
+// otherwise each cell by itself reads the window or, past it, global memory (sample_win).  The
+// arithmetic is the reference's, term for term (avgU/V/W, sample_ref), so the results are the bits of
+// the per-cell kernel.
+//
+// Instruction issue bounds it (75 % of the slots, 46 % of the warps at 64 registers): 256^3 FP32 took
+// 200 us with one cell a thread and scalar arithmetic (388 instructions a cell, 203 M in all), 162 us now
+// (143 M); its 510 MB would take 75 us at the copy rate.  85 registers and three CTAs an SM: 165 us.
 //
 // Each iteration has one barrier: after it every thread has finished plane z - 1, so thread 0
 // refills the slot of plane z - 2 with plane z + 2.  Waits on the ring's mbarriers are bounded;
@@ -20,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -31,13 +38,13 @@ namespace {
 
 using namespace tb;
 
-constexpr int AT_TX = 32, AT_TY = 8;
+constexpr int AT_TX = 32, AT_TY = 8;          // threads
+constexpr int AT_ROWS = 2 * AT_TY;             // cell rows of the tile: two per thread
 constexpr int AT_W = 40;                  // window columns: x in [x_tile - 4, x_tile + 36)
-constexpr int AT_H = AT_TY + 2;           // window rows: y in [y_tile - 1, y_tile + 9)
-constexpr int AT_PSTR = 416;              // floats per field plane: 40 x 10, padded to 128 bytes
+constexpr int AT_H = AT_ROWS + 2;         // window rows: y in [y_tile - 1, y_tile + 17)
+constexpr int AT_PSTR = 736;              // floats per field plane: 40 x 18, padded to 128 bytes
 constexpr int AT_SLOTS = 4;
 constexpr int AT_BOX_BYTES = AT_W * AT_H * 4;
-constexpr int AT_ZC = 16;                 // planes per CTA
 constexpr int AT_OX = 4;                  // a cell's column in the window = tx + AT_OX
 
 static_assert(AT_PSTR * 4 % 128 == 0 && AT_PSTR >= AT_W * AT_H, "plane stride");
@@ -115,19 +122,102 @@ __device__ __forceinline__ float sample_win(const float* __restrict__ f, const G
     return p0.x + p0.y + p1.x + p1.y + p2.x + p2.y + p3.x + p3.y;
 }
 
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+
+// Multipliers of packed sums: a x 1 and a x -1 with a factor the compiler does not know.  It would
+// contract a packed addition (or a product with a literal 1) with the product before it.
+struct Ones {
+    float2 one, mone;
+};
+
+// The clamp's upper ends n - 1 of the three axes, and the bits of 2^23 + them.
+struct Tops {
+    float x, y, z;
+    int bx, by, bz;
+};
+
+// The same sample for the cells of rows y and y + 1 at once (lane x: row y), for positions at most
+// REACH cells from the cells' own: their corners lie in the window, so there is no fallback.  win: the
+// field's window; fm, fc, fp: where the planes z - 1, z, z + 1 would have the column and row whose floats
+// have no bits set, so that the bits of 2^23 + a column and a row index them; kz: the bits of 2^23 + z.
+// Floors are packed sums with 2^23 rounded down.
+// EDGE: the positions may need the clamp to [1, n - 1].
+template <int HX, int HY, int HZ, bool EDGE>
+__device__ __forceinline__ float2 sample_pair(const float* win, const Tops& top, unsigned fm, unsigned fc, unsigned fp, int kz,
+                                              float2 px, float2 py, float2 pz, const Ones& k) {
+    if (EDGE) {
+        const float mx = top.x, my = top.y, mz = top.z;
+        px = make_float2(fmaxf(fminf(px.x, mx), 1.0f), fmaxf(fminf(px.y, mx), 1.0f));
+        py = make_float2(fmaxf(fminf(py.x, my), 1.0f), fmaxf(fminf(py.y, my), 1.0f));
+        pz = make_float2(fmaxf(fminf(pz.x, mz), 1.0f), fmaxf(fminf(pz.y, mz), 1.0f));
+    }
+    if (HX) px = __fadd2_rn(px, both(-0.5f));
+    if (HY) py = __fadd2_rn(py, both(-0.5f));
+    if (HZ) pz = __fadd2_rn(pz, both(-0.5f));
+    const float2 bx = __fadd2_rd(px, both(8388608.0f)), by = __fadd2_rd(py, both(8388608.0f)),
+                 bz = __fadd2_rd(pz, both(8388608.0f));
+    const float2 x1 = __ffma2_rn(__fadd2_rn(bx, both(-8388608.0f)), k.mone, px);
+    const float2 y1 = __ffma2_rn(__fadd2_rn(by, both(-8388608.0f)), k.mone, py);
+    const float2 z1 = __ffma2_rn(__fadd2_rn(bz, both(-8388608.0f)), k.mone, pz);
+    const float2 x0 = __ffma2_rn(x1, k.mone, both(1.0f)), y0 = __ffma2_rn(y1, k.mone, both(1.0f)),
+                 z0 = __ffma2_rn(z1, k.mone, both(1.0f));
+    float2 a[8];  // corners 000, 100, 010, 110, 001, 101, 011, 111
+    auto corners = [&](float cbx, float cby, float cbz, auto put) {
+        const int jx = __float_as_int(cbx), jy = __float_as_int(cby), jz = __float_as_int(cbz);
+        const unsigned o = (unsigned)jx + AT_W * (unsigned)jy;
+        const bool at = jz == kz;
+        const int l = (int)((at ? fc : fm) + o);
+        int h = (int)((at ? fp : fc) + o), oy = AT_W;
+        bool sx = true;
+        if (EDGE) {  // the upper corner repeats the lower one on a delta-0 axis clamped to the last cell
+            if (!HZ && jz == top.bz) h = l;
+            if (!HY && jy == top.by) oy = 0;
+            if (!HX) sx = jx != top.bx;
+        }
+        const float q0 = win[l], q2 = win[l + oy], q4 = win[h], q6 = win[h + oy];
+        put(0, q0);
+        put(1, sx ? win[l + 1] : q0);
+        put(2, q2);
+        put(3, sx ? win[l + oy + 1] : q2);
+        put(4, q4);
+        put(5, sx ? win[h + 1] : q4);
+        put(6, q6);
+        put(7, sx ? win[h + oy + 1] : q6);
+    };
+    corners(bx.x, by.x, bz.x, [&](int i, float v) { a[i].x = v; });
+    corners(bx.y, by.y, bz.y, [&](int i, float v) { a[i].y = v; });
+    // trilinear_ref, term for term
+    const float2 w00 = __fmul2_rn(x0, y0), w10 = __fmul2_rn(x1, y0), w01 = __fmul2_rn(x0, y1), w11 = __fmul2_rn(x1, y1);
+    float2 s = __fmul2_rn(__fmul2_rn(w00, z0), a[0]);
+    s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w10, z0), a[1]), k.one, s);
+    s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w01, z0), a[2]), k.one, s);
+    s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w11, z0), a[3]), k.one, s);
+    s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w00, z1), a[4]), k.one, s);
+    s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w10, z1), a[5]), k.one, s);
+    s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w01, z1), a[6]), k.one, s);
+    return __ffma2_rn(__fmul2_rn(__fmul2_rn(w11, z1), a[7]), k.one, s);
+}
+
+// max(m, |x|); NaN if either is, so that a NaN never counts as near.
+__device__ __forceinline__ float reach(float m, float x) {
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(x)));
+    return m;
+}
+constexpr float REACH = 0.9f;  // a backtrace of one cell at most, with room for the positions' rounding
+
 template <typename To>
 __global__ void __launch_bounds__(AT_TX * AT_TY, 4)
 k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float* __restrict__ u0,
                        const float* __restrict__ v0, const float* __restrict__ w0, To* __restrict__ u1,
                        To* __restrict__ v1, To* __restrict__ w1, const uint8_t* __restrict__ flags, float dt,
-                       int* kerr, int cz0) {
+                       int* kerr, int cz0, int zc, float one, Tops top) {
     __shared__ alignas(128) float win[AT_SLOTS][3][AT_PSTR];
     __shared__ alignas(8) uint64_t mbar[AT_SLOTS];
     const int tx = (int)threadIdx.x, ty = (int)threadIdx.y;
     const bool leader = tx == 0 && ty == 0;
-    const int xt = (int)blockIdx.x * AT_TX, yt = 1 + (int)blockIdx.y * AT_TY;
-    const int zs = 1 + (cz0 + (int)blockIdx.z) * AT_ZC;
-    const int ze = min(zs + AT_ZC, g.nz);  // planes [zs, ze) are advected; [zs - 1, ze] are read
+    const int xt = (int)blockIdx.x * AT_TX, yt = 1 + (int)blockIdx.y * AT_ROWS;
+    const int zs = 1 + (cz0 + (int)blockIdx.z) * zc;
+    const int ze = min(zs + zc, g.nz);  // planes [zs, ze) are advected; [zs - 1, ze] are read
     const int wx0 = xt - AT_OX, wy0 = yt - 1;
 
     // plane p goes to slot p & 3; its barrier phase counts the slot's earlier uses in this CTA
@@ -148,11 +238,23 @@ k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float
     }
     __syncthreads();
 
-    const int x = xt + tx, y = yt + ty;
-    const bool live = x >= 1 && x < g.nx && y < g.ny;
-    const bool inx = x <= g.nx - 2, iny = y <= g.ny - 2;
-    const int oc = (ty + 1) * AT_W + tx + AT_OX;  // the cell's offset in a window plane
+    const int x = xt + tx, y = yt + 2 * ty;
+    // the faces of row y + r that this thread may advect below the last plane, as flag bits
+    auto may = [&](int r) {
+        const bool live = x >= 1 && x < g.nx && y + r < g.ny, inx = x <= g.nx - 2, iny = y + r <= g.ny - 2;
+        return !live ? 0u : (iny ? F_XM : 0u) | (inx ? F_YM : 0u) | (inx && iny ? F_ZM : 0u);
+    };
+    const unsigned may0 = may(0), may1 = may(1);
+    const uint8_t* fl = flags + g.idx(x, y, zs);  // loaded one plane ahead
+    unsigned f0 = may0 ? fl[0] : 0u, f1 = may1 ? fl[g.X] : 0u;
+    const int oc = (2 * ty + 1) * AT_W + tx + AT_OX;  // row y's offset in a window plane
     const float xf = (float)x, yf = (float)y;
+    const Ones k{both(one), both(-one)};
+    const float2 dt2 = both(dt);
+    const unsigned kxy = 0x4b000000u + (unsigned)wx0 + AT_W * (0x4b000000u + (unsigned)wy0);
+    // no position of this tile's columns and rows leaves [1, n - 1]
+    const bool inner = xt >= 2 && xt + AT_TX <= g.nx - 2 && yt >= 2 && yt + AT_ROWS <= g.ny - 2;
+    const float* wf = &win[0][0][0];
     int issued = min(zs + 1, ze);  // last plane issued (leader)
     int waited = zs - 2;           // last plane this thread has seen complete
     if (mbar_wait(smem_u32(&mbar[(zs - 1) & 3]), parity(zs - 1))) {
@@ -169,63 +271,92 @@ k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float
         } else if (leader && z + 2 <= ze) {
             issue(issued = z + 2);
         }
+        const unsigned in = z <= g.nz - 2 ? F_XM | F_YM | F_ZM : F_ZM;
+        const unsigned m0 = f0 & F_SELF ? f0 & may0 & in : 0u, m1 = f1 & F_SELF ? f1 & may1 & in : 0u;
+        fl += g.XY;
+        if (z + 1 < ze) {
+            if (may0) f0 = fl[0];
+            if (may1) f1 = fl[g.X];
+        }
         if (ok) ok = mbar_wait(smem_u32(&mbar[(z + 1) & 3]), parity(z + 1));
         if (!ok) continue;
         waited = z + 1;
-        if (!live) continue;
+        if (!(m0 | m1)) continue;
         const int i = g.idx(x, y, z);
-        const unsigned f = flags[i];
-        if (!(f & F_SELF)) continue;
-        const bool inz = z <= g.nz - 2;
-        const bool du = iny && inz && (f & F_XM), dv = inx && inz && (f & F_YM), dw = inx && iny && (f & F_ZM);
-        if (!(du || dv || dw)) continue;
-        const float* um = &win[(z - 1) & 3][0][0];
-        const float* uc = &win[z & 3][0][0];
-        const float* up = &win[(z + 1) & 3][0][0];
-        const float* vm = um + AT_PSTR;
-        const float* vc = uc + AT_PSTR;
-        const float* vp = up + AT_PSTR;
-        const float* wm = vm + AT_PSTR;
-        const float* wc = vc + AT_PSTR;
-        const float* wp = vp + AT_PSTR;
-        // avgU/avgV/avgW at this index, in the reference's order (common.cuh)
-        // avgU and avgV as one packed chain of sums (lane x: u, lane y: v), avgW alone
-        const float* a = um + oc;
-        const float* b = uc + oc;
-        const float* c = vm + oc;
-        const float* d = vc + oc;
-        float2 s2 = __fadd2_rn(make_float2(a[0], c[0]), make_float2(a[1], c[-1]));
-        s2 = __fadd2_rn(s2, make_float2(a[-AT_W], c[AT_W]));
-        s2 = __fadd2_rn(s2, make_float2(a[1 - AT_W], c[AT_W - 1]));
-        s2 = __fadd2_rn(s2, make_float2(b[0], d[0]));
-        s2 = __fadd2_rn(s2, make_float2(b[1], d[-1]));
-        s2 = __fadd2_rn(s2, make_float2(b[-AT_W], d[AT_W]));
-        s2 = __fadd2_rn(s2, make_float2(b[1 - AT_W], d[AT_W - 1]));
-        const float au = s2.x / 8.0f, av = s2.y / 8.0f;
-        a = wc + oc;
-        b = wm + oc;
-        const float aw = (a[0] + a[-1] + a[-AT_W] + a[-1 - AT_W] + b[0] + b[-1] + b[-AT_W] + b[-1 - AT_W]) / 8.0f;
+        // planes z - 1, z, z + 1 of u; v and w follow at AT_PSTR and 2 AT_PSTR
+        const int um = ((z - 1) & 3) * 3 * AT_PSTR, uc = (z & 3) * 3 * AT_PSTR, up = ((z + 1) & 3) * 3 * AT_PSTR;
+        auto pair = [&](int o) { return make_float2(wf[o], wf[o + AT_W]); };
+        // avgU/avgV/avgW of both cells, in the reference's order (common.cuh)
+        auto average = [&](int a, int b, int dx, int dy) {
+            float2 s = __fadd2_rn(pair(a), pair(a + dx));
+            s = __fadd2_rn(s, pair(a + dy));
+            s = __fadd2_rn(s, pair(a + dx + dy));
+            s = __fadd2_rn(s, pair(b));
+            s = __fadd2_rn(s, pair(b + dx));
+            s = __fadd2_rn(s, pair(b + dy));
+            s = __fadd2_rn(s, pair(b + dx + dy));
+            return __fmul2_rn(s, both(0.125f));
+        };
+        const int vo = AT_PSTR + oc, wo = 2 * AT_PSTR + oc;
+        const float2 au = average(um + oc, uc + oc, 1, -AT_W);
+        const float2 av = average(um + vo, uc + vo, -1, AT_W);
+        const float2 aw = average(uc + wo, um + wo, -1, -AT_W);
+        const float2 cu = pair(uc + oc), cv = pair(uc + vo), cw = pair(uc + wo);
+        const float2 tu = __fmul2_rn(dt2, au), tv = __fmul2_rn(dt2, av), tw = __fmul2_rn(dt2, aw);
+        const float2 su = __fmul2_rn(dt2, cu), sv = __fmul2_rn(dt2, cv), sw = __fmul2_rn(dt2, cw);
+        float far = fabsf(tu.x);
+        for (float t : {tu.y, tv.x, tv.y, tw.x, tw.y, su.x, su.y, sv.x, sv.y, sw.x, sw.y}) far = reach(far, t);
         const float zf = (float)z;
-        if (du) {
-            float px = xf, py = yf + 0.5f, pz = zf + 0.5f;
-            px = px - dt * uc[oc];
-            py = py - dt * av;
-            pz = pz - dt * aw;
-            stv(u1, i, sample_win<0, 1, 1>(u0, g, um, uc, up, wx0, wy0, z, px, py, pz));
+        if (far <= REACH) {
+            auto near_by = [&](auto edge) {
+                constexpr bool EDGE = decltype(edge)::value;
+                const float2 x2 = both(xf), xh = both(xf + 0.5f), z2 = both(zf), zh = both(zf + 0.5f);
+                const float2 y2 = make_float2(yf, yf + 1.0f), yh = make_float2(yf + 0.5f, yf + 1.5f);
+                const int kz = 0x4b000000 + z;
+                if ((m0 | m1) & F_XM) {
+                    const float2 r = sample_pair<0, 1, 1, EDGE>(wf, top, um - kxy, uc - kxy, up - kxy, kz, __ffma2_rn(su, k.mone, x2),
+                                                                __ffma2_rn(tv, k.mone, yh), __ffma2_rn(tw, k.mone, zh), k);
+                    if (m0 & F_XM) stv(u1, i, r.x);
+                    if (m1 & F_XM) stv(u1, i + g.X, r.y);
+                }
+                if ((m0 | m1) & F_YM) {
+                    const float2 r = sample_pair<1, 0, 1, EDGE>(wf + AT_PSTR, top, um - kxy, uc - kxy, up - kxy, kz,
+                                                                __ffma2_rn(tu, k.mone, xh), __ffma2_rn(sv, k.mone, y2),
+                                                                __ffma2_rn(tw, k.mone, zh), k);
+                    if (m0 & F_YM) stv(v1, i, r.x);
+                    if (m1 & F_YM) stv(v1, i + g.X, r.y);
+                }
+                if ((m0 | m1) & F_ZM) {
+                    const float2 r = sample_pair<1, 1, 0, EDGE>(wf + 2 * AT_PSTR, top, um - kxy, uc - kxy, up - kxy, kz,
+                                                                __ffma2_rn(tu, k.mone, xh), __ffma2_rn(tv, k.mone, yh),
+                                                                __ffma2_rn(sw, k.mone, z2), k);
+                    if (m0 & F_ZM) stv(w1, i, r.x);
+                    if (m1 & F_ZM) stv(w1, i + g.X, r.y);
+                }
+            };
+            if (inner && z >= 2 && z <= g.nz - 3)
+                near_by(std::false_type{});
+            else
+                near_by(std::true_type{});
+            continue;
         }
-        if (dv) {
-            float px = xf + 0.5f, py = yf, pz = zf + 0.5f;
-            px = px - dt * au;
-            py = py - dt * vc[oc];
-            pz = pz - dt * aw;
-            stv(v1, i, sample_win<1, 0, 1>(v0, g, vm, vc, vp, wx0, wy0, z, px, py, pz));
-        }
-        if (dw) {
-            float px = xf + 0.5f, py = yf + 0.5f, pz = zf;
-            px = px - dt * au;
-            py = py - dt * av;
-            pz = pz - dt * wc[oc];
-            stv(w1, i, sample_win<1, 1, 0>(w0, g, wm, wc, wp, wx0, wy0, z, px, py, pz));
+        // a longer backtrace in one of the two cells: each by itself, window or global memory
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            const unsigned m = c ? m1 : m0;
+            const int ic = i + (c ? g.X : 0);
+            const float yc = yf + (float)c;
+            const float du = c ? su.y : su.x, dv = c ? sv.y : sv.x, dw = c ? sw.y : sw.x;
+            const float eu = c ? tu.y : tu.x, ev = c ? tv.y : tv.x, ew = c ? tw.y : tw.x;
+            const float *pm = wf + um, *pc = wf + uc, *pp = wf + up;
+            if (m & F_XM)
+                stv(u1, ic, sample_win<0, 1, 1>(u0, g, pm, pc, pp, wx0, wy0, z, xf - du, yc + 0.5f - ev, zf + 0.5f - ew));
+            if (m & F_YM)
+                stv(v1, ic, sample_win<1, 0, 1>(v0, g, pm + AT_PSTR, pc + AT_PSTR, pp + AT_PSTR, wx0, wy0, z,
+                                                xf + 0.5f - eu, yc - dv, zf + 0.5f - ew));
+            if (m & F_ZM)
+                stv(w1, ic, sample_win<1, 1, 0>(w0, g, pm + 2 * AT_PSTR, pc + 2 * AT_PSTR, pp + 2 * AT_PSTR, wx0, wy0, z,
+                                                xf + 0.5f - eu, yc + 0.5f - ev, zf - dw));
         }
     }
     if (__syncthreads_or(!ok)) {
@@ -239,6 +370,9 @@ k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float
 }
 
 }  // namespace
+
+static int tiles_x(const Grid& g) { return (g.nx + AT_TX - 1) / AT_TX; }
+static int tiles_y(const Grid& g) { return (g.ny - 1 + AT_ROWS - 1) / AT_ROWS; }
 
 struct AdvectMaps {
     AdvMaps set[2];
@@ -274,16 +408,27 @@ int launch_advect_velocity_tile(const AdvectMaps* m, int set, const Grid& g, con
     if (c1 < 0 || c1 > chunks) c1 = chunks;
     if (c0 < 0) c0 = 0;
     if (c1 <= c0) return 0;
-    const dim3 grid((unsigned)((g.nx + AT_TX - 1) / AT_TX), (unsigned)((g.ny - 1 + AT_TY - 1) / AT_TY),
-                    (unsigned)(c1 - c0));
-    k_advect_velocity_tile<To><<<grid, dim3(AT_TX, AT_TY), 0, st>>>(m->set[set], g, u0, v0, w0, u1, v1, w1, flags,
-                                                                     dt, kerr, c0);
+    const dim3 grid((unsigned)tiles_x(g), (unsigned)tiles_y(g), (unsigned)(c1 - c0));
+    const Tops top{(float)(g.nx - 1), (float)(g.ny - 1), (float)(g.nz - 1),
+                   0x4b000000 + g.nx - 1, 0x4b000000 + g.ny - 1, 0x4b000000 + g.nz - 1};
+    k_advect_velocity_tile<To><<<grid, dim3(AT_TX, AT_TY), 0, st>>>(m->set[set], g, u0, v0, w0, u1, v1, w1, flags, dt,
+                                                                     kerr, c0, advect_velocity_chunk_planes(g), 1.0f, top);
     return 0;
 }
 
-int advect_velocity_chunk_planes() { return AT_ZC; }
+// Sixteen planes a chunk read each plane 1.1 times; small grids halve the chunks until two CTAs an SM have
+// work, as a CTA's planes follow one another (32^3, two tiles: both advections take 28 us with two chunks,
+// 12 with thirty-one; 80^3: 11 us less).
+int advect_velocity_chunk_planes(const Grid& g) {
+    int zc = 16;
+    while (zc > 1 && tiles_x(g) * tiles_y(g) * ((g.nz - 1 + zc - 1) / zc) < 304) zc /= 2;
+    return zc;
+}
 
-int advect_velocity_chunks(const Grid& g) { return g.nz < 2 ? 0 : (g.nz - 1 + AT_ZC - 1) / AT_ZC; }
+int advect_velocity_chunks(const Grid& g) {
+    const int zc = advect_velocity_chunk_planes(g);
+    return g.nz < 2 ? 0 : (g.nz - 1 + zc - 1) / zc;
+}
 
 template int launch_advect_velocity_tile<float>(const AdvectMaps*, int, const Grid&, const float*, const float*,
                                                 const float*, float*, float*, float*, const uint8_t*, float, int*,

@@ -583,7 +583,7 @@ int smk_sim::enqueue(float dt, cudaStream_t st) {
     // advects velocity chunks [c0, c1), then the density cells whose faces those chunks
     // finished (cell z reads the faces of planes z and z + 1), and its density planes go to the
     // host on rb_stream while the next slab computes.  Every cell's arithmetic is the same.
-    const int chunks = advect_velocity_chunks(g), chunk_planes = advect_velocity_chunk_planes();
+    const int chunks = advect_velocity_chunks(g), chunk_planes = advect_velocity_chunk_planes(g);
     const int nslab = rb_host ? std::max(1, std::min(readback_slabs(), chunks)) : 1;
     int zz_done = 0, plane_done = 0;
     for (int sl = 0; sl < nslab; ++sl) {
