@@ -261,4 +261,20 @@ __device__ __forceinline__ float ld_eager(const __nv_bfloat16* p) {
     return __bfloat162float(__ushort_as_bfloat16(h));
 }
 
+// Tiles of the density advection: 256 (x, row pair) units of the interior by a run of planes.  The units go
+// through strips of DENSITY_STRIP columns row pair by row pair, without gaps.
+constexpr int DENSITY_THREADS = 256, DENSITY_STRIP = 64;
+__host__ __device__ inline int density_units(const Grid& g) {
+    return g.nx < 3 || g.ny < 3 ? 0 : (g.nx - 2) * ((g.ny - 1) / 2);
+}
+__host__ __device__ inline int density_blocks(const Grid& g) {
+    return (density_units(g) + DENSITY_THREADS - 1) / DENSITY_THREADS;
+}
+__device__ __forceinline__ void density_unit(const Grid& g, int unit, int& x, int& y) {
+    const int pairs = (g.ny - 1) / 2, strip = unit / (DENSITY_STRIP * pairs), left = strip * DENSITY_STRIP;
+    const int wide = min(DENSITY_STRIP, g.nx - 2 - left), r = unit - left * pairs;
+    x = 1 + left + r % wide;
+    y = 1 + 2 * (r / wide);
+}
+
 }  // namespace smk

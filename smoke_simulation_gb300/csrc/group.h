@@ -159,6 +159,7 @@ __host__ __device__ inline void group_extent(int stage, const GroupGrid& d, int&
 
 // Advection tiles walk GROUP_ADV_ZC consecutive planes (as the single-grid advection kernels).
 constexpr int GROUP_ADV_ZC = 4;
+constexpr int GROUP_RHO_ZC = 8;
 
 // 4-wide tiles (grids with vec4): 16 groups of 4 consecutive x by 16 rows of one plane, over
 // gx groups (from x = 0), ry rows and rz planes.
@@ -199,6 +200,7 @@ __host__ __device__ inline int group_tiles(int stage, const GroupGrid& d, int zs
         case GS_ADV_RHO: {
             int rx, ry, rz;
             group_extent(stage, d, rx, ry, rz);
+            if (stage == GS_ADV_RHO) return rz > 0 ? density_blocks(g) * group_div_up(rz, GROUP_RHO_ZC) : 0;
             return group_block_tiles(rx, ry, group_div_up(rz, GROUP_ADV_ZC));
         }
         default: {

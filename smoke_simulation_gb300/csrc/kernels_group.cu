@@ -180,26 +180,25 @@ __global__ void __launch_bounds__(GROUP_TILE, 8) k_group_adv_vel(const GroupArgs
     });
 }
 
-__global__ void __launch_bounds__(GROUP_TILE, 8) k_group_adv_rho(const GroupArgs a) {
+__global__ void __launch_bounds__(GROUP_TILE, 4) k_group_adv_rho(const GroupArgs a, float one) {
     for_tiles(a, GS_ADV_RHO, nullptr, 0, [&](int j, int local) {
         const GroupGrid& d = a.grids[j];
         const Grid gg = d.g;  // in registers: the stores of the body cannot alias it
-        const uint3 bid = tile_bid(local, d.g.nx - 2, d.g.ny - 2);
+        const int blocks = density_blocks(gg), unit = (local % blocks) * DENSITY_THREADS + tid256();
+        if (unit >= density_units(gg)) return;
+        int x, y;
+        density_unit(gg, unit, x, y);
+        const int z0 = 1 + (local / blocks) * GROUP_RHO_ZC, z1 = min(z0 + GROUP_RHO_ZC, gg.nz - 1);
         typedef __nv_bfloat16 h;
-        for (int k = 0; k < GROUP_ADV_ZC; ++k) {
-            const uint3 b = make_uint3(bid.x, bid.y, bid.z * GROUP_ADV_ZC + k);
-            if ((int)b.z >= d.g.nz - 2) break;
-            if (d.kind == GK_BF16)
-                body_advect_density<h, h>(gg, (const h*)d.rho_now, (h*)d.rho_past, (const h*)d.u_past,
-                                          (const h*)d.v_past, (const h*)d.w_past, d.flags, d.dt, b);
-            else if (d.kind == GK_BF16_VEL)
-                body_advect_density<float, h>(gg, (const float*)d.rho_now, (float*)d.rho_past, (const h*)d.u_past,
-                                              (const h*)d.v_past, (const h*)d.w_past, d.flags, d.dt, b);
-            else
-                body_advect_density<float, float>(gg, (const float*)d.rho_now, (float*)d.rho_past,
-                                                  (const float*)d.u_past, (const float*)d.v_past,
-                                                  (const float*)d.w_past, d.flags, d.dt, b);
-        }
+        if (d.kind == GK_BF16)
+            density_rows(gg, (const h*)d.rho_now, (h*)d.rho_past, (const h*)d.u_past, (const h*)d.v_past,
+                         (const h*)d.w_past, d.flags, d.dt, one, x, y, z0, z1);
+        else if (d.kind == GK_BF16_VEL)
+            density_rows(gg, (const float*)d.rho_now, (float*)d.rho_past, (const h*)d.u_past, (const h*)d.v_past,
+                         (const h*)d.w_past, d.flags, d.dt, one, x, y, z0, z1);
+        else
+            density_rows(gg, (const float*)d.rho_now, (float*)d.rho_past, (const float*)d.u_past,
+                         (const float*)d.v_past, (const float*)d.w_past, d.flags, d.dt, one, x, y, z0, z1);
     });
 }
 
@@ -532,7 +531,8 @@ int launch_grid_stride(const void* kernel, int total, int occ, const GroupArgs& 
     if (total <= 0) return 0;
     const int cap = occ * g_sms;
     const int ctas = per_tile || total < cap ? total : cap;
-    void* args[] = {(void*)&a};
+    float one = 1.0f;  // the density advection's second argument
+    void* args[] = {(void*)&a, (void*)&one};
     return (int)cudaLaunchKernel(kernel, dim3((unsigned)ctas), dim3(SB_BX, SB_BY), args, 0, st);
 }
 

@@ -586,29 +586,91 @@ __device__ __forceinline__ void body_advect_velocity(const Grid& g, const Ti* __
 // so it is exact in double unless |b| < a*2^-29; then a - b lies strictly inside a's float
 // rounding interval, in double too.  Either way float(double(a) - double(b)) equals the single-
 // rounded float subtraction, which avoids GB300's slow FP64 pipe (golden-vector tests pin it).
+//
+// A thread computes the cells of two rows y and y + 1 (lane x: row y) for planes z0 <= z < z1 in packed
+// arithmetic and loads the next plane's flags and face velocities before it gathers this plane's corners;
+// the lower w face of a plane is the upper one of the plane before it.  `one` is 1 as a value the
+// compiler does not know: packed sums of products are products with it, as a packed addition (or a product
+// with a literal 1) would be contracted with them.  Floors are packed sums with 2^23 rounded down: after
+// the clamp the positions lie in [0.5, n - 1.5].
 template <typename T, typename Tv>
-__device__ __forceinline__ void body_advect_density(const Grid& g, const T* __restrict__ r0,
-                                                    T* __restrict__ r1, const Tv* __restrict__ u,
-                                                    const Tv* __restrict__ v,
-                                                    const Tv* __restrict__ w,
-                                                    const uint8_t* __restrict__ flags, float dt,
-                                                    uint3 bid) {
-    const int x = 1 + (int)bid.x * SB_BX + (int)threadIdx.x;
-    const int y = 1 + (int)bid.y * SB_BY + (int)threadIdx.y;
-    const int z = 1 + (int)bid.z;
-    if (x > g.nx - 2 || y > g.ny - 2 || z > g.nz - 2) return;
-    const int i = g.idx(x, y, z);
-    // the face velocities are loaded with the flag byte, not after it (ld_eager)
-    const float ua = ld_eager(u + i), ub = ld_eager(u + i + 1), va = ld_eager(v + i),
-                vb = ld_eager(v + i + g.X), wa = ld_eager(w + i), wb = ld_eager(w + i + g.XY);
-    if (!(flags[i] & F_SELF)) return;
-    const float ut = (ua + ub) / 2.0f;
-    const float vt = (va + vb) / 2.0f;
-    const float wt = (wa + wb) / 2.0f;
-    const float xt = __fsub_rn((float)x + 0.5f, ut * dt);
-    const float yt = __fsub_rn((float)y + 0.5f, vt * dt);
-    const float zt = __fsub_rn((float)z + 0.5f, wt * dt);
-    stv(r1, i, sample_ref<1, 1, 1>(r0, g, xt, yt, zt));
+__device__ __forceinline__ void density_rows(const Grid& g, const T* __restrict__ r0, T* __restrict__ r1,
+                                             const Tv* __restrict__ u, const Tv* __restrict__ v,
+                                             const Tv* __restrict__ w, const uint8_t* __restrict__ flags, float dt,
+                                             float one, int x, int y, int z0, int z1) {
+    const bool two = y + 1 <= g.ny - 2;
+    const int dy = two ? g.X : 0;  // a lone last row is computed twice and stored once
+    const float mx = (float)(g.nx - 1), my = (float)(g.ny - 1), mz = (float)(g.nz - 1);
+    auto both = [](float a) { return make_float2(a, a); };
+    const float2 one2 = both(one), mone = both(-one);
+    const float yh = (float)y + 0.5f;
+    const float2 xh2 = both((float)x + 0.5f), yh2 = make_float2(yh, two ? yh + 1.0f : yh);
+    const unsigned base = 0x4b000000u + (unsigned)g.X * 0x4b000000u + (unsigned)g.XY * 0x4b000000u;
+    struct Faces {
+        float2 ua, ub, va, vb, wb;
+        unsigned f0, f1;
+    };
+    auto load = [&](int i) {
+        Faces a;
+        a.ua = make_float2(ld_eager(u + i), ld_eager(u + i + dy));
+        a.ub = make_float2(ld_eager(u + i + 1), ld_eager(u + i + dy + 1));
+        const float vm = ld_eager(v + i + g.X);
+        a.va = make_float2(ld_eager(v + i), two ? vm : ld_eager(v + i));
+        a.vb = make_float2(vm, two ? ld_eager(v + i + 2 * g.X) : vm);
+        a.wb = make_float2(ld_eager(w + i + g.XY), ld_eager(w + i + dy + g.XY));
+        a.f0 = flags[i];
+        a.f1 = flags[i + dy];
+        return a;
+    };
+    int i = g.idx(x, y, z0);
+    float2 wa = make_float2(ld_eager(w + i), ld_eager(w + i + dy));
+    Faces n = load(i);
+    for (int z = z0; z < z1; ++z, i += g.XY) {
+        const Faces a = n;
+        const float2 wl = wa;
+        wa = a.wb;
+        if (z + 1 < z1) n = load(i + g.XY);
+        const bool s0 = a.f0 & F_SELF, s1 = two && (a.f1 & F_SELF);
+        if (!(s0 || s1)) continue;
+        auto back = [&](float2 lo, float2 hi, float2 at) {
+            return __ffma2_rn(__fmul2_rn(__fmul2_rn(__fadd2_rn(lo, hi), both(0.5f)), both(dt)), mone, at);
+        };
+        auto clamp = [&](float2 p, float m) {
+            p = make_float2(fmaxf(fminf(p.x, m), 1.0f), fmaxf(fminf(p.y, m), 1.0f));
+            return __fadd2_rn(p, both(-0.5f));
+        };
+        const float2 px = clamp(back(a.ua, a.ub, xh2), mx), py = clamp(back(a.va, a.vb, yh2), my),
+                     pz = clamp(back(wl, a.wb, both((float)z + 0.5f)), mz);
+        const float2 bx = __fadd2_rd(px, both(8388608.0f)), by = __fadd2_rd(py, both(8388608.0f)),
+                     bz = __fadd2_rd(pz, both(8388608.0f));
+        auto at = [&](float cx, float cy, float cz) {
+            return r0 + (int)(__float_as_uint(cx) + (unsigned)g.X * __float_as_uint(cy) +
+                              (unsigned)g.XY * __float_as_uint(cz) - base);
+        };
+        const T *q = at(bx.x, by.x, bz.x), *t = at(bx.y, by.y, bz.y);
+        const T *qz = q + g.XY, *tz = t + g.XY;
+        const float2 c000 = make_float2(ldv(q, 0), ldv(t, 0)), c100 = make_float2(ldv(q, 1), ldv(t, 1));
+        const float2 c010 = make_float2(ldv(q, g.X), ldv(t, g.X)), c110 = make_float2(ldv(q + g.X, 1), ldv(t + g.X, 1));
+        const float2 c001 = make_float2(ldv(qz, 0), ldv(tz, 0)), c101 = make_float2(ldv(qz, 1), ldv(tz, 1));
+        const float2 c011 = make_float2(ldv(qz, g.X), ldv(tz, g.X)),
+                     c111 = make_float2(ldv(qz + g.X, 1), ldv(tz + g.X, 1));
+        auto part = [&](float2 p, float2 b) { return __ffma2_rn(__fadd2_rn(b, both(-8388608.0f)), mone, p); };
+        const float2 x1 = part(px, bx), y1 = part(py, by), zz1 = part(pz, bz);
+        const float2 x0 = __ffma2_rn(x1, mone, both(1.0f)), y0 = __ffma2_rn(y1, mone, both(1.0f)),
+                     zz0 = __ffma2_rn(zz1, mone, both(1.0f));
+        // trilinear_ref, term for term
+        const float2 w00 = __fmul2_rn(x0, y0), w10 = __fmul2_rn(x1, y0), w01 = __fmul2_rn(x0, y1), w11 = __fmul2_rn(x1, y1);
+        float2 s = __fmul2_rn(__fmul2_rn(w00, zz0), c000);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w10, zz0), c100), one2, s);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w01, zz0), c010), one2, s);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w11, zz0), c110), one2, s);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w00, zz1), c001), one2, s);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w10, zz1), c101), one2, s);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w01, zz1), c011), one2, s);
+        s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w11, zz1), c111), one2, s);
+        if (s0) stv(r1, i, s.x);
+        if (s1) stv(r1, i + g.X, s.y);
+    }
 }
 
 }  // namespace smk

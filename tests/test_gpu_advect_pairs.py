@@ -1,4 +1,4 @@
-"""GPU test of the velocity advection's two-row form: tiles with and without positions at the clamp,
+"""GPU test of the two advections' two-row forms (the density's strips of columns with a lone last row): tiles with and without positions at the clamp,
 backtraces below, around and above the reach of its window within one warp, one-plane chunks up to
 sixteen-plane ones, and velocities that are infinite or NaN, against the restatement of the step."""
 import numpy as np
@@ -23,9 +23,11 @@ def _same(a, b):
     ((66, 35, 11), 0.3, False),     # exactly one tile without clamps
     ((67, 51, 40), 2.5, False),     # near and far backtraces in the same warps
     ((67, 51, 40), 0.89, True),
+    ((131, 6, 12), 1.1, False),     # two full strips and one column more, an even number of rows
+    ((24, 9, 21), 4.0, True),
     ((200, 120, 70), 1.2, True),    # longer chunks
 ])
-def test_velocity_advection_equals_restatement(gpu, dims, reach, special):
+def test_advection_equals_restatement(gpu, dims, reach, special):
     sc = S.small_scene(*dims, steps=2, seed=9, iterations=1, obstacles=1 if min(dims) > 8 else 0, noise=0.0)
     rng = np.random.default_rng(4)
     out = []
