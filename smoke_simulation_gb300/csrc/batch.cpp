@@ -92,6 +92,10 @@ struct TableImage {
     std::vector<int> tb_starts;
     std::vector<int> tb_order;  // member of each record
     size_t off_tb = 0, off_tb_starts = 0, off_tb_counter = 0;
+    // velocity advection: one record per grid (tensor maps, buffers), tile prefix sums per output type
+    std::vector<unsigned char> adv_recs;
+    std::vector<int> adv_starts[2];
+    size_t off_adv = 0, off_adv_starts[2] = {0, 0};
 };
 
 // The blocked solve needs every member to share the tolerance group size and the sweep cap,
@@ -233,6 +237,29 @@ void fill_record(smk_sim* s, float dt, TableImage& t, GroupGrid& d) {
     }
 }
 
+// The velocity advection's records.  Sixteen planes a tile, halved until two CTAs an SM have work (as the
+// single-grid launcher does).
+int fill_advection(smk_sim* const* sims, int n, TableImage& t) {
+    const size_t rb = group_advect_record_bytes();
+    for (int zc = 16;; zc /= 2) {
+        long long acc[2] = {0, 0};
+        t.adv_recs.assign(rb * n, 0);
+        for (auto& s : t.adv_starts) s.assign(n + 1, 0);
+        for (int i = 0; i < n; ++i) {
+            const GroupGrid& d = t.grids[i];
+            const float* in[3] = {d.pu, d.pv, d.pw};
+            void* out[3] = {d.u_past, d.v_past, d.w_past};
+            const int k = d.kind == GK_F32 ? 0 : 1;
+            for (int q = 0; q < 2; ++q) t.adv_starts[q][i] = (int)acc[q];
+            acc[k] += group_advect_fill(&t.adv_recs[rb * i], sims[i]->amaps, k == 0 ? sims[i]->index_now ^ 1 : 0, d.g, in,
+                                        out, d.flags, d.kerr, d.dt, zc);
+            if (acc[k] > INT_MAX / 2) return smk_fail(SMK_ERR_INVALID, "batch too large for one grouped launch");
+        }
+        for (int q = 0; q < 2; ++q) t.adv_starts[q][n] = (int)acc[q];
+        if (zc == 1 || acc[0] + acc[1] >= 304) return SMK_OK;
+    }
+}
+
 int build_table(smk_sim* const* sims, int n, const float* dts, float dt_all, const GroupSchedule& sch,
                 TableImage& t) {
     t.grids.resize(n);
@@ -281,6 +308,8 @@ int build_table(smk_sim* const* sims, int n, const float* dts, float dt_all, con
         }
         t.starts[(size_t)s * (n + 1) + n] = (int)acc;
     }
+    const int arc = fill_advection(sims, n, t);
+    if (arc) return arc;
     size_t off = align_up(sizeof(GroupSync), 256);
     t.off_grids = off;
     off = align_up(off + sizeof(GroupGrid) * n, 256);
@@ -290,6 +319,12 @@ int build_table(smk_sim* const* sims, int n, const float* dts, float dt_all, con
     off = align_up(off + sizeof(BoxObj) * std::max<size_t>(1, t.boxes.size()), 256);
     t.off_spheres = off;
     off = align_up(off + sizeof(SphereObj) * std::max<size_t>(1, t.spheres.size()), 256);
+    t.off_adv = off;  // 256-byte aligned: the tensor maps in the records need 64
+    off = align_up(off + t.adv_recs.size(), 256);
+    for (int q = 0; q < 2; ++q) {
+        t.off_adv_starts[q] = off;
+        off = align_up(off + sizeof(int) * t.adv_starts[q].size(), 256);
+    }
     if (t.blocked) {
         t.off_tb = off;  // 256-byte aligned: the tensor maps in the records need 64
         off = align_up(off + t.tb_recs.size(), 256);
@@ -309,6 +344,9 @@ void pack_table(const TableImage& t, char* blob) {
     memcpy(blob + t.off_starts, t.starts.data(), sizeof(int) * t.starts.size());
     if (!t.boxes.empty()) memcpy(blob + t.off_boxes, t.boxes.data(), sizeof(BoxObj) * t.boxes.size());
     if (!t.spheres.empty()) memcpy(blob + t.off_spheres, t.spheres.data(), sizeof(SphereObj) * t.spheres.size());
+    memcpy(blob + t.off_adv, t.adv_recs.data(), t.adv_recs.size());
+    for (int q = 0; q < 2; ++q)
+        memcpy(blob + t.off_adv_starts[q], t.adv_starts[q].data(), sizeof(int) * t.adv_starts[q].size());
     if (t.blocked) {
         memcpy(blob + t.off_tb, t.tb_recs.data(), t.tb_recs.size());
         memcpy(blob + t.off_tb_starts, t.tb_starts.data(), sizeof(int) * t.tb_starts.size());
@@ -343,7 +381,8 @@ void table_args(const TableImage& t, void* dev, GroupArgs& a, int n) {
     a.zslab = t.zslab;
     a.nwaves = t.nwaves;
     a.sweeps_only = 0;
-    a.phases = GP_ALL;
+    a.adv = base + t.off_adv;
+    for (int q = 0; q < 2; ++q) a.adv_starts[q] = reinterpret_cast<const int*>(base + t.off_adv_starts[q]);
 }
 
 // Copy a table image into `dev` (synchronous; callers hold no step that reads it in flight).
@@ -361,13 +400,19 @@ int launch_config(const GroupSchedule& sched, const TableImage& t, GroupLaunch& 
     if (rc) return smk_fail(SMK_ERR_CUDA, std::string("grouped kernels: ") + cudaGetErrorString((cudaError_t)rc));
     if (coop < 1) return smk_fail(SMK_ERR_CUDA, "grouped projection kernel cannot be resident");
     const int n = (int)t.grids.size();
-    kernels = 1;  // the projection
     for (int s = 0; s < GS_COUNT; ++s) {
         L.total[s] = t.starts[(size_t)s * (n + 1) + n];
         L.ctas[s] = 0;
     }
-    const int launched[4] = {GS_OBJECTS, GS_FORCE, GS_ADV_VEL, GS_ADV_RHO};
+    // the projection: one cooperative kernel, or the blocked solve's start and the phases around it
+    kernels = 1;
+    const int launched[3] = {GS_OBJECTS, GS_FORCE, GS_ADV_RHO}, blocked[3] = {GS_RHS, GS_PROJECT, GS_DIV};
     for (int s : launched) kernels += L.total[s] > 0 ? 1 : 0;
+    for (int s : blocked) kernels += t.blocked && L.total[s] > 0 ? 1 : 0;
+    for (int q = 0; q < 2; ++q) {
+        L.adv_total[q] = t.adv_starts[q][n];
+        kernels += L.adv_total[q] > 0 ? 1 : 0;
+    }
     const int per_sm = sched.ctas_per_sm > 0 ? std::min(sched.ctas_per_sm, coop) : coop;
     L.coop_ctas = per_sm * sms;
     return SMK_OK;
@@ -446,7 +491,6 @@ int grouped_step(smk_batch* b, const float* dts, float dt_all, cudaStream_t st) 
         if (t.blocked) {
             slot->tb = tb_launch(t, slot->dev, n, b->body);
             slot->tb.launches = b->dev_launches;
-            slot->kernels += 1;  // the projection's second cooperative launch
         }
         if (b->use_graphs && b->graphs_ok) {
             cudaGraph_t graph = nullptr;
@@ -702,7 +746,7 @@ int group_runner_step(GroupRunner* r, smk_sim* const* sims, const float* dts, in
     SMK_CUDA(cudaEventRecord(sl.done, st));
     sl.used = true;
     for (int i = 0; i < n; ++i) after_step(sims[i]);
-    if (kernels) *kernels = k + nk + (t.blocked ? 1 + tb.issued : 0);
+    if (kernels) *kernels = k + nk + (t.blocked ? tb.issued : 0);
     return SMK_OK;
 }
 

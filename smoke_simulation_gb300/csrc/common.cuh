@@ -169,83 +169,19 @@ template <> struct Raw4<__nv_bfloat16> { typedef Raw4h type; };
 
 // ---- reference-exact helpers ---------------------------------------------------------------
 
-// avgU/avgV/avgW (smokeSimulation.cu:409-447): 8-point sums in the reference's order, / 8.
-template <typename T>
-__device__ __forceinline__ float avgU(const T* __restrict__ f, const Grid& g, int i) {
-    const int X = g.X, XY = g.XY;
-    float s = ldv(f, i - XY) + ldv(f, i + 1 - XY) + ldv(f, i - X - XY) + ldv(f, i + 1 - X - XY) + ldv(f, i) +
-              ldv(f, i + 1) + ldv(f, i - X) + ldv(f, i + 1 - X);
-    return s / 8.0f;
-}
-template <typename T>
-__device__ __forceinline__ float avgV(const T* __restrict__ f, const Grid& g, int i) {
-    const int X = g.X, XY = g.XY;
-    float s = ldv(f, i - XY) + ldv(f, i - 1 - XY) + ldv(f, i + X - XY) + ldv(f, i - 1 + X - XY) + ldv(f, i) +
-              ldv(f, i - 1) + ldv(f, i + X) + ldv(f, i - 1 + X);
-    return s / 8.0f;
-}
-template <typename T>
-__device__ __forceinline__ float avgW(const T* __restrict__ f, const Grid& g, int i) {
-    const int X = g.X, XY = g.XY;
-    float s = ldv(f, i) + ldv(f, i - 1) + ldv(f, i - X) + ldv(f, i - 1 - X) + ldv(f, i - XY) + ldv(f, i - 1 - XY) +
-              ldv(f, i - X - XY) + ldv(f, i - 1 - X - XY);
-    return s / 8.0f;
-}
-
-// The eight weighted corner terms of sampleSmoke (smokeSimulation.cu:474-482), summed in the
-// reference's order.
-__device__ __forceinline__ float trilinear_ref(float xw0, float xw1, float yw0, float yw1, float zw0, float zw1,
-                                               float a000, float a100, float a010, float a110, float a001,
-                                               float a101, float a011, float a111) {
-    return xw0 * yw0 * zw0 * a000 + xw1 * yw0 * zw0 * a100 + xw0 * yw1 * zw0 * a010 +
-           xw1 * yw1 * zw0 * a110 + xw0 * yw0 * zw1 * a001 + xw1 * yw0 * zw1 * a101 +
-           xw0 * yw1 * zw1 * a011 + xw1 * yw1 * zw1 * a111;
-}
-
-// sampleSmoke (smokeSimulation.cu:451-484): clamp the position to [1, n-1] with the CELL
-// dims, trilinear weights from (c - delta) - i0, eight terms summed in the reference's order.
-// HX, HY, HZ: delta = 0.5 on that axis (1) or 0 (0); every call site has n >= 2 on every axis
-// (it samples only from cells with an interior neighbour).  After the clamp c lies in [1, n-1],
-// so c - delta >= 0.5 and floorf equals truncation, and the reference's fminf(i0, n-1) never
-// changes i0.  Its upper corner fminf(i0 + 1, n - 1): with delta = 0.5, c - delta <= n - 1.5,
-// so i0 <= n - 2 and the corner is always i0 + 1; with delta = 0 it is i0 + 1 unless i0 = n - 1
-// (a position clamped to the last cell), where it repeats i0.  Integer index arithmetic with
-// these facts gives every result of the reference's float index arithmetic.
-template <int HX, int HY, int HZ, typename T>
-__device__ __forceinline__ float sample_ref(const T* __restrict__ f, const Grid& g, float px,
-                                           float py, float pz) {
-    const int lx = g.nx - 1, ly = g.ny - 1, lz = g.nz - 1;
-    const float mx = (float)(unsigned)lx, my = (float)(unsigned)ly, mz = (float)(unsigned)lz;
-    const float xs = fmaxf(fminf(px, mx), 1.0f) - (HX ? 0.5f : 0.0f);
-    const float ys = fmaxf(fminf(py, my), 1.0f) - (HY ? 0.5f : 0.0f);
-    const float zs = fmaxf(fminf(pz, mz), 1.0f) - (HZ ? 0.5f : 0.0f);
-    const int x0 = __float2int_rz(xs);
-    const float xw1 = xs - (float)x0;
-    const float xw0 = 1.0f - xw1;
-    const int y0 = __float2int_rz(ys);
-    const float yw1 = ys - (float)y0;
-    const float yw0 = 1.0f - yw1;
-    const int z0 = __float2int_rz(zs);
-    const float zw1 = zs - (float)z0;
-    const float zw0 = 1.0f - zw1;
-    // The upper corner is +1 on each axis except where a delta-0 axis was clamped to the last
-    // cell (then it repeats the lower one).  Every +1 neighbour lies inside the arrays (rows
-    // hold >= nx+1 elements, planes >= ny+1 rows, the field >= nz+1 planes), so the x+1 values
-    // are loaded at a fixed offset and replaced by the x0 values where the corner repeats: the
-    // eight loads need four row addresses, not eight index computations.
-    const int sy = (HY || y0 < ly) ? g.X : 0;
-    const int sz = (HZ || z0 < lz) ? g.XY : 0;
-    const T* r00 = f + (x0 + y0 * g.X + z0 * g.XY);
-    const T* r10 = r00 + sy;
-    const T* r01 = r00 + sz;
-    const T* r11 = r01 + sy;
-    const float a000 = ldv(r00, 0), a010 = ldv(r10, 0), a001 = ldv(r01, 0), a011 = ldv(r11, 0);
-    const float b100 = ldv(r00, 1), b110 = ldv(r10, 1), b101 = ldv(r01, 1), b111 = ldv(r11, 1);
-    const bool sx = HX || x0 < lx;
-    const float a100 = sx ? b100 : a000, a110 = sx ? b110 : a010, a101 = sx ? b101 : a001,
-                a111 = sx ? b111 : a011;
-    return trilinear_ref(xw0, xw1, yw0, yw1, zw0, zw1, a000, a100, a010, a110, a001, a101, a011, a111);
-}
+// The advections (kernels_advect_tile.cu, density_rows) keep the reference's arithmetic, term for term:
+//   - avgU/avgV/avgW (smokeSimulation.cu:409-447): 8-point sums in the reference's order, / 8;
+//   - sampleSmoke (smokeSimulation.cu:451-484): clamp the position to [1, n-1] with the CELL dims,
+//     trilinear weights from (c - delta) - i0, delta 0.5 on an axis or 0, and the eight terms
+//     xw * yw * zw * a summed in the order 000, 100, 010, 110, 001, 101, 011, 111 (digits: x, y, z).
+// Every call has n >= 2 on every axis (it samples only from cells with an interior neighbour).  After the
+// clamp c lies in [1, n-1], so c - delta >= 0.5 and floorf equals truncation, and the reference's
+// fminf(i0, n-1) never changes i0.  Its upper corner fminf(i0 + 1, n - 1): with delta = 0.5,
+// c - delta <= n - 1.5, so i0 <= n - 2 and the corner is always i0 + 1; with delta = 0 it is i0 + 1 unless
+// i0 = n - 1 (a position clamped to the last cell), where it repeats i0.  Integer index arithmetic with
+// these facts gives every result of the reference's float index arithmetic.  Every +1 neighbour lies inside
+// the arrays (rows hold >= nx+1 elements, planes >= ny+1 rows, the field >= nz+1 planes), so the x+1
+// values are loaded at a fixed offset and replaced by the x0 values where the corner repeats.
 
 // Loads issued where they stand (volatile inline PTX): the compiler can neither sink them into
 // the conditional block that consumes them nor merge them away, so a warp has a cell's loads in
@@ -275,6 +211,20 @@ __device__ __forceinline__ void density_unit(const Grid& g, int unit, int& x, in
     const int wide = min(DENSITY_STRIP, g.nx - 2 - left), r = unit - left * pairs;
     x = 1 + left + r % wide;
     y = 1 + 2 * (r / wide);
+}
+
+// The grid j that tile t of a grouped launch belongs to: the last one with starts[j] <= t (starts[0] = 0,
+// n grids, t below starts[n]).  Every lane of a warp calls it: one load a lane narrows 32-fold.
+__device__ __forceinline__ int find_grid(const int* __restrict__ starts, int n, int t) {
+    const int lane = (int)((threadIdx.x + blockDim.x * threadIdx.y) & 31u);
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) / 32, k = lo + lane * step;
+        const unsigned at = __ballot_sync(0xffffffffu, k < hi && starts[k] <= t);
+        lo += (__popc(at) - 1) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
 }
 
 }  // namespace smk

@@ -25,7 +25,6 @@ enum GroupStage : int {
     GS_RESID,        // residual of a tolerance check (flattened tiles, interior)
     GS_PROJECT,      // gradient subtract (FP32) or FP32 projection + BF16 rounding
     GS_DIV,          // max |div u| (flattened tiles, interior); 0 tiles when not reported
-    GS_ADV_VEL,      // velocity advection
     GS_ADV_RHO,      // density advection
     GS_COUNT
 };
@@ -85,20 +84,18 @@ struct GroupSync {
     int left;                  // CTAs that left the kernel because a barrier gave up
 };
 
-// Phases of the cooperative projection kernel.
-enum : int { GP_RHS = 1, GP_SOLVE = 2, GP_FINISH = 4, GP_ALL = 7 };
-
 struct GroupArgs {
     const GroupGrid* grids;
     const int* starts;  // GS_COUNT rows of n + 1 tile prefix sums
     const BoxObj* boxes;
     const SphereObj* spheres;
     GroupSync* sync;
+    const void* adv;           // velocity advection records (group_advect_record_bytes() each)
+    const int* adv_starts[2];  // their tile prefix sums: FP32 output, BF16 output
     int n;
     int zslab;        // z planes per sweep / residual / divergence tile (a thread walks them)
     int nwaves;       // solve waves (every grid's `wave` is below this)
     int sweeps_only;  // tuning: only the sweep passes (fixed count, no checks), on scratch buffers
-    int phases;       // GP_* bits: rhs + pressure start, colour-pass solve, subtract + divergence
     unsigned long long wait_ns;  // a barrier wait gives up after this long (%globaltimer)
     int skip_barrier;            // testing: CTA 0 does not arrive at this barrier (1-based; 0 = none)
 };
@@ -151,22 +148,19 @@ __host__ __device__ inline void group_extent(int stage, const GroupGrid& d, int&
             if (d.kind == GK_F32) { rx = g.nx - 1; ry = g.ny - 1; rz = g.nz - 1; }
             else { rx = g.nx + 1; ry = g.ny + 1; rz = g.nz + 1; }
             break;
-        case GS_ADV_VEL: rx = g.nx - 1; ry = g.ny - 1; rz = g.nz - 1; break;
-        case GS_ADV_RHO: rx = g.nx - 2; ry = g.ny - 2; rz = g.nz - 2; break;
         default: break;
     }
 }
 
-// Advection tiles walk GROUP_ADV_ZC consecutive planes (as the single-grid advection kernels).
-constexpr int GROUP_ADV_ZC = 4;
+// Planes of a density advection tile (as the single-grid kernel on large grids).
 constexpr int GROUP_RHO_ZC = 8;
 
-// 4-wide tiles (grids with vec4): 16 groups of 4 consecutive x by 16 rows of one plane, over
-// gx groups (from x = 0), ry rows and rz planes.
-constexpr int GX4_GX = 16, GX4_GY = 16;
+// 4-wide tiles (grids with vec4): 256 groups of 4 consecutive x, flattened over the gx groups (from x = 0)
+// of ry rows, by GX4_ZC planes that each thread walks.
+constexpr int GX4_ZC = 4;
 __host__ __device__ inline int group_x4_tiles(int gx, int ry, int rz) {
     if (gx <= 0 || ry <= 0 || rz <= 0) return 0;
-    return group_div_up(gx, GX4_GX) * group_div_up(ry, GX4_GY) * rz;
+    return group_div_up(gx * ry, GROUP_TILE) * group_div_up(rz, GX4_ZC);
 }
 // Range of a 4-wide stage: groups of x, rows (from y0) and planes (from z0).
 __host__ __device__ inline bool group_x4_extent(int stage, const GroupGrid& d, int& gx, int& ry, int& rz, int& y0,
@@ -196,13 +190,7 @@ __host__ __device__ inline int group_tiles(int stage, const GroupGrid& d, int zs
         case GS_SWEEP: return group_sweep_tpp(g) * slabs;
         case GS_RESID: return group_interior_tpp(g) * slabs;
         case GS_DIV: return d.report_div ? group_interior_tpp(g) * slabs : 0;
-        case GS_ADV_VEL:
-        case GS_ADV_RHO: {
-            int rx, ry, rz;
-            group_extent(stage, d, rx, ry, rz);
-            if (stage == GS_ADV_RHO) return rz > 0 ? density_blocks(g) * group_div_up(rz, GROUP_RHO_ZC) : 0;
-            return group_block_tiles(rx, ry, group_div_up(rz, GROUP_ADV_ZC));
-        }
+        case GS_ADV_RHO: return g.nz >= 3 ? density_blocks(g) * group_div_up(g.nz - 2, GROUP_RHO_ZC) : 0;
         default: {
             int rx, ry, rz;
             group_extent(stage, d, rx, ry, rz);
@@ -224,6 +212,7 @@ struct GroupLaunch {
     int total[GS_COUNT];  // tiles per stage over the batch
     int ctas[GS_COUNT];   // CTAs of each grid-stride launch
     int coop_ctas;        // CTAs of the cooperative projection kernel
+    int adv_total[2];     // velocity advection tiles: FP32 output, BF16 output
 };
 
 // Host launchers (kernels_group.cu).  Return 0 or a cudaError_t value.

@@ -216,6 +216,13 @@ int launch_advect_velocity_tile(const AdvectMaps* m, int set, const Grid& g, con
                                 const float* w0, To* u1, To* v1, To* w1, const uint8_t* flags, float dt, int* kerr,
                                 cudaStream_t st, int c0 = 0, int c1 = -1);
 int advect_velocity_chunk_planes(const Grid& g);
+// The grouped form: a record per grid (in / out: u, v, w; zc planes a tile), filled into a table that is
+// copied to the device; group_advect_fill returns the grid's tiles, a launch runs every tile of the grids
+// with one output type (starts: their prefix sums, other grids empty).
+size_t group_advect_record_bytes();
+int group_advect_fill(void* rec, const AdvectMaps* m, int set, const Grid& g, const float* const* in, void* const* out,
+                      const uint8_t* flags, int* kerr, float dt, int zc);
+int launch_group_advect_velocity(const void* recs, const int* starts, int n, int total, bool bf16, cudaStream_t st);
 int advect_velocity_chunks(const Grid& g);
 template <typename T, typename Tv>
 void launch_advect_density(const Grid& g, const T* r0, T* r1, const Tv* u1, const Tv* v1, const Tv* w1,

@@ -10,8 +10,8 @@
 // the two cells is shorter than REACH, the eight corners of each sample lie in the window and both
 // cells go through packed arithmetic (sample_pair; without the clamps in tiles that cannot need them);
 // otherwise each cell by itself reads the window or, past it, global memory (sample_win).  The
-// arithmetic is the reference's, term for term (avgU/V/W, sample_ref), so the results are the bits of
-// the per-cell kernel.
+// arithmetic is the reference's, term for term (avgU/V/W and sampleSmoke, common.cuh).  The grouped
+// form runs the same tiles over every grid of a batch.
 //
 // Instruction issue bounds it (75 % of the slots, 46 % of the warps at 64 registers): 256^3 FP32 took
 // 200 us with one cell a thread and scalar arithmetic (388 instructions a cell, 203 M in all), 162 us now
@@ -26,6 +26,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <cstring>
 #include <type_traits>
 
 #include "common.cuh"
@@ -53,7 +54,7 @@ struct AdvMaps {
     CUtensorMap u, v, w;
 };
 
-// A trilinear sample of one field (sample_ref's arithmetic) whose corners are read from the
+// A trilinear sample of one field (sampleSmoke's arithmetic) whose corners are read from the
 // window planes pm, pc, pp (planes z - 1, z, z + 1; the window's origin is (wx0, wy0)) when
 // they lie there, else from global memory.
 template <int HX, int HY, int HZ>
@@ -109,7 +110,7 @@ __device__ __forceinline__ float sample_win(const float* __restrict__ f, const G
     }
     const float a100 = sx ? b100 : a000, a110 = sx ? b110 : a010, a101 = sx ? b101 : a001,
                 a111 = sx ? b111 : a011;
-    // trilinear_ref's products as packed pairs (each lane one IEEE product, the same bits).  The
+    // the eight terms' products as packed pairs (each lane one IEEE product, the same bits).  The
     // products feed products and scalar sums only: ptxas contracts a packed product followed by a
     // packed add into a fused multiply-add, even with -fmad=false and explicit .rn forms
     const float2 xw = make_float2(xw0, xw1);
@@ -186,7 +187,7 @@ __device__ __forceinline__ float2 sample_pair(const float* win, const Tops& top,
     };
     corners(bx.x, by.x, bz.x, [&](int i, float v) { a[i].x = v; });
     corners(bx.y, by.y, bz.y, [&](int i, float v) { a[i].y = v; });
-    // trilinear_ref, term for term
+    // the eight terms in the reference's order
     const float2 w00 = __fmul2_rn(x0, y0), w10 = __fmul2_rn(x1, y0), w01 = __fmul2_rn(x0, y1), w11 = __fmul2_rn(x1, y1);
     float2 s = __fmul2_rn(__fmul2_rn(w00, z0), a[0]);
     s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w10, z0), a[1]), k.one, s);
@@ -205,18 +206,23 @@ __device__ __forceinline__ float reach(float m, float x) {
 }
 constexpr float REACH = 0.9f;  // a backtrace of one cell at most, with room for the positions' rounding
 
+struct AdvWindow {
+    alignas(128) float win[AT_SLOTS][3][AT_PSTR];
+    alignas(8) uint64_t mbar[AT_SLOTS];
+};
+
+// The tile (bx, by) for planes zs .. zs + zc - 1.
 template <typename To>
-__global__ void __launch_bounds__(AT_TX * AT_TY, 4)
-k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float* __restrict__ u0,
-                       const float* __restrict__ v0, const float* __restrict__ w0, To* __restrict__ u1,
-                       To* __restrict__ v1, To* __restrict__ w1, const uint8_t* __restrict__ flags, float dt,
-                       int* kerr, int cz0, int zc, float one, Tops top) {
-    __shared__ alignas(128) float win[AT_SLOTS][3][AT_PSTR];
-    __shared__ alignas(8) uint64_t mbar[AT_SLOTS];
+__device__ __forceinline__ void advect_tile(AdvWindow& sh, const AdvMaps& maps, const Grid& g,
+                                            const float* __restrict__ u0, const float* __restrict__ v0,
+                                            const float* __restrict__ w0, To* __restrict__ u1, To* __restrict__ v1,
+                                            To* __restrict__ w1, const uint8_t* __restrict__ flags, float dt, int* kerr,
+                                            int bx, int by, int zs, int zc, float one, const Tops& top) {
+    auto& win = sh.win;
+    auto& mbar = sh.mbar;
     const int tx = (int)threadIdx.x, ty = (int)threadIdx.y;
     const bool leader = tx == 0 && ty == 0;
-    const int xt = (int)blockIdx.x * AT_TX, yt = 1 + (int)blockIdx.y * AT_ROWS;
-    const int zs = 1 + (cz0 + (int)blockIdx.z) * zc;
+    const int xt = bx * AT_TX, yt = 1 + by * AT_ROWS;
     const int ze = min(zs + zc, g.nz);  // planes [zs, ze) are advected; [zs - 1, ze] are read
     const int wx0 = xt - AT_OX, wy0 = yt - 1;
 
@@ -369,6 +375,54 @@ k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float
     }
 }
 
+template <typename To>
+__global__ void __launch_bounds__(AT_TX * AT_TY, 4)
+k_advect_velocity_tile(const __grid_constant__ AdvMaps maps, Grid g, const float* __restrict__ u0,
+                       const float* __restrict__ v0, const float* __restrict__ w0, To* __restrict__ u1,
+                       To* __restrict__ v1, To* __restrict__ w1, const uint8_t* __restrict__ flags, float dt,
+                       int* kerr, int cz0, int zc, float one, Tops top) {
+    __shared__ AdvWindow sh;
+    advect_tile(sh, maps, g, u0, v0, w0, u1, v1, w1, flags, dt, kerr, (int)blockIdx.x, (int)blockIdx.y,
+                1 + (cz0 + (int)blockIdx.z) * zc, zc, one, top);
+}
+
+// One grid of a grouped velocity advection.
+struct GroupAdvGrid {
+    AdvMaps maps;
+    Grid g;
+    Tops top;
+    const float *u0, *v0, *w0;
+    void *u1, *v1, *w1;
+    const uint8_t* flags;
+    int* kerr;
+    float dt;
+    int tiles_x, tiles_y, zc;
+};
+
+// Every tile of the grids whose advected faces are To, one CTA a tile (starts: prefix sums of the tiles).
+template <typename To>
+__global__ void __launch_bounds__(AT_TX * AT_TY, 4)
+k_group_advect_velocity(const GroupAdvGrid* __restrict__ grids, const int* __restrict__ starts, int n, float one) {
+    __shared__ AdvWindow sh;
+    const int j = find_grid(starts, n, (int)blockIdx.x);
+    const GroupAdvGrid& d = grids[j];
+    const int local = (int)blockIdx.x - starts[j], tx = d.tiles_x, ty = d.tiles_y, zc = d.zc;
+    const Grid g = d.g;
+    const Tops top = d.top;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {  // the maps were written by a copy into the table
+        tensormap_acquire(&d.maps.u);
+        tensormap_acquire(&d.maps.v);
+        tensormap_acquire(&d.maps.w);
+    }
+    advect_tile(sh, d.maps, g, d.u0, d.v0, d.w0, (To*)d.u1, (To*)d.v1, (To*)d.w1, d.flags, d.dt, d.kerr, local % tx,
+                (local / tx) % ty, 1 + (local / (tx * ty)) * zc, zc, one, top);
+}
+
+Tops tops_of(const Grid& g) {
+    return Tops{(float)(g.nx - 1),     (float)(g.ny - 1),     (float)(g.nz - 1),
+                0x4b000000 + g.nx - 1, 0x4b000000 + g.ny - 1, 0x4b000000 + g.nz - 1};
+}
+
 }  // namespace
 
 static int tiles_x(const Grid& g) { return (g.nx + AT_TX - 1) / AT_TX; }
@@ -409,10 +463,8 @@ int launch_advect_velocity_tile(const AdvectMaps* m, int set, const Grid& g, con
     if (c0 < 0) c0 = 0;
     if (c1 <= c0) return 0;
     const dim3 grid((unsigned)tiles_x(g), (unsigned)tiles_y(g), (unsigned)(c1 - c0));
-    const Tops top{(float)(g.nx - 1), (float)(g.ny - 1), (float)(g.nz - 1),
-                   0x4b000000 + g.nx - 1, 0x4b000000 + g.ny - 1, 0x4b000000 + g.nz - 1};
     k_advect_velocity_tile<To><<<grid, dim3(AT_TX, AT_TY), 0, st>>>(m->set[set], g, u0, v0, w0, u1, v1, w1, flags, dt,
-                                                                     kerr, c0, advect_velocity_chunk_planes(g), 1.0f, top);
+                                                                     kerr, c0, advect_velocity_chunk_planes(g), 1.0f, tops_of(g));
     return 0;
 }
 
@@ -428,6 +480,42 @@ int advect_velocity_chunk_planes(const Grid& g) {
 int advect_velocity_chunks(const Grid& g) {
     const int zc = advect_velocity_chunk_planes(g);
     return g.nz < 2 ? 0 : (g.nz - 1 + zc - 1) / zc;
+}
+
+size_t group_advect_record_bytes() { return sizeof(GroupAdvGrid); }
+
+int group_advect_fill(void* rec, const AdvectMaps* m, int set, const Grid& g, const float* const* in, void* const* out,
+                      const uint8_t* flags, int* kerr, float dt, int zc) {
+    if (m == nullptr || set < 0 || set >= m->n || g.nx < 2 || g.ny < 2 || g.nz < 2) return 0;
+    GroupAdvGrid d;
+    memset(&d, 0, sizeof(d));
+    d.maps = m->set[set];
+    d.g = g;
+    d.top = tops_of(g);
+    d.u0 = in[0];
+    d.v0 = in[1];
+    d.w0 = in[2];
+    d.u1 = out[0];
+    d.v1 = out[1];
+    d.w1 = out[2];
+    d.flags = flags;
+    d.kerr = kerr;
+    d.dt = dt;
+    d.tiles_x = tiles_x(g);
+    d.tiles_y = tiles_y(g);
+    d.zc = zc;
+    memcpy(rec, &d, sizeof(d));
+    return d.tiles_x * d.tiles_y * ((g.nz - 1 + zc - 1) / zc);
+}
+
+int launch_group_advect_velocity(const void* recs, const int* starts, int n, int total, bool bf16, cudaStream_t st) {
+    if (total <= 0) return 0;
+    const GroupAdvGrid* d = static_cast<const GroupAdvGrid*>(recs);
+    if (bf16)
+        k_group_advect_velocity<__nv_bfloat16><<<(unsigned)total, dim3(AT_TX, AT_TY), 0, st>>>(d, starts, n, 1.0f);
+    else
+        k_group_advect_velocity<float><<<(unsigned)total, dim3(AT_TX, AT_TY), 0, st>>>(d, starts, n, 1.0f);
+    return (int)cudaGetLastError();
 }
 
 template int launch_advect_velocity_tile<float>(const AdvectMaps*, int, const Grid&, const float*, const float*,

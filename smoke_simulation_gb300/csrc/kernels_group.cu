@@ -1,15 +1,23 @@
-// Grouped kernels of a batch step: one persistent launch per stage over every grid (group.h).
+// Grouped kernels of a batch step: one launch per stage over every grid (group.h).
 //
 //   k_group_objects     emitters (boxes, then spheres) of every grid
 //   k_group_forcing     integrate + clamp
-//   k_group_project     the whole projection as ONE cooperative kernel: b and the pressure
+//   k_group_rhs, k_group_solve_start, [blocked sweeps], k_group_finish, k_group_div
+//                       the projection around the blocked solve: b and the pressure start, the status
+//                       words, the gradient subtract (or the BF16 projection), and max |div u|
+//   k_group_project     or the whole projection as ONE cooperative kernel: b and the pressure
 //                       start, every red-black colour pass of every grid with the per-grid
 //                       tolerance rule, the gradient subtract (or the BF16 projection), and
 //                       max |div u|; phases are separated by a bounded grid barrier
-//   k_group_adv_vel     velocity advection
+//   velocity advection  kernels_advect_tile.cu, over every grid's tiles
 //   k_group_adv_rho     density advection
-// The grid-stride kernels are sized to the resident CTAs of the device; every tile runs the
-// stage body of the single-grid kernel, so a grid's results are the same alone and batched.
+// Every tile runs the stage body of the single-grid kernel, so a grid's results are the same alone and
+// batched.  The streaming stages are bound by memory: a tile is 256 groups of 4 x, flattened over a plane's
+// rows, by 4 planes that a thread walks, one CTA a tile, which finds its grid with two loads a lane
+// (find_grid).  64 grids of 32^3 to 128^3 (31.8 M cells, FP32, cold cache): forcing 182 -> 143 us, rhs
+// 311 -> 249 and subtract 226 -> 207 out of the cooperative kernel, whose 64 registers and grid barriers they
+// shared, velocity advection 541 -> 369 in the single-grid kernel's tiles, density 282 -> 205.  1, 2 and 8
+// planes a tile: the whole step 270 us, 25 us and 0 us slower; 40 registers a thread: 320 us slower (spills).
 //
 // Tolerance rule (the single-grid sweep loop's): at the start of check group k (sweep k*G) a
 // grid whose residual recorded at the start of group k-1 is within tolerance is done; any other
@@ -59,13 +67,15 @@ __device__ __forceinline__ uint3 tile_bid(int local, int rx, int ry) {
     return b;
 }
 
-// Group of 4 x, row and plane of this thread in tile `local` of a 4-wide stage (group_x4_tiles).
-__device__ __forceinline__ void x4_coords(int local, int gx, int ry, int y0, int z0, int& x, int& y, int& z) {
-    const int nbx = group_div_up(gx, GX4_GX), nby = group_div_up(ry, GX4_GY);
-    const int t = tid256();
-    x = 4 * ((local % nbx) * GX4_GX + t % GX4_GX);
-    y = y0 + ((local / nbx) % nby) * GX4_GY + t / GX4_GX;
-    z = z0 + local / (nbx * nby);
+// f(x, y, z) for the groups of 4 x of this thread in tile `local` of a 4-wide stage (group_x4_tiles).
+template <class F>
+__device__ __forceinline__ void x4_walk(int local, int gx, int ry, int rz, int y0, int z0, F&& f) {
+    const int blocks = group_div_up(gx * ry, GROUP_TILE);
+    const int unit = (local % blocks) * GROUP_TILE + tid256();
+    if (unit >= gx * ry) return;
+    const int x = 4 * (unit % gx), y = y0 + unit / gx, za = z0 + (local / blocks) * GX4_ZC;
+    const int ze = min(za + GX4_ZC, z0 + rz);
+    for (int z = za; z < ze; ++z) f(x, y, z);
 }
 
 // f(j, local) for every tile of `stage` this CTA owns (grid-stride over the batch's tiles).
@@ -76,16 +86,7 @@ __device__ __forceinline__ void for_tiles(const GroupArgs& a, int stage, const u
     const int* st = a.starts + stage * (a.n + 1);
     const int total = st[a.n];
     const int step = (int)gridDim.x;
-    int j = 0;
-    if ((int)blockIdx.x < total) {  // the grid of this CTA's first tile (binary search)
-        int lo = 0, hi = a.n - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (st[mid] <= (int)blockIdx.x) lo = mid;
-            else hi = mid - 1;
-        }
-        j = lo;
-    }
+    int j = (int)blockIdx.x < total ? find_grid(st, a.n, (int)blockIdx.x) : 0;
     for (int t = (int)blockIdx.x; t < total; t += step) {
         while (st[j + 1] <= t) ++j;
         if (mask != nullptr && !(mask[j] & need)) {
@@ -129,18 +130,23 @@ __global__ void __launch_bounds__(GROUP_TILE) k_group_forcing(const GroupArgs a)
         int gx, ry, rz, y0, z0;
         typedef __nv_bfloat16 h;
         if (group_x4_extent(GS_FORCE, d, gx, ry, rz, y0, z0)) {
-            int x, y, z;
-            x4_coords(local, gx, ry, y0, z0, x, y, z);
             if (d.kind == GK_BF16)
-                body_forcing_x4<h, h>(gg, (h*)d.u_now, (h*)d.v_now, (h*)d.w_now, (const h*)d.rho_now, d.flags, d.dt,
-                                      d.gravity, d.alpha, d.lim_sq, d.lim, d.clamp_mode, x, y, z);
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_forcing_x4<h, h>(gg, (h*)d.u_now, (h*)d.v_now, (h*)d.w_now, (const h*)d.rho_now, d.flags,
+                                          d.dt, d.gravity, d.alpha, d.lim_sq, d.lim, d.clamp_mode, x, y, z);
+                });
             else if (d.kind == GK_BF16_VEL)
-                body_forcing_x4<h, float>(gg, (h*)d.u_now, (h*)d.v_now, (h*)d.w_now, (const float*)d.rho_now,
-                                          d.flags, d.dt, d.gravity, d.alpha, d.lim_sq, d.lim, d.clamp_mode, x, y, z);
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_forcing_x4<h, float>(gg, (h*)d.u_now, (h*)d.v_now, (h*)d.w_now, (const float*)d.rho_now,
+                                              d.flags, d.dt, d.gravity, d.alpha, d.lim_sq, d.lim, d.clamp_mode, x, y,
+                                              z);
+                });
             else
-                body_forcing_x4<float, float>(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now,
-                                              (const float*)d.rho_now, d.flags, d.dt, d.gravity, d.alpha, d.lim_sq,
-                                              d.lim, d.clamp_mode, x, y, z);
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_forcing_x4<float, float>(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now,
+                                                  (const float*)d.rho_now, d.flags, d.dt, d.gravity, d.alpha,
+                                                  d.lim_sq, d.lim, d.clamp_mode, x, y, z);
+                });
             return;
         }
         const uint3 bid = tile_bid(local, d.g.nx, d.g.ny - 1);
@@ -154,29 +160,6 @@ __global__ void __launch_bounds__(GROUP_TILE) k_group_forcing(const GroupArgs a)
             body_forcing<float, float>(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now,
                                        (const float*)d.rho_now, d.flags, d.dt, d.gravity, d.alpha, d.lim_sq,
                                        d.lim, d.clamp_mode, bid);
-    });
-}
-
-// The advection tiles walk GROUP_ADV_ZC consecutive planes (the planes neighbouring cells'
-// averages and samples share stay in L1); register caps of 8 CTAs per SM (32 registers: the
-// velocity kernel spills 56 bytes there and the 64-grid batch step still runs 1.5% faster than
-// with 5 CTAs and 48 registers).
-__global__ void __launch_bounds__(GROUP_TILE, 8) k_group_adv_vel(const GroupArgs a) {
-    for_tiles(a, GS_ADV_VEL, nullptr, 0, [&](int j, int local) {
-        const GroupGrid& d = a.grids[j];
-        const Grid gg = d.g;  // in registers: the stores of the body cannot alias it
-        const uint3 bid = tile_bid(local, d.g.nx - 1, d.g.ny - 1);
-        typedef __nv_bfloat16 h;
-        for (int k = 0; k < GROUP_ADV_ZC; ++k) {
-            const uint3 b = make_uint3(bid.x, bid.y, bid.z * GROUP_ADV_ZC + k);
-            if ((int)b.z >= d.g.nz - 1) break;
-            if (d.kind == GK_F32)
-                body_advect_velocity<float, float>(gg, d.pu, d.pv, d.pw, (float*)d.u_past, (float*)d.v_past,
-                                                   (float*)d.w_past, d.flags, d.dt, b);
-            else
-                body_advect_velocity<float, h>(gg, d.pu, d.pv, d.pw, (h*)d.u_past, (h*)d.v_past, (h*)d.w_past,
-                                               d.flags, d.dt, b);
-        }
     });
 }
 
@@ -200,6 +183,109 @@ __global__ void __launch_bounds__(GROUP_TILE, 4) k_group_adv_rho(const GroupArgs
             density_rows(gg, (const float*)d.rho_now, (float*)d.rho_past, (const float*)d.u_past,
                          (const float*)d.v_past, (const float*)d.w_past, d.flags, d.dt, one, x, y, z0, z1);
     });
+}
+
+// b and the pressure start of every grid.
+__device__ __forceinline__ void rhs_tiles(const GroupArgs& a) {
+    for_tiles(a, GS_RHS, nullptr, 0, [&](int j, int local) {
+        const GroupGrid& d = a.grids[j];
+        const Grid gg = d.g;  // in registers: the stores of the body cannot alias it
+        typedef __nv_bfloat16 h;
+        int gx, ry, rz, y0, z0;
+        if (group_x4_extent(GS_RHS, d, gx, ry, rz, y0, z0)) {
+            if (d.kind == GK_F32)
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_rhs_x4<float>(gg, (const float*)d.u_now, (const float*)d.v_now, (const float*)d.w_now,
+                                       d.flags, d.b, d.P, d.P2, d.pcur, d.warm, x, y, z, d.Ph, d.extrap);
+                });
+            else
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_rhs_x4<h>(gg, (const h*)d.u_now, (const h*)d.v_now, (const h*)d.w_now, d.flags, d.b, d.P,
+                                   d.P2, d.pcur, d.warm, x, y, z, d.Ph, d.extrap);
+                });
+            return;
+        }
+        const uint3 bid = tile_bid(local, d.g.nx, d.g.ny);
+        if (d.kind == GK_F32)
+            body_rhs<float>(gg, (const float*)d.u_now, (const float*)d.v_now, (const float*)d.w_now, d.flags, d.b,
+                            d.P, d.P2, d.pcur, d.warm, bid, d.Ph, d.extrap);
+        else
+            body_rhs<h>(gg, (const h*)d.u_now, (const h*)d.v_now, (const h*)d.w_now, d.flags, d.b, d.P, d.P2, d.pcur,
+                        d.warm, bid, d.Ph, d.extrap);
+    });
+}
+
+// The gradient subtract (FP32) or the BF16 projection of every grid.  The pressure is the first buffer after
+// the colour-pass solve (*pcur == 0), or where the blocked solve's last launch left it.
+__device__ __forceinline__ void finish_tiles(const GroupArgs& a) {
+    for_tiles(a, GS_PROJECT, nullptr, 0, [&](int j, int local) {
+        const GroupGrid& d = a.grids[j];
+        const Grid gg = d.g;  // in registers: the stores of the body cannot alias it
+        typedef __nv_bfloat16 h;
+        int gx, y0, z0, rx, ry, rz;
+        if (group_x4_extent(GS_PROJECT, d, gx, ry, rz, y0, z0)) {
+            const float* P = (d.pcur != nullptr && *d.pcur == 1) ? d.P2 : d.P;
+            if (d.kind == GK_F32)
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_gradient_subtract_x4(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now, P, d.flags, x, y,
+                                              z);
+                });
+            else
+                x4_walk(local, gx, ry, rz, y0, z0, [&](int x, int y, int z) {
+                    body_project_bf16_x4(gg, (h*)d.u_now, (h*)d.v_now, (h*)d.w_now, P, d.flags, d.pu, d.pv, d.pw, x,
+                                         y, z);
+                });
+            return;
+        }
+        group_extent(GS_PROJECT, d, rx, ry, rz);
+        const uint3 bid = tile_bid(local, rx, ry);
+        if (d.kind == GK_F32)
+            body_gradient_subtract(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now, d.P, d.P2, d.pcur,
+                                   d.flags, bid);
+        else
+            body_project_bf16(gg, (h*)d.u_now, (h*)d.v_now, (h*)d.w_now, d.P, d.P2, d.pcur, d.flags, d.pu, d.pv, d.pw,
+                              bid);
+    });
+}
+
+// max |div u| of the grids that report it.
+__device__ __forceinline__ void div_tiles(const GroupArgs& a) {
+    int cur = -1;
+    unsigned mb = 0u;
+    for_tiles(a, GS_DIV, nullptr, 0, [&](int j, int local) {
+        if (j != cur) {
+            if (cur >= 0) block_max_to(mb, &a.grids[cur].status->div_bits);
+            cur = j;
+            mb = 0u;
+        }
+        const GroupGrid& d = a.grids[j];
+        const Grid g = d.g;  // in registers: the stores below cannot alias it
+        const int tpp = group_interior_tpp(g);
+        const int z0 = 1 + (local / tpp) * a.zslab;
+        const int z1 = min(z0 + a.zslab, g.nz - 1);
+        const int f = (local % tpp) * GROUP_TILE + tid256();
+        const int L = g.nx - 2;
+        if (f < L * (g.ny - 2)) {
+            int i = g.idx(1 + f % L, 1 + f / L, z0);
+            for (int z = z0; z < z1; ++z, i += g.XY)
+                mb = max(mb, __float_as_uint(cell_div(g, d.pu, d.pv, d.pw, d.flags, i)));
+        }
+    });
+    if (cur >= 0) block_max_to(mb, &a.grids[cur].status->div_bits);
+}
+
+// The blocked solve's projection around its sweep launches, one kernel a phase.
+__global__ void __launch_bounds__(GROUP_TILE) k_group_rhs(const GroupArgs a) { rhs_tiles(a); }
+__global__ void __launch_bounds__(GROUP_TILE, 4) k_group_finish(const GroupArgs a) { finish_tiles(a); }
+__global__ void __launch_bounds__(GROUP_TILE) k_group_div(const GroupArgs a) { div_tiles(a); }
+
+// Between k_group_rhs, which may start from the second pressure buffer, and the solve, which starts in the
+// first: one CTA a grid resets *pcur and this step's status words.
+__global__ void __launch_bounds__(GROUP_TILE) k_group_solve_start(const GroupArgs a) {
+    const GroupGrid& d = a.grids[blockIdx.x];
+    unsigned* w = reinterpret_cast<unsigned*>(d.status);
+    for (int k = tid256(); k < d.status_words; k += GROUP_TILE) w[k] = 0u;
+    if (tid256() == 0) *d.pcur = 0;
 }
 
 // ---- cooperative projection -----------------------------------------------------------------
@@ -296,43 +382,19 @@ __device__ __forceinline__ unsigned resid_column(const Grid& g, const float* P, 
 // Per-grid byte of the active set (dynamic shared memory).
 enum : uint8_t { GA_DONE = 1, GA_SWEEP = 2, GA_CHECK = 4 };
 
-__global__ void __launch_bounds__(GROUP_TILE) k_group_project(const GroupArgs a) {
+__global__ void __launch_bounds__(GROUP_TILE, 4) k_group_project(const GroupArgs a) {
     extern __shared__ uint8_t gst[];
     const int tid = tid256();
     unsigned long long target = 0;
     for (int j = tid; j < a.n; j += GROUP_TILE) gst[j] = 0;
 
-    if (!a.sweeps_only && (a.phases & GP_RHS)) {
+    if (!a.sweeps_only) {
         // this step's status words (zeroed by one CTA per grid), then b and the pressure start
         for (int j = (int)blockIdx.x; j < a.n; j += (int)gridDim.x) {
             unsigned* w = reinterpret_cast<unsigned*>(a.grids[j].status);
             for (int k = tid; k < a.grids[j].status_words; k += GROUP_TILE) w[k] = 0u;
         }
-        for_tiles(a, GS_RHS, nullptr, 0, [&](int j, int local) {
-            const GroupGrid& d = a.grids[j];
-            const Grid gg = d.g;  // in registers: the stores of the body cannot alias it
-            int gx, ry, rz, y0, z0;
-            if (group_x4_extent(GS_RHS, d, gx, ry, rz, y0, z0)) {
-                int x, y, z;
-                x4_coords(local, gx, ry, y0, z0, x, y, z);
-                if (d.kind == GK_F32)
-                    body_rhs_x4<float>(gg, (const float*)d.u_now, (const float*)d.v_now, (const float*)d.w_now,
-                                       d.flags, d.b, d.P, d.P2, d.pcur, d.warm, x, y, z, d.Ph, d.extrap);
-                else
-                    body_rhs_x4<__nv_bfloat16>(gg, (const __nv_bfloat16*)d.u_now, (const __nv_bfloat16*)d.v_now,
-                                               (const __nv_bfloat16*)d.w_now, d.flags, d.b, d.P, d.P2, d.pcur,
-                                               d.warm, x, y, z, d.Ph, d.extrap);
-                return;
-            }
-            const uint3 bid = tile_bid(local, d.g.nx, d.g.ny);
-            if (d.kind == GK_F32)
-                body_rhs<float>(gg, (const float*)d.u_now, (const float*)d.v_now, (const float*)d.w_now, d.flags,
-                                d.b, d.P, d.P2, d.pcur, d.warm, bid, d.Ph, d.extrap);
-            else
-                body_rhs<__nv_bfloat16>(gg, (const __nv_bfloat16*)d.u_now, (const __nv_bfloat16*)d.v_now,
-                                        (const __nv_bfloat16*)d.w_now, d.flags, d.b, d.P, d.P2, d.pcur, d.warm,
-                                        bid, d.Ph, d.extrap);
-        });
+        rhs_tiles(a);
         if (!group_barrier(a, target)) {
             group_abort(a);
             return;
@@ -344,8 +406,7 @@ __global__ void __launch_bounds__(GROUP_TILE) k_group_project(const GroupArgs a)
 
     // the solve waves run one after another; inside a wave every grid runs its own colour
     // passes and tolerance rule, pass by pass in lockstep with the wave's other grids
-    const int nwaves = (a.phases & GP_SOLVE) ? a.nwaves : 0;
-    for (int wave = 0; wave < nwaves; ++wave)
+    for (int wave = 0; wave < a.nwaves; ++wave)
     for (int s = 0;; ++s) {
         // which grids sweep now, and which record a residual first (group starts)
         int act = 0, chk = 0;
@@ -443,76 +504,30 @@ __global__ void __launch_bounds__(GROUP_TILE) k_group_project(const GroupArgs a)
             }
         }
     }
-    if (a.sweeps_only || !(a.phases & GP_FINISH)) return;
+    if (a.sweeps_only) return;
 
-    // the pressure is the first buffer after the colour-pass solve (*pcur == 0), or where the
-    // blocked solve's last launch left it
-    for_tiles(a, GS_PROJECT, nullptr, 0, [&](int j, int local) {
-        const GroupGrid& d = a.grids[j];
-        const Grid gg = d.g;  // in registers: the stores of the body cannot alias it
-        int gx, y0, z0, rx, ry, rz;
-        if (group_x4_extent(GS_PROJECT, d, gx, ry, rz, y0, z0)) {
-            int x, y, z;
-            x4_coords(local, gx, ry, y0, z0, x, y, z);
-            const float* P = (d.pcur != nullptr && *d.pcur == 1) ? d.P2 : d.P;
-            if (d.kind == GK_F32)
-                body_gradient_subtract_x4(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now, P, d.flags, x, y, z);
-            else
-                body_project_bf16_x4(gg, (__nv_bfloat16*)d.u_now, (__nv_bfloat16*)d.v_now, (__nv_bfloat16*)d.w_now, P,
-                                     d.flags, d.pu, d.pv, d.pw, x, y, z);
-            return;
-        }
-        group_extent(GS_PROJECT, d, rx, ry, rz);
-        const uint3 bid = tile_bid(local, rx, ry);
-        if (d.kind == GK_F32)
-            body_gradient_subtract(gg, (float*)d.u_now, (float*)d.v_now, (float*)d.w_now, d.P, d.P2, d.pcur,
-                                   d.flags, bid);
-        else
-            body_project_bf16(gg, (__nv_bfloat16*)d.u_now, (__nv_bfloat16*)d.v_now, (__nv_bfloat16*)d.w_now,
-                              d.P, d.P2, d.pcur, d.flags, d.pu, d.pv, d.pw, bid);
-    });
+    finish_tiles(a);
 
     if (a.starts[GS_DIV * (a.n + 1) + a.n] > 0) {
         if (!group_barrier(a, target)) {
             group_abort(a);
             return;
         }
-        int cur = -1;
-        unsigned mb = 0u;
-        for_tiles(a, GS_DIV, nullptr, 0, [&](int j, int local) {
-            if (j != cur) {
-                if (cur >= 0) block_max_to(mb, &a.grids[cur].status->div_bits);
-                cur = j;
-                mb = 0u;
-            }
-            const GroupGrid& d = a.grids[j];
-            const Grid g = d.g;  // in registers: the stores below cannot alias it
-            const int tpp = group_interior_tpp(g);
-            const int z0 = 1 + (local / tpp) * a.zslab;
-            const int z1 = min(z0 + a.zslab, g.nz - 1);
-            const int f = (local % tpp) * GROUP_TILE + tid;
-            const int L = g.nx - 2;
-            if (f < L * (g.ny - 2)) {
-                int i = g.idx(1 + f % L, 1 + f / L, z0);
-                for (int z = z0; z < z1; ++z, i += g.XY)
-                    mb = max(mb, __float_as_uint(cell_div(g, d.pu, d.pv, d.pw, d.flags, i)));
-            }
-        });
-        if (cur >= 0) block_max_to(mb, &a.grids[cur].status->div_bits);
+        div_tiles(a);
     }
 }
 
 int g_sms = 0;
-int g_occ[6] = {0, 0, 0, 0, 0, 0};  // resident CTAs per SM: project, objects, forcing, adv_vel, adv_rho
+int g_occ[4] = {0, 0, 0, 0};  // resident CTAs per SM: project, objects, forcing, div
 
 int ensure_occupancy() {
     if (g_sms > 0) return 0;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-    const void* ks[5] = {(const void*)k_group_project, (const void*)k_group_objects, (const void*)k_group_forcing,
-                         (const void*)k_group_adv_vel, (const void*)k_group_adv_rho};
-    for (int k = 0; k < 5 && e == cudaSuccess; ++k)
+    const void* ks[4] = {(const void*)k_group_project, (const void*)k_group_objects, (const void*)k_group_forcing,
+                         (const void*)k_group_div};
+    for (int k = 0; k < 4 && e == cudaSuccess; ++k)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_occ[k], ks[k], GROUP_TILE, k == 0 ? 16384 : 0);
     if (e != cudaSuccess) {
         g_sms = 0;
@@ -521,16 +536,12 @@ int ensure_occupancy() {
     return 0;
 }
 
-// per_tile: one CTA per tile, so the block scheduler hands out tiles in index order as CTAs
-// finish and the tiles in flight (and the planes they share) stay close together in L2, where a
-// fixed set of grid-striding CTAs drifts apart; it pays for the gather-heavy velocity advection
-// (1.00 -> 0.88 ms on the 64-grid batch) but not for the light stages, whose short CTAs then
-// cost more to launch than they save (forcing 0.31 -> 0.46 ms).
-int launch_grid_stride(const void* kernel, int total, int occ, const GroupArgs& a, cudaStream_t st,
-                       bool per_tile = false) {
+// One CTA per tile (occ 0): the block scheduler hands out tiles in index order as CTAs finish, and the tiles
+// in flight (and the planes they share) stay close together in L2, where a fixed set of grid-striding
+// CTAs drifts apart.  occ > 0: at most the resident CTAs, each striding over the tiles.
+int launch_tiles(const void* kernel, int total, int occ, const GroupArgs& a, cudaStream_t st) {
     if (total <= 0) return 0;
-    const int cap = occ * g_sms;
-    const int ctas = per_tile || total < cap ? total : cap;
+    const int ctas = occ > 0 && occ * g_sms < total ? occ * g_sms : total;
     float one = 1.0f;  // the density advection's second argument
     void* args[] = {(void*)&a, (void*)&one};
     return (int)cudaLaunchKernel(kernel, dim3((unsigned)ctas), dim3(SB_BX, SB_BY), args, 0, st);
@@ -654,20 +665,20 @@ int launch_tb_solve(GroupTBLaunch& tb, cudaStream_t st) {
 
 int launch_group_step(const GroupArgs& a, const GroupLaunch& L, cudaStream_t st, GroupTBLaunch* tb) {
     int rc = ensure_occupancy();
-    if (!rc) rc = launch_grid_stride((const void*)k_group_objects, L.total[GS_OBJECTS], g_occ[1], a, st);
-    if (!rc) rc = launch_grid_stride((const void*)k_group_forcing, L.total[GS_FORCE], g_occ[2], a, st);
+    if (!rc) rc = launch_tiles((const void*)k_group_objects, L.total[GS_OBJECTS], g_occ[1], a, st);
+    if (!rc) rc = launch_tiles((const void*)k_group_forcing, L.total[GS_FORCE], 0, a, st);
     if (tb == nullptr) {
         if (!rc) rc = launch_project(a, L, st);
     } else {
-        GroupArgs r = a;
-        r.phases = GP_RHS;
-        if (!rc) rc = launch_project(r, L, st);
+        if (!rc) rc = launch_tiles((const void*)k_group_rhs, L.total[GS_RHS], 0, a, st);
+        if (!rc) rc = launch_tiles((const void*)k_group_solve_start, a.n, 0, a, st);
         if (!rc) rc = launch_tb_solve(*tb, st);
-        r.phases = GP_FINISH;
-        if (!rc) rc = launch_project(r, L, st);
+        if (!rc) rc = launch_tiles((const void*)k_group_finish, L.total[GS_PROJECT], 0, a, st);
+        if (!rc) rc = launch_tiles((const void*)k_group_div, L.total[GS_DIV], g_occ[3], a, st);
     }
-    if (!rc) rc = launch_grid_stride((const void*)k_group_adv_vel, L.total[GS_ADV_VEL], g_occ[3], a, st, true);
-    if (!rc) rc = launch_grid_stride((const void*)k_group_adv_rho, L.total[GS_ADV_RHO], g_occ[4], a, st);
+    for (int k = 0; k < 2 && !rc; ++k)
+        rc = launch_group_advect_velocity(a.adv, a.adv_starts[k], a.n, L.adv_total[k], k == 1, st);
+    if (!rc) rc = launch_tiles((const void*)k_group_adv_rho, L.total[GS_ADV_RHO], 0, a, st);
     return rc;
 }
 

@@ -132,13 +132,6 @@ __device__ __forceinline__ unsigned resid_bits(float pc, float bc, float2 c, boo
 // flag word -> table index: bits 0-5 the six fluid-neighbour bits, bit 6 "projectable"
 __device__ __forceinline__ unsigned fidx(unsigned f, int k) { return (f >> (8 * k + 1)) & 0x7fu; }
 
-// Make the tensor map at `map` (global memory, written before the launch) current for the
-// TMA unit's tensor-map reads from this CTA.
-__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map) {
-    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map))
-                 : "memory");
-}
-
 // Cluster barrier: every thread of every CTA of the cluster arrives (release) and waits
 // (acquire); it also orders this CTA's shared-memory accesses like __syncthreads.
 __device__ __forceinline__ void cluster_sync_all() {

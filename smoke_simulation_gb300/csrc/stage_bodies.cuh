@@ -535,51 +535,6 @@ __device__ __forceinline__ void body_project_bf16(const Grid& g, __nv_bfloat16* 
 
 // ---- advection --------------------------------------------------------------------------------
 
-// velocityAdvectionU/V/W (smokeSimulation.cu:527-615), the three fused per staggered index.
-template <typename Ti, typename To>
-__device__ __forceinline__ void body_advect_velocity(const Grid& g, const Ti* __restrict__ u0,
-                                                     const Ti* __restrict__ v0,
-                                                     const Ti* __restrict__ w0, To* __restrict__ u1,
-                                                     To* __restrict__ v1, To* __restrict__ w1,
-                                                     const uint8_t* __restrict__ flags, float dt,
-                                                     uint3 bid) {
-    const int x = 1 + (int)bid.x * SB_BX + (int)threadIdx.x;
-    const int y = 1 + (int)bid.y * SB_BY + (int)threadIdx.y;
-    const int z = 1 + (int)bid.z;
-    if (x >= g.nx || y >= g.ny || z >= g.nz) return;
-    const int i = g.idx(x, y, z);
-    const uint8_t f = flags[i];
-    if (!(f & F_SELF)) return;
-    const bool inx = x <= g.nx - 2, iny = y <= g.ny - 2, inz = z <= g.nz - 2;
-    const bool du = iny && inz && (f & F_XM), dv = inx && inz && (f & F_YM),
-               dw = inx && iny && (f & F_ZM);
-    if (!(du || dv || dw)) return;
-    // The three 8-point averages at one index serve two faces each (avgU: v and w faces, avgV:
-    // u and w, avgW: u and v), so each is evaluated once.
-    const float au = avgU(u0, g, i), av = avgV(v0, g, i), aw = avgW(w0, g, i);
-    if (du) {
-        float xt = (float)x, yt = (float)y + 0.5f, zt = (float)z + 0.5f;
-        xt = xt - dt * ldv(u0, i);
-        yt = yt - dt * av;
-        zt = zt - dt * aw;
-        stv(u1, i, sample_ref<0, 1, 1>(u0, g, xt, yt, zt));
-    }
-    if (dv) {
-        float xt = (float)x + 0.5f, yt = (float)y, zt = (float)z + 0.5f;
-        xt = xt - dt * au;
-        yt = yt - dt * ldv(v0, i);
-        zt = zt - dt * aw;
-        stv(v1, i, sample_ref<1, 0, 1>(v0, g, xt, yt, zt));
-    }
-    if (dw) {
-        float xt = (float)x + 0.5f, yt = (float)y + 0.5f, zt = (float)z;
-        xt = xt - dt * au;
-        yt = yt - dt * av;
-        zt = zt - dt * ldv(w0, i);
-        stv(w1, i, sample_ref<1, 1, 0>(w0, g, xt, yt, zt));
-    }
-}
-
 // advectSmoke (smokeSimulation.cu:617-638) with the NEW velocities.  The reference evaluates
 // the backtrace x + 0.5 - u*dt in double and rounds to float.  With a = x + 0.5 (exact, lowest
 // bit 2^-1) and b = u*dt (a float), the exact a - b needs at most max(e_a - e_b, 0) + 24 bits,
@@ -658,7 +613,7 @@ __device__ __forceinline__ void density_rows(const Grid& g, const T* __restrict_
         const float2 x1 = part(px, bx), y1 = part(py, by), zz1 = part(pz, bz);
         const float2 x0 = __ffma2_rn(x1, mone, both(1.0f)), y0 = __ffma2_rn(y1, mone, both(1.0f)),
                      zz0 = __ffma2_rn(zz1, mone, both(1.0f));
-        // trilinear_ref, term for term
+        // the eight terms in the reference's order
         const float2 w00 = __fmul2_rn(x0, y0), w10 = __fmul2_rn(x1, y0), w01 = __fmul2_rn(x0, y1), w11 = __fmul2_rn(x1, y1);
         float2 s = __fmul2_rn(__fmul2_rn(w00, zz0), c000);
         s = __ffma2_rn(__fmul2_rn(__fmul2_rn(w10, zz0), c100), one2, s);

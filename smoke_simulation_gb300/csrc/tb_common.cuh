@@ -111,5 +111,12 @@ bool encode_3d_box(CUtensorMap* m, const void* base, bool is_u8, const Grid& g, 
 // A map over the sweep codes (16 bits per 2 x 2 patch), boxes of box_w x box_h x 1 patches.
 bool encode_codes(CUtensorMap* m, const void* base, const Grid& g, int box_w, int box_h);
 
+// Make the tensor map at `map` (global memory, written before the launch) current for the
+// TMA unit's tensor-map reads from this CTA.
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map))
+                 : "memory");
+}
+
 }  // namespace tb
 }  // namespace smk
