@@ -271,7 +271,7 @@ k_resident_sor(const __grid_constant__ ResidentArgs a, float* __restrict__ P, co
     int group = 0;
     bool bad = false;
     for (int sweep = 0; sweep < max_sweeps && !bad; ++sweep) {
-        if (tol > 0.0f && sweep % check_every == 0) {
+        if (tol != 0.0f && sweep % check_every == 0) {  // below 0: residuals are recorded and end nothing
             unsigned m = 0u;
 #pragma unroll
             for (int s = 0; s < NS; ++s)

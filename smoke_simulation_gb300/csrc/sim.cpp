@@ -25,6 +25,10 @@ using namespace smk;
 
 namespace {
 
+// The autotuner times the resident solve over this many tolerance groups.
+constexpr int TUNE_GROUPS = 4;
+constexpr size_t TUNE_STATUS_BYTES = sizeof(StepStatus) + TUNE_GROUPS * sizeof(unsigned);
+
 thread_local std::string g_last_error;
 
 // A stored field as BF16 (the allocation is 2 bytes per element in the BF16 storage form).
@@ -220,7 +224,7 @@ int smk_sim::alloc() {
     SMK_CUDA(cudaMalloc((void**)&status, status_bytes + exchange_bytes));
     SMK_CUDA(cudaMemset(status, 0, status_bytes + exchange_bytes));
     exchange = reinterpret_cast<unsigned char*>(status) + status_bytes;
-    SMK_CUDA(cudaMalloc((void**)&tune_status, sizeof(StepStatus) + sizeof(unsigned)));
+    SMK_CUDA(cudaMalloc((void**)&tune_status, TUNE_STATUS_BYTES));
     for (auto& e : ev) SMK_CUDA(cudaEventCreate(&e));
     SMK_CUDA(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
     SMK_CUDA(cudaStreamCreateWithFlags(&body_stream, cudaStreamNonBlocking));
@@ -1419,9 +1423,11 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
     const int now = sim->index_now;
     const OmegaSplit os = omega_split(sim->p.omega);
     constexpr int RESIDENT = -1;  // the resident solve, where the grid has one
-    // microseconds per iteration of one candidate, issued as a step issues it
+    // microseconds per iteration of one candidate, issued as a step issues it.  The resident solve reads and
+    // writes the whole state once a launch, so it is timed over a solve's iterations: over four of them it lost
+    // to one pass per launch (240 x 24 x 150: 10.6 us an iteration that way, 7.1 resident over thirty).
     auto time_it = [&](int depth, int zc, float* us) -> int {
-        const int iters = 4;
+        const int iters = depth == RESIDENT ? std::max(1, std::min(sim->p.max_sweeps, 32)) : 4;
         auto run = [&]() -> int {
             if (depth == RESIDENT) {
                 SMK_CUDA(cudaMemsetAsync(sim->exchange, 0, sim->exchange_bytes, st));
@@ -1591,7 +1597,7 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
     int nl = 0;
     // tolerance -1: the check launch records its residual but never ends the timed solve
     auto run_group = [&](int d, int rows, int zc) -> int {
-        if (use_tol) SMK_CUDA(cudaMemsetAsync(sim->tune_status, 0, sizeof(StepStatus) + sizeof(unsigned), st));
+        if (use_tol) SMK_CUDA(cudaMemsetAsync(sim->tune_status, 0, TUNE_STATUS_BYTES, st));
         for (int h = 0; h < 2 * G;) {
             const int nh = (h == 0 && (2 * G) % d != 0) ? (2 * G) % d : d;
             const bool in_a = saved.p == nullptr || (nl & 1) == 0;
@@ -1655,23 +1661,24 @@ int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sw
             best_z = c.zc;
         }
     }
-    // the resident solve, where the grid has one: a group of sweeps as one launch
+    // the resident solve, where the grid has one: up to four groups as one launch, as it reads and writes the
+    // pressure once a launch
     bool resident = false;
-    if (sim->res_p_fits && sim->p.solver == SMK_SOLVER_RBSOR) {
+    if (sim->res_p_fits && sim->p.solver == SMK_SOLVER_RBSOR && saved.p != nullptr) {
         float us = 1e30f;
+        const int sweeps = std::max(1, std::min(sim->p.max_sweeps, TUNE_GROUPS * G));
         for (int round = 0; round < 4; ++round) {  // the first one warms up
             SMK_CUDA(cudaMemsetAsync(sim->exchange, 0, sim->exchange_bytes, st));
-            SMK_CUDA(cudaMemsetAsync(sim->tune_status, 0, sizeof(StepStatus) + sizeof(unsigned), st));
+            SMK_CUDA(cudaMemsetAsync(sim->tune_status, 0, TUNE_STATUS_BYTES, st));
             SMK_CUDA(cudaEventRecord(e0, st));
-            // a tolerance no residual meets but zero: the check runs, the sweeps go on
-            if (launch_resident_sor(g, sim->res_p, sim->exchange, sim->kerr, sim->P, sim->b, sim->flags, wacc, G, G,
-                                    use_tol ? 1e-38f : 0.0f, sim->tune_status, st) != 0)
+            if (launch_resident_sor(g, sim->res_p, sim->exchange, sim->kerr, sim->P, sim->b, sim->flags, wacc, sweeps, G,
+                                    use_tol ? -1.0f : 0.0f, sim->tune_status, st) != 0)
                 return fail(SMK_ERR_CUDA, "resident solve launch failed");
             SMK_CUDA(cudaEventRecord(e1, st));
             SMK_CUDA(cudaEventSynchronize(e1));
             float ms = 0.0f;
             SMK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (round > 0) us = std::min(us, 1e3f * ms / G);
+            if (round > 0) us = std::min(us, 1e3f * ms / sweeps);
         }
         resident = us < best;
         if (resident) best = us;
