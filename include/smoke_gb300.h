@@ -294,9 +294,9 @@ int smk_batch_autotune(smk_batch* batch, int* ctas_per_sm, float* us_per_sweep);
 int smk_batch_get_schedule(const smk_batch* batch, int* ctas_per_sm, int* zslab, long long* wave_bytes);
 int smk_batch_set_schedule(smk_batch* batch, int ctas_per_sm, int zslab, long long wave_bytes);
 /* The grouped form's blocked solve: zchunk > 0 replaces the cooperative kernel's colour passes
- * by launches of the temporally blocked sweep kernel over every member's tiles (3 sweeps per
- * launch, z-chunks of `zchunk` planes, the tolerance groups as a device-side loop in the
- * captured step), when every member has a tolerance rule with the same group size and sweep
+ * by launches of the temporally blocked sweep kernel over every member's tiles (2 sweeps per
+ * launch, z-chunks of at most `zchunk` planes: fewer where the batch has too few tiles for the chip; the
+ * tolerance groups as a device-side loop in the captured step), when every member has a tolerance rule with the same group size and sweep
  * cap; 0 = colour passes.  smk_batch_set_schedule resets it to 0.  Results do not depend on
  * it. */
 int smk_batch_set_blocked(smk_batch* batch, int zchunk);
@@ -356,7 +356,7 @@ int smk_server_set_mode(smk_server* server, int mode);
 /* smk_set_graph_loops for the requests admitted from now on (default off: with many request
  * graphs in flight at once, the loop's per-iteration cost exceeds the launches it saves). */
 int smk_server_set_graph_loops(smk_server* server, int enable);
-/* GROUPED form: the blocked solve, with z-chunks of `zchunk` planes, for the ticks whose requests
+/* GROUPED form: the blocked solve, with z-chunks of at most `zchunk` planes, for the ticks whose requests
  * share a tolerance group size and sweep cap (smk_batch_set_blocked; default 137; 0 = cooperative
  * colour passes for every tick). */
 int smk_server_set_blocked(smk_server* server, int zchunk);

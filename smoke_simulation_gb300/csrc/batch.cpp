@@ -19,6 +19,8 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <functional>
+#include <queue>
 #include <string>
 #include <utility>
 #include <vector>
@@ -260,8 +262,68 @@ int fill_advection(smk_sim* const* sims, int n, TableImage& t) {
     }
 }
 
+// The blocked solve's z-chunk: the one of at most `cap` planes with which the launch's CTAs, longest first
+// on the first free of the SMs (one CTA each), are done soonest; a CTA marches its chunk and the halo of T
+// planes on both sides.  The measured steps follow this sum within a few percent (10 grids of 26^3 to 121^3,
+// us a step by planes: 8 1213, 17 1001, 27 1216, 64 2040, 137 3291; 12 of 61^3 to 63^3: 10 835, 12 672,
+// 17 738, 137 1414; 64 of 32^3 to 128^3: 17 6263, 64 5294, 137 5347).  From four tiles an SM on the cap stays.
+struct ZChunk {
+    std::vector<int> key;  // cap, then (nz, columns) of every grid: the choice below is theirs
+    int planes = 0;
+};
+int blocked_zchunk(smk_sim* const* sims, int n, int cap, ZChunk& memo) {
+    int longest = 1, sms = 0;
+    for (int i = 0; i < n; ++i) longest = std::max(longest, sims[i]->g.nz);
+    cap = std::min(cap, longest);
+    std::vector<int> key{cap};
+    long long tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        const int nz = sims[i]->g.nz, columns = group_tb_columns(sims[i]->g);
+        key.push_back(nz);
+        key.push_back(columns);
+        tiles += (long long)columns * ((nz + cap - 1) / cap);
+    }
+    if (key == memo.key) return memo.planes;
+    if (group_occupancy(nullptr, nullptr, &sms) != 0 || sms < 1) return cap;  // the launch reports it
+    memo.planes = cap;
+    if (tiles < 4LL * sms) {
+        const int halo = 2 * GROUP_TB_DEPTH + 1;
+        long long best = -1;
+        int last = 0;
+        for (int k = 1; k <= longest; ++k) {
+            const int zc = std::min(cap, (longest + k - 1) / k);
+            if (k > 1 && zc < 4) break;
+            if (zc == last) continue;
+            last = zc;
+            std::vector<int> cost;
+            for (int i = 0; i < n; ++i)
+                for (int z = 0; z < key[1 + 2 * i]; z += zc)
+                    cost.insert(cost.end(), key[2 + 2 * i], std::min(zc, key[1 + 2 * i] - z) + halo);
+            if ((long long)cost.size() > 16LL * sms) break;
+            std::sort(cost.begin(), cost.end(), std::greater<int>());
+            std::priority_queue<long long, std::vector<long long>, std::greater<long long>> sm;
+            long long end = 0;
+            for (size_t i = 0; i < cost.size(); ++i) {
+                long long at = cost[i];
+                if ((int)sm.size() == sms) {
+                    at += sm.top();
+                    sm.pop();
+                }
+                sm.push(at);
+                end = std::max(end, at);
+            }
+            if (best < 0 || end < best) {
+                best = end;
+                memo.planes = zc;
+            }
+        }
+    }
+    memo.key.swap(key);
+    return memo.planes;
+}
+
 int build_table(smk_sim* const* sims, int n, const float* dts, float dt_all, const GroupSchedule& sch,
-                TableImage& t) {
+                TableImage& t, ZChunk& zchunk) {
     t.grids.resize(n);
     t.boxes.clear();
     t.spheres.clear();
@@ -271,7 +333,7 @@ int build_table(smk_sim* const* sims, int n, const float* dts, float dt_all, con
     t.blocked = sch.blocked_zchunk > 0 && blocked_eligible(sims, n);
     if (t.blocked) {
         const size_t rb = group_tb_record_bytes();
-        t.tb_zchunk = sch.blocked_zchunk;
+        t.tb_zchunk = blocked_zchunk(sims, n, sch.blocked_zchunk, zchunk);
         t.tb_check_every = sims[0]->p.check_every;
         t.tb_max_sweeps = sims[0]->p.max_sweeps;
         t.tb_recs.assign(rb * n, 0);
@@ -467,7 +529,8 @@ int grouped_step(smk_batch* b, const float* dts, float dt_all, cudaStream_t st) 
     if (!slot) {
         slot = b->slots[0].used <= b->slots[1].used ? &b->slots[0] : &b->slots[1];
         TableImage t;
-        int rc = build_table(b->sims.data(), n, dts, dt_all, b->sched, t);
+        ZChunk zchunk;
+        int rc = build_table(b->sims.data(), n, dts, dt_all, b->sched, t, zchunk);
         if (rc) return rc;
         // the slot being replaced may still be read by a step in flight
         SMK_CUDA(cudaDeviceSynchronize());
@@ -674,6 +737,7 @@ struct GroupRunner {
     static constexpr int RING = 4;
     Slot ring[RING];
     int next = 0;
+    ZChunk zchunk;  // of the last tick's grids
 };
 
 GroupRunner* group_runner_create() {
@@ -716,7 +780,7 @@ int group_runner_step(GroupRunner* r, smk_sim* const* sims, const float* dts, in
     for (int i = 0; i < n; ++i)
         if (sims[i]->mask_dirty || sims[i]->obstacles_dirty) k += sims[i]->prepare_mask(st);
     TableImage t;
-    int rc = build_table(sims, n, dts, 0.0f, sched, t);
+    int rc = build_table(sims, n, dts, 0.0f, sched, t, r->zchunk);
     if (rc) return rc;
     GroupRunner::Slot& sl = r->ring[r->next];
     r->next = (r->next + 1) % GroupRunner::RING;
@@ -881,6 +945,7 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
     if (!grouped_eligible(b)) return smk_fail(SMK_ERR_INVALID, "the batch cannot use the grouped form");
     DeviceGuard dg(b->device);
     SMK_CUDA(cudaDeviceSynchronize());
+    ZChunk zchunk;
     const int n = (int)b->sims.size();
     for (smk_sim* s : b->sims) {
         int pc = 0;
@@ -913,7 +978,7 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
         for (long long wb : waves) {
             if (rc) break;
             TableImage t;
-            rc = build_table(b->sims.data(), n, nullptr, 0.0f, GroupSchedule{0, zs, wb}, t);
+            rc = build_table(b->sims.data(), n, nullptr, 0.0f, GroupSchedule{0, zs, wb}, t, zchunk);
             if (rc) break;
             if (wb > 0 && t.nwaves == 1) continue;  // same schedule as one wave
             for (GroupGrid& d : t.grids) {
@@ -960,11 +1025,11 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
     }
     // the blocked solve (when every member can use it): launches over all grids' tiles,
     // timed without tolerance checks, reading P and writing the scratch P2 (no status, no pcur)
-    const int zchunks[] = {17, 27, 37, 57, 117, 137, 257};  // 10 m - 13: no padding of the 10-plane unroll
+    const int zchunks[] = {17, 27, 37, 57, 117, 137, 257};
     if (!rc && blocked_eligible(b->sims.data(), n)) {
         for (int zc : zchunks) {
             TableImage t;
-            rc = build_table(b->sims.data(), n, nullptr, 0.0f, GroupSchedule{0, 4, 0, zc}, t);
+            rc = build_table(b->sims.data(), n, nullptr, 0.0f, GroupSchedule{0, 4, 0, zc}, t, zchunk);
             if (rc) break;
             const size_t rb = group_tb_record_bytes();
             for (int i = 0; i < n; ++i) {
@@ -973,7 +1038,7 @@ int smk_batch_autotune(smk_batch* b, int* ctas_per_sm, float* us_per_sweep) {
                 wacc[0] = 0.0f;
                 for (int a = 1; a <= 6; ++a) wacc[a] = (float)sm->p.omega / (float)a;
                 group_tb_fill(&t.tb_recs[rb * i], sm->maps, sm->g, sm->P, sm->P2, nullptr, nullptr, sm->kerr, wacc,
-                              sm->p.tol, zc);
+                              sm->p.tol, t.tb_zchunk);
             }
             if (cap < t.bytes) {
                 if (dev) cudaFree(dev);

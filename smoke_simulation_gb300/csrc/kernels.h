@@ -137,6 +137,8 @@ int launch_sweep_tb(const SweepMaps* m, const Grid& g, bool in_is_a, float* Pout
 // tensor maps, buffers and tolerance), tiles of all grids in one launch.
 constexpr int GROUP_TB_DEPTH = 4;
 size_t group_tb_record_bytes();
+// Tiles of a grid in x-y (each cut into z-chunks).
+int group_tb_columns(const Grid& g);
 // Fill one record (rec: group_tb_record_bytes(), 64-byte aligned in the device copy); returns
 // the grid's tile count for `zchunk`-plane chunks.
 int group_tb_fill(void* rec, const SweepMaps* m, const Grid& g, float* P, float* P2, StepStatus* status, int* pcur,

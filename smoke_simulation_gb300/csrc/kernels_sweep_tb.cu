@@ -1400,6 +1400,11 @@ void launch_build_codes(const Grid& g, const uint8_t* flags, uint16_t* codes, cu
 
 size_t group_tb_record_bytes() { return sizeof(GroupTBGrid); }
 
+int group_tb_columns(const Grid& g) {
+    constexpr int T = GROUP_TB_DEPTH;
+    return sweep_windows(g.nx, 2 * TB_TX, T) * sweep_windows(g.ny, PairGeom<T>::ROWS, T);
+}
+
 int group_tb_fill(void* rec, const SweepMaps* m, const Grid& g, float* P, float* P2, StepStatus* status, int* pcur,
                   int* kerr, const float* wacc7, float tol, int zchunk) {
     constexpr int T = GROUP_TB_DEPTH;

@@ -22,7 +22,7 @@ def _member(i):
 
 
 @pytest.mark.parametrize("count", [1, 33, 70])
-@pytest.mark.parametrize("blocked", [True, False])
+@pytest.mark.parametrize("blocked", [0, 17, 137])  # the cap of the z-chunks: few grids get shorter ones
 def test_grouped_tiles_equal_alone(gpu, count, blocked):
     scs = [_member(i) for i in range(count)]
     kinds = [STORAGES[(i // 2) % 3] for i in range(count)]
@@ -30,7 +30,8 @@ def test_grouped_tiles_equal_alone(gpu, count, blocked):
     b = [smk.from_scene(sc, report_div=1, storage=k) for sc, k in zip(scs, kinds)]
     batch = smk.Batch(a, mode=smk.BATCH_GROUPED)
     if blocked:
-        batch.set_blocked(17)
+        batch.set_blocked(blocked)
+        assert batch.blocked() == blocked
     else:
         batch.set_schedule(0, 4, 0)
     for _ in range(3):
