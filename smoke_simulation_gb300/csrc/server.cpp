@@ -61,6 +61,7 @@ struct Request {
     int error = SMK_OK;
     size_t bytes = 0;
     bool cancel = false;  // smk_server_cancel on an active request: no new steps, then released
+    bool alone = false;   // STREAMS form: the only request, its solves take the whole chip
     smk_sim* sim = nullptr;
     // STREAMS form: the request's own stream and two step slots (issue / collect)
     cudaStream_t stream = nullptr;
@@ -308,16 +309,21 @@ static void note_admission(smk_server* s, Request* r) {
     s->peak_bytes = std::max(s->peak_bytes, s->used);
 }
 
+// The form of r's solves: resident over the whole chip when it is the only request, else blocked over its share
+// of the SMs next to the requests that are active or waiting (cooperative kernels would run one by one).
+static void share_chip(smk_server* s, Request* r, bool alone) {
+    double total = (double)r->nx * r->ny * r->nz;
+    for (const Request* q : s->active)
+        if (q != r) total += (double)q->nx * q->ny * q->nz;
+    for (const Request* q : s->queue) total += (double)q->nx * q->ny * q->nz;
+    r->alone = alone;
+    r->sim->resident_ok = alone;
+    r->sim->choose_sweep(r->sim->sweep_share(total));
+}
+
 static int admit(smk_server* s, Request* r) {
     int rc = smk_create(r->nx, r->ny, r->nz, &r->params, &r->sim);
-    if (rc == SMK_OK && s->mode == SMK_SERVE_STREAMS) {
-        // its steps run next to those of the requests that are active or waiting
-        double total = (double)r->nx * r->ny * r->nz;
-        for (const Request* q : s->active) total += (double)q->nx * q->ny * q->nz;
-        for (const Request* q : s->queue) total += (double)q->nx * q->ny * q->nz;
-        r->sim->choose_sweep(r->sim->sweep_share(total));
-        r->sim->resident_ok = false;
-    }
+    if (rc == SMK_OK && s->mode == SMK_SERVE_STREAMS) share_chip(s, r, s->active.empty() && s->queue.empty());
     if (rc == SMK_OK) rc = smk_set_graph_loops(r->sim, s->graph_loops);
     if (rc == SMK_OK && !r->mask.empty()) rc = smk_set_solid_mask(r->sim, r->mask.data());
     for (size_t k = 0; rc == SMK_OK && k < r->boxes.size() / 9; ++k) {
@@ -412,6 +418,30 @@ static void collect_req(smk_server* s, Request* r, int k) {
     s->cell_updates += (double)r->nx * r->ny * r->nz;
 }
 
+// The next step of r on its own stream; a failure marks the request.
+static void issue_step(smk_server* s, Request* r) {
+    if (r->steps_issued >= r->steps || r->cancel) return;
+    const int k = r->steps_issued & 1;
+    if (r->pending[k]) {  // its previous use is still in flight (not collected yet)
+        if (cudaEventSynchronize(r->ev_end[k]) != cudaSuccess) {
+            r->error = SMK_ERR_CUDA;
+            r->state = SMK_REQ_FAILED;
+            return;
+        }
+        collect_req(s, r, k);
+    }
+    cudaEventRecord(r->ev_start[k], r->stream);
+    int rc = smk_step(r->sim, r->dt, r->stream);
+    cudaEventRecord(r->ev_end[k], r->stream);
+    if (rc != SMK_OK) {
+        r->error = rc;
+        r->state = SMK_REQ_FAILED;
+        return;
+    }
+    r->pending[k] = true;
+    r->steps_issued++;
+}
+
 static int tick_streams(smk_server* s) {
     // (1) collect finished steps and retire finished requests.  A request keeps at most one
     // step in flight while the next is issued: the step issued two ticks ago is waited for,
@@ -449,7 +479,18 @@ static int tick_streams(smk_server* s) {
         }
     }
     s->active.swap(still);
-    // (2) admit in arrival order while memory and slots allow
+    // (2) one step per active request, each on its own stream.  A request left alone takes the whole chip when
+    // its remaining steps pay for the new graphs, and gives it back when another arrives (51^3, 33 steps: 12.7 ms
+    // in its share, 7.3 alone).
+    for (Request* r : s->active) {
+        const bool alone = s->active.size() == 1 && s->queue.empty();
+        if (alone != r->alone && r->state == SMK_REQ_ACTIVE && (!alone || r->steps - r->steps_issued >= 8))
+            share_chip(s, r, alone);
+    }
+    for (Request* r : s->active) issue_step(s, r);
+    // (3) admit in arrival order while memory and slots allow.  A request's first step is issued as soon as it
+    // is admitted: the GPU runs it and the steps above while the host builds the next request's fields
+    // (a burst of 8 requests of 48^3 to 192^3: the first step began after 17 ms of admissions).
     while (!s->queue.empty() && (int)s->active.size() < s->max_active &&
            s->used + s->queue.front()->bytes <= s->budget) {
         Request* r = s->queue.front();
@@ -457,32 +498,10 @@ static int tick_streams(smk_server* s) {
         if (admit(s, r) == SMK_OK) {
             s->active.push_back(r);
             note_admission(s, r);
+            issue_step(s, r);
         }
     }
     s->peak_queued = std::max(s->peak_queued, (int)s->queue.size());
-    // (3) one step per active request, each on its own stream
-    for (Request* r : s->active) {
-        if (r->steps_issued >= r->steps || r->cancel) continue;
-        const int k = r->steps_issued & 1;
-        if (r->pending[k]) {  // its previous use is still in flight (not collected yet)
-            if (cudaEventSynchronize(r->ev_end[k]) != cudaSuccess) {
-                r->error = SMK_ERR_CUDA;
-                r->state = SMK_REQ_FAILED;
-                continue;
-            }
-            collect_req(s, r, k);
-        }
-        cudaEventRecord(r->ev_start[k], r->stream);
-        int rc = smk_step(r->sim, r->dt, r->stream);
-        cudaEventRecord(r->ev_end[k], r->stream);
-        if (rc != SMK_OK) {
-            r->error = rc;
-            r->state = SMK_REQ_FAILED;
-            continue;
-        }
-        r->pending[k] = true;
-        r->steps_issued++;
-    }
     // drop requests that failed while stepping
     std::vector<Request*> ok;
     for (Request* r : s->active) {
