@@ -1520,6 +1520,13 @@ static int autotune_velocity_sweep(smk_sim* sim, int* depth_out, int* zchunk_out
 int smk_autotune(smk_sim* sim, int* depth_out, int* zchunk_out, float* us_per_sweep_out) {
     if (!sim) return fail(SMK_ERR_INVALID, "sim is null");
     DeviceGuard dg(sim->device);
+    if (sim->mask_dirty) {
+        // before the first step nothing is projectable: the sweeps would be timed without their work, where one
+        // pass per launch looks best (256^3 REFERENCE: 41 us an iteration so, 171 in a step; blocked 83).  The step
+        // builds them again, after the obstacles.
+        launch_build_flags(sim->g, sim->s, sim->flags, nullptr);
+        launch_build_codes(sim->g, sim->flags, sim->codes, nullptr);
+    }
     if (sim->p.projection == SMK_PROJECT_REFERENCE)
         return autotune_velocity_sweep(sim, depth_out, zchunk_out, us_per_sweep_out);
     const Grid& g = sim->g;
