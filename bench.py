@@ -332,7 +332,7 @@ def main():
         ncl = (rows >> 9) & 0xF
         kname = "k_sweep_tb_ycl<%d> (%s)" % (depth, "clusters of %d" % ncl if ncl else "one cluster spanning y")
     else:
-        kname = "k_sweep_tb<%d, %d>" % (depth, rows)
+        kname = "k_sweep_pair<%d>" % depth if rows == 2 else "k_sweep_tb<%d, %d>" % (depth, rows)
 
     # warm-up steps (graph capture, caches); the timed segments restart from the initial state
     for _ in range(max(args.warmup, 0)):

@@ -200,7 +200,9 @@ long long smk_launch_count(const smk_sim* sim);
 /* Pressure sweep kernel (PRESSURE projection).  depth 0: one colour pass per launch.
  * depth 2, 4 or 6: temporally blocked, `depth` colour passes per pass over HBM, the grid
  * cut into z-chunks of `zchunk` planes (>= 1).  A new simulation has the shape that fits its grid
- * (a request of a server: its share of the GPU).  Results are bit-identical for every choice; only
+ * (a request of a server: its share of the GPU); until a shape is set, a grid whose fields fit the
+ * chip's shared memory (up to about 128^3 cells) runs its whole solve in one resident launch instead,
+ * unless it is stepped next to others (a server's streams, a batch's branches).  Results are bit-identical for every choice; only
  * speed differs.  No counterpart in the reference (its projection is fixed,
  * smokeSimulation.cu:795-801). */
 int smk_set_sweep_kernel(smk_sim* sim, int depth, int zchunk);
@@ -221,9 +223,10 @@ int smk_get_sweep_shape(const smk_sim* sim, int* depth, int* rows, int* zchunk);
  * as the reference launches it; depth 2 or 4: temporally blocked, `depth` colour passes per pass
  * over HBM on z-chunks of `zchunk` planes (0: chosen from the grid), with the simulation's pressure
  * buffers as scratch (a later PRESSURE step then restarts its pressure from zero).  Until it is
- * called the grid decides: blocked with depth 4 above about 110^3 cells while no PRESSURE step has
- * left a pressure in those buffers, else one pass per launch.  smk_autotune times them and picks the
- * fastest.  Results are bit-identical for every choice.  FP32 storage only.
+ * called the grid decides: all passes in one resident launch where the faces fit the chip's shared
+ * memory (up to about 128^3 cells; smk_get_velocity_sweep gives depth 0 then), above it blocked with
+ * depth 4 while no PRESSURE step has left a pressure in those buffers, else one pass per launch.
+ * smk_autotune times them and picks the fastest.  Results are bit-identical for every choice.  FP32 storage only.
  * smk_get_velocity_sweep gives the kernel the next step uses.  No counterpart in the reference's API. */
 int smk_set_velocity_sweep(smk_sim* sim, int depth, int zchunk);
 int smk_get_velocity_sweep(const smk_sim* sim, int* depth, int* zchunk);
@@ -249,10 +252,11 @@ int smk_set_vector_stages(smk_sim* sim, int enable);
  * the separate pass (smk_stats.subtract_fused reports which way a step went).  Reference: the
  * face updates inside every colour pass of divergence(), smokeSimulation.cu:384-391. */
 int smk_set_fused_subtract(smk_sim* sim, int enable);
-/* Time the blocked sweep kernel's shapes (depth, patch rows) and z-chunk sizes on this simulation's buffers and
- * keep the fastest (cached per grid shape and device for the process).  With the REFERENCE
- * projection it times the velocity sweep instead (one colour pass per launch, or the blocked
- * kernel with depth 2 or 4 over its z-chunks; smk_set_velocity_sweep) and reports the time per
+/* Time the blocked sweep kernel's shapes (depth, patch rows) and z-chunk sizes, and the resident solve
+ * where the grid has one, on this simulation's buffers and keep the fastest (cached per grid shape and
+ * device for the process; where the resident solve wins, depth and zchunk are the shape it replaces).  With
+ * the REFERENCE projection it times the velocity sweep instead (one colour pass per launch, the resident
+ * solve, or the blocked kernel with depth 2 or 4 over its z-chunks; smk_set_velocity_sweep) and reports the time per
  * iteration.  Synchronises; does not change the simulation's results.  Outputs may be NULL;
  * us_per_sweep is -1 on a cache hit.  No counterpart in the reference. */
 int smk_autotune(smk_sim* sim, int* depth, int* zchunk, float* us_per_sweep);
@@ -444,7 +448,7 @@ int smk_proxy_planes(const float view_origin[3], const float view_dir[3], const 
 int smk_inject_alloc_failures(int count);
 /* Testing: the next cooperative grouped-projection launch made outside a graph capture (batch
  * GROUPED form with graphs off) has its CTA 0 skip its arrival at grid barrier `barrier`
- * (1-based; 0 cancels a pending injection), and its barrier waits give up after wait_ms
+ * (1-based; 0 cancels a pending injection; the blocked solve has no such barriers), and its barrier waits give up after wait_ms
  * (1..10000) instead of 2 s: every wait on that barrier runs out, every CTA leaves the kernel, and
  * the members' next synchronisation reports SMK_ERR_TIMEOUT.  No device fault is involved; the
  * context stays usable.  smk_barrier_timeout_report synchronises the device and gives, for that

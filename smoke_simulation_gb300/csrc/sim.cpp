@@ -200,8 +200,9 @@ int smk_sim::alloc() {
     if (!bf16) {
         vmaps = create_vsweep_maps(g, u, v, w, P, P2, b, flags);
         if (!vmaps) return fail(SMK_ERR_CUDA, "could not encode the TMA tensor maps of the velocity sweep kernel");
-        // blocked above about 110^3: 256^3 x 30 iterations 2.6 ms (5.2 ms with one pass per launch);
-        // below it a march has too few planes to fill the SMs (80^3: 17 us per 4 passes either way)
+        // blocked above about 110^3, where no resident plan fits (resident_velocity comes first):
+        // 256^3 x 30 iterations 2.6 ms (5.2 ms with one pass per launch); below it a march has too few
+        // planes to fill the SMs (80^3: 17 us per 4 passes either way)
         const int zc = default_vsweep_zchunk(g, 4);
         if (vsweep_launch_us(g, 4, zc, device_sms()) < 0.9f * 4.0f * one_pass_us(g))
             vsweep_auto = VelocitySweep{4, zc, default_vsweep_zchunk(g, 2)};

@@ -89,3 +89,26 @@ def test_forms_may_change_between_steps_and_streams(gpu):
     pair.close()
     for s in (a, b, c):
         s.close()
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_resident_solves_on_several_streams_at_once(gpu, graphs):
+    """Simulations stepped on their own streams, their resident solves (each a cooperative launch over the
+    whole chip) in flight together: the same fields as stepped one after another."""
+    import torch
+    scs = [S.small_scene(60 + 9 * i, 52, 47 + 5 * i, seed=30 + i, iterations=12, obstacles=1, scheme=i % 2, tol=0.0)
+           for i in range(4)]
+    a, b = [smk.from_scene(sc) for sc in scs], [smk.from_scene(sc) for sc in scs]
+    streams = [torch.cuda.Stream() for _ in scs]
+    for s in a:
+        s.set_graphs(graphs)
+    for _ in range(12):
+        for s, sc, st in zip(a, scs, streams):
+            s.step(sc.dt, st.cuda_stream)
+    torch.cuda.synchronize()
+    for s, sc in zip(b, scs):
+        for _ in range(12):
+            s.step(sc.dt)
+    for i, (x, y) in enumerate(zip(a, b)):
+        x.sync()
+        assert H.first_mismatch(x.read_state(), y.read_state()) == "", i
