@@ -21,6 +21,8 @@ void launch_fill_smoke(const Grid& g, T* rho0, T* rho1, const SphereObj* sp, int
 bool sphere_bounds(const Grid& g, const SphereObj* sp, int ns, int a0[3], int a1[3]);
 void launch_fill_obstacles(const Grid& g, uint8_t* s, const ObstacleObj* ob, int no, cudaStream_t st);
 // Neighbour flags from the mask; zeroes the pressure where a cell is not projectable.
+void launch_default_mask(const Grid& g, uint8_t* s, cudaStream_t st);
+void launch_normalise_mask(const Grid& g, uint8_t* s, cudaStream_t st);
 void launch_build_flags(const Grid& g, const uint8_t* s, uint8_t* flags, cudaStream_t st);
 
 // Moving-obstacle boundary (smk_params.obstacle_velocity): faces touching a cell of `last`

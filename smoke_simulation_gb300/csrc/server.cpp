@@ -490,7 +490,7 @@ static int tick_streams(smk_server* s) {
     for (Request* r : s->active) issue_step(s, r);
     // (3) admit in arrival order while memory and slots allow.  A request's first step is issued as soon as it
     // is admitted: the GPU runs it and the steps above while the host builds the next request's fields
-    // (a burst of 8 requests of 48^3 to 192^3: the first step began after 17 ms of admissions).
+    // (a burst of 8 requests of 51^3 to 183^3: the first step would begin after 11 ms of admissions).
     while (!s->queue.empty() && (int)s->active.size() < s->max_active &&
            s->used + s->queue.front()->bytes <= s->budget) {
         Request* r = s->queue.front();

@@ -234,11 +234,8 @@ int smk_sim::alloc() {
     SMK_CUDA(cudaEventCreateWithFlags(&rb_join, cudaEventDisableTiming));
     if (prepare_sweep_kernels() != 0 || prepare_vsweep_kernels() != 0 || prepare_resident_kernels() != 0)
         return fail(SMK_ERR_CUDA, "sweep kernel configuration failed");
-    // initializeVolume's mask: fluid except the y = 0 floor (smokeSimulation.cu:200-207)
-    std::vector<uint8_t> host((size_t)g.nx * g.ny * g.nz, 1);
-    for (int z = 0; z < g.nz; ++z)
-        for (int x = 0; x < g.nx; ++x) host[(size_t)x + (size_t)z * g.nx * g.ny] = 0;
-    return upload_mask(host.data());
+    launch_default_mask(g, s, nullptr);
+    return mask_set();
 }
 
 void smk_sim::release() {
@@ -269,10 +266,16 @@ void smk_sim::release() {
 }
 
 int smk_sim::upload_mask(const uint8_t* host) {
-    std::vector<uint8_t> norm((size_t)g.nx * g.ny * g.nz);
-    for (size_t i = 0; i < norm.size(); ++i) norm[i] = host[i] ? 1 : 0;
-    auto m = copy3d(s, g.X, g.ny + 1, norm.data(), g.nx, g.ny, g.nx, g.ny, g.nz, cudaMemcpyHostToDevice);
+    auto m = copy3d(s, g.X, g.ny + 1, host, g.nx, g.ny, g.nx, g.ny, g.nz, cudaMemcpyHostToDevice);
     SMK_CUDA(cudaMemcpy3D(&m));
+    launch_normalise_mask(g, s, nullptr);
+    return mask_set();
+}
+
+// The mask is complete before any stream's next step.
+int smk_sim::mask_set() {
+    SMK_CUDA(cudaGetLastError());
+    SMK_CUDA(cudaStreamSynchronize(nullptr));
     mask_dirty = true;
     return SMK_OK;
 }

@@ -178,6 +178,7 @@ struct smk_sim {
     int alloc();
     void release();
     int upload_mask(const uint8_t* host);
+    int mask_set();
     // CUDA graph replay of steady-state steps, one graph per ping-pong parity
     struct GraphSlot {
         cudaGraphExec_t exec = nullptr;
