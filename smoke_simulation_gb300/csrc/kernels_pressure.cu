@@ -225,26 +225,44 @@ __device__ __forceinline__ uint3 vblock(int vb, int nbx, int nby) {
 // FP64 |div u| per projectable cell (read only): the max (as IEEE bits) and whether any cell
 // exceeds tol.
 //
-// A cell's FP64 sum costs five passes through a pipe that takes a few lanes per clock and SM, and
-// bound this kernel (3.4 ms at 512^3, where its 13 bytes a cell take 0.26 ms).  Its FP32 sum d is off
-// by at most 5 * 2^-24 of the sum of the six magnitudes (five roundings, each of a partial sum no
-// larger), so a cell whose |d| + 2^-21 * that sum stays below a maximum already found cannot raise
-// it: only the others (a NaN among them) are summed in FP64.  The CTA's threads share the maximum
-// they found, which starts from the other CTAs'.  Four cells of a row per thread where the rows allow.
+// A cell's FP64 sum and its conversions go through a pipe that takes two lanes per clock and SM, and bound
+// this kernel (3.4 ms at 512^3 with every cell in FP64, where its 13 bytes a cell take 0.26 ms).  An FP32 sum d is
+// off by at most 2^-24 of the sum of its five partial sums' magnitudes (each rounding by 2^-24 of its result), so
+// with e = 3 * 2^-24 of that sum, |d| - e is a lower bound of the maximum, and a cell whose |d| + e stays below
+// a bound already found cannot raise the maximum (the third 2^-24 covers the roundings of e, of the bounds and of
+// the FP64 sum): only the others (a NaN among them) are summed in FP64.  The CTA's threads share their largest
+// lower bound, in FP32; a warp adds its own before it tests (one reduction per four cells of a row and lane).
+// 256^3: 97 us with e = 2^-21 of the six magnitudes and the shared maximum in FP64 (1.34 M FP64 instructions), 76
+// with that e and the shared bound, 52 now (0.33 M).
 __device__ __forceinline__ double div64(float u0, float u1, float v0, float v1, float w0, float w1) {
     return ((((-(double)u0 + (double)u1) + -(double)v0) + (double)v1) + -(double)w0) + (double)w1;
 }
 
-__device__ __forceinline__ void measure_cell(float u0, float u1, float v0, float v1, float w0, float w1, double& m,
-                                             unsigned long long* shared_max) {
-    const float d = ((((-u0 + u1) + -v0) + v1) + -w0) + w1;
-    const float mag = ((fabsf(u0) + fabsf(u1)) + (fabsf(v0) + fabsf(v1))) + (fabsf(w0) + fabsf(w1));
-    const float found = __double2float_rd(__longlong_as_double((long long)*(volatile unsigned long long*)shared_max));
-    if (fmaf(mag, 0x1p-21f, fabsf(d)) < found) return;
-    const double a = fabs(div64(u0, u1, v0, v1, w0, w1));
-    if (!(a <= m)) {
-        m = a;  // NaN propagates as the largest value
-        atomicMax(shared_max, (unsigned long long)__double_as_longlong(a));
+// N cells of a lane, all lanes of the warp together: f[k] their flags (0: none), c[k] their six faces.
+template <int N>
+__device__ __forceinline__ void measure_cells(const unsigned (&f)[N], const float (&c)[N][6], double& m, bool& nan,
+                                              unsigned* shared_bound) {
+    float up[N], low = 0.0f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const float* q = c[k];
+        const float s1 = -q[0] + q[1], s2 = s1 + -q[2], s3 = s2 + q[3], s4 = s3 + -q[4], d = fabsf(s4 + q[5]);
+        const float sums = ((fabsf(s1) + fabsf(s2)) + (fabsf(s3) + fabsf(s4))) + d;
+        up[k] = fmaf(sums, 0x1.8p-23f, d);
+        if (f[k] & F_PROJ) low = fmaxf(low, fmaf(sums, -0x1.8p-23f, d));  // a NaN leaves it
+    }
+    const unsigned warp_low = __reduce_max_sync(0xffffffffu, __float_as_uint(low));
+    unsigned found = *(volatile unsigned*)shared_bound;
+    if (warp_low > found) {
+        if (((threadIdx.x + threadIdx.y * BX) & 31) == 0) atomicMax(shared_bound, warp_low);
+        found = warp_low;
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        if (!(f[k] & F_PROJ) || (up[k] < __uint_as_float(found) && !nan)) continue;
+        const double a = fabs(div64(c[k][0], c[k][1], c[k][2], c[k][3], c[k][4], c[k][5]));
+        if (!(a <= m)) m = a;  // NaN propagates as the largest value
+        nan = m != m;
     }
 }
 
@@ -252,31 +270,40 @@ template <bool VEC>
 __global__ void k_refine_measure(Grid g, const float* u, const float* v, const float* w,
                                  const uint8_t* __restrict__ flags, RefineStatus* rs, double tol, int nbx,
                                  int nby, int nvb) {
-    __shared__ unsigned long long found;
+    __shared__ unsigned bound;
     if (*(volatile int*)&rs->stop) return;
-    if (threadIdx.x == 0 && threadIdx.y == 0) found = *(volatile unsigned long long*)&rs->div_bits;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        const double d = __longlong_as_double((long long)*(volatile unsigned long long*)&rs->div_bits);
+        bound = d == d ? __float_as_uint(__double2float_rd(d)) : 0u;
+    }
     __syncthreads();
     double m = 0.0;
+    bool nan = false;
     for (int vb = (int)blockIdx.x; vb < nvb; vb += (int)gridDim.x) {
         const uint3 bid = vblock(vb, nbx, nby);
         const int x = ((int)bid.x * BX + (int)threadIdx.x) * (VEC ? 4 : 1);
         const int y = (int)bid.y * BY + (int)threadIdx.y;
         const int z = (int)bid.z;
-        if (x >= g.nx || y >= g.ny || z >= g.nz) continue;
-        const int i = g.idx(x, y, z);
+        const bool in = x < g.nx && y < g.ny && z < g.nz;
+        const int i = in ? g.idx(x, y, z) : 0;
         if (VEC) {
             // a row holds at least nx + 1 elements and starts on 16 bytes: the group's loads stay in it
-            const uchar4 f = *reinterpret_cast<const uchar4*>(flags + i);
-            if (!((f.x | f.y | f.z | f.w) & F_PROJ)) continue;
+            uchar4 f = *reinterpret_cast<const uchar4*>(flags + i);
             const float4 ua = *reinterpret_cast<const float4*>(u + i);
+            const float u4 = u[i + 4];
             const float4 va = *reinterpret_cast<const float4*>(v + i), vb4 = *reinterpret_cast<const float4*>(v + i + g.X);
             const float4 wa = *reinterpret_cast<const float4*>(w + i), wb = *reinterpret_cast<const float4*>(w + i + g.XY);
-            if (f.x & F_PROJ) measure_cell(ua.x, ua.y, va.x, vb4.x, wa.x, wb.x, m, &found);
-            if (f.y & F_PROJ) measure_cell(ua.y, ua.z, va.y, vb4.y, wa.y, wb.y, m, &found);
-            if (f.z & F_PROJ) measure_cell(ua.z, ua.w, va.z, vb4.z, wa.z, wb.z, m, &found);
-            if (f.w & F_PROJ) measure_cell(ua.w, u[i + 4], va.w, vb4.w, wa.w, wb.w, m, &found);
-        } else if (flags[i] & F_PROJ) {
-            measure_cell(u[i], u[i + 1], v[i], v[i + g.X], w[i], w[i + g.XY], m, &found);
+            if (!in) f = make_uchar4(0, 0, 0, 0);
+            const unsigned fs[4] = {f.x, f.y, f.z, f.w};
+            const float c[4][6] = {{ua.x, ua.y, va.x, vb4.x, wa.x, wb.x},
+                                   {ua.y, ua.z, va.y, vb4.y, wa.y, wb.y},
+                                   {ua.z, ua.w, va.z, vb4.z, wa.z, wb.z},
+                                   {ua.w, u4, va.w, vb4.w, wa.w, wb.w}};
+            measure_cells<4>(fs, c, m, nan, &bound);
+        } else {
+            const unsigned fs[1] = {in ? flags[i] : 0u};
+            const float c[1][6] = {{u[i], u[i + 1], v[i], v[i + g.X], w[i], w[i + g.XY]}};
+            measure_cells<1>(fs, c, m, nan, &bound);
         }
     }
     // one flag store and at most one atomic per CTA, each only when it changes the stored value

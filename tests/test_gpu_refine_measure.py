@@ -10,7 +10,7 @@ from smoke_simulation_gb300 import scenes as S
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(3, 3, 3), (5, 4, 6), (13, 9, 7), (64, 5, 5), (131, 20, 18), (200, 70, 66)])
-@pytest.mark.parametrize("noise", [0.5, 1e6])
+@pytest.mark.parametrize("noise", [0.5, 1e6, 1e-30, 3e-39])  # the last two: partial sums near and below 2^-126
 def test_measured_divergence_is_numpys_float64(gpu, dims, noise):
     sc = S.Scene("m", *dims, dt=0.05, steps=1, scheme=1, iterations=6, tol=1e-12, check_every=3, refine=1,
                  refine_sweeps=2, clamp_mode=2)
