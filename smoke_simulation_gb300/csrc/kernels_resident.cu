@@ -11,9 +11,10 @@
 // element until the number is there.  That is one trip through L2 per pass (about 0.7 us) instead of
 // a barrier's three (fence, flag, data), and CTAs only wait for their neighbours.  The two colours have
 // elements of their own: a box may send its next pass before the neighbour has read this one, but
-// the pass after that needs the neighbour's next values, which are sent after it has read these.  The elements start at zero (a memset ahead of every launch),
-// pass numbers at 1.  The tolerance check exchanges one maximum per CTA, all to all, the same way.  Waits
-// are bounded: a thread that gives up, or sees *kerr set, makes its CTA record the error and leave,
+// the pass after that needs the neighbour's next values, which are sent after it has read these.  The
+// elements start at zero (a memset ahead of every launch), pass numbers at 1.  The tolerance check gathers
+// one maximum per CTA in the first one, which hands out the largest, the same way (the largest form: all
+// to all).  Waits are bounded: a thread that gives up, or sees *kerr set, makes its CTA record the error and leave,
 // and the others follow.
 //
 // Layout.  The two colours of a row are separate: cell x of parity c = (x + y + z) & 1 is element x / 2
@@ -27,8 +28,8 @@
 // What bounds it: up to about 64^3 the exchange (0.95 us a pass at 32^3, of which a pass's arithmetic is
 // 0.1), above it instruction issue (about 60 warp instructions a cell in the pressure form, 120 in the
 // velocity form).  us per 30 sweeps (a check every 6) and per 30 iterations, before (the faster of one pass per
-// launch and blocked) and now: 32^3 155 -> 87 and 113 -> 66; 64^3 205 -> 96 and 155 -> 82; 80^3 218 -> 117
-// and 261 -> 129; 100^3 238 -> 162 and 369 -> 234; 127^3 286 -> 265 and 552 -> 369.  Not kept: all loads of four
+// launch and blocked) and now: 32^3 155 -> 68 and 113 -> 66; 64^3 205 -> 78 and 155 -> 82; 80^3 218 -> 95
+// and 261 -> 129; 100^3 238 -> 150 and 369 -> 234; 127^3 286 -> 265 and 552 -> 369.  Not kept: all loads of four
 // cells ahead of their updates in the pressure form (80^3 83 -> 100 us without checks), 1024 threads on small
 // grids (64^3 65 -> 73), 512 with 14 cells each on large ones (127^3 228 -> 324).
 #include <cuda_runtime.h>
@@ -55,7 +56,8 @@ struct ResidentArgs {
     int hp;               // elements of a colour row
     int sy, sz;           // elements of a y side and of a z side in the exchange buffer
     int half;             // elements of all sides of all boxes
-    unsigned long long* ex;  // [colour][cta][y sides, z sides], then [group parity][cta] check maxima
+    unsigned long long* ex;  // [colour][cta][y sides, z sides], then [group parity][cta] check maxima and
+                             // [group parity] their maximum
     int* kerr;
 };
 
@@ -222,7 +224,9 @@ k_resident_sor(const __grid_constant__ ResidentArgs a, float* __restrict__ P, co
                float tol, StepStatus* __restrict__ status) {
     extern __shared__ float sm[];
     __shared__ float wtab[8 * 32];  // omega/acc, one copy per lane
+    constexpr bool GATHER = RT * NS <= 4096;
     __shared__ unsigned red[RT / 32];
+    __shared__ unsigned red2[GATHER ? RT / 32 : 1], all;  // GATHER: every box's maxima, the result
     const Grid g = a.g;
     const Box box(a);
     const int tid = (int)threadIdx.x, lane = tid & 31;
@@ -281,23 +285,64 @@ k_resident_sor(const __grid_constant__ ResidentArgs a, float* __restrict__ P, co
                     float pc;
                     if (acc) m = max(m, __float_as_uint(fabsf(residual(w, c, acc, bv[s][c], pc))));
                 }
-            for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (lane == 0) red[tid >> 5] = m;
-            __syncthreads();
+            const unsigned tag = (unsigned)group + 1u;
             unsigned long long* at = maxima + (size_t)(group & 1) * ctas;
-            if (tid == 0) {
-                for (int k = 1; k < RT / 32; ++k) m = max(m, red[k]);
-                ex_put(at + box.cta, __uint_as_float(m), (unsigned)group + 1u);
+            if constexpr (GATHER) {
+                // Box 0 gathers every box's maximum and hands the result out in one word: with every box polling
+                // every other's, the polls of 144 boxes met at the same lines (5.5 us a check at 32^3, 1.8 now).  The
+                // sweeps' barriers lie between the uses of `red` and `all` by two checks.
+                auto warps = [&](const unsigned* r) {
+                    return __reduce_max_sync(0xffffffffu, lane < RT / 32 ? r[lane] : 0u);
+                };
+                unsigned long long* const verdict = maxima + 2 * (size_t)ctas + (group & 1);
+                m = __reduce_max_sync(0xffffffffu, m);
+                if (lane == 0) red[tid >> 5] = m;
+                __syncthreads();
+                if (tid < 32) {
+                    m = warps(red);
+                    if (tid == 0) ex_put(at + box.cta, __uint_as_float(m), tag);
+                }
+                if (box.cta == 0) {
+                    const unsigned one[1] = {tid < ctas ? (unsigned)tid : SLOT_NONE};
+                    m = 0u;
+                    bad = !receive<1>(a, at, one, tag, [&](int, float v) { m = __float_as_uint(v); });
+                    m = __reduce_max_sync(0xffffffffu, m);
+                    if (lane == 0) red2[tid >> 5] = m;
+                    bad = __syncthreads_or(bad);
+                    if (tid < 32 && !bad) {
+                        m = warps(red2);
+                        if (tid == 0) {
+                            ex_put(verdict, __uint_as_float(m), tag);
+                            all = m;
+                        }
+                    }
+                } else if (tid == 0) {
+                    const unsigned one[1] = {0u};
+                    bad = !receive<1>(a, verdict, one, tag, [&](int, float v) { all = __float_as_uint(v); });
+                }
+                bad = __syncthreads_or(bad);
+                if (bad) break;
+                m = all;
+            } else {
+                // every box polls every other's: the gather's code costs the sweeps of this form its registers
+                // (127^3 without checks 232 -> 236 us, a check 6.5 -> 5.2)
+                for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+                if (lane == 0) red[tid >> 5] = m;
+                __syncthreads();
+                if (tid == 0) {
+                    for (int k = 1; k < RT / 32; ++k) m = max(m, red[k]);
+                    ex_put(at + box.cta, __uint_as_float(m), tag);
+                }
+                unsigned one[1] = {tid < ctas ? (unsigned)tid : SLOT_NONE};
+                m = 0u;
+                bad = !receive<1>(a, at, one, tag, [&](int, float v) { m = __float_as_uint(v); });
+                for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+                __syncthreads();  // red has been read
+                if (lane == 0) red[tid >> 5] = m;
+                bad = __syncthreads_or(bad);
+                if (bad) break;
+                for (int k = 0; k < RT / 32; ++k) m = max(m, red[k]);
             }
-            unsigned one[1] = {tid < ctas ? (unsigned)tid : SLOT_NONE};
-            m = 0u;
-            bad = !receive<1>(a, at, one, (unsigned)group + 1u, [&](int, float v) { m = __float_as_uint(v); });
-            for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-            __syncthreads();  // red has been read
-            if (lane == 0) red[tid >> 5] = m;
-            bad = __syncthreads_or(bad);
-            if (bad) break;
-            for (int k = 0; k < RT / 32; ++k) m = max(m, red[k]);
             const bool done = __uint_as_float(m) <= tol;
             if (box.cta == 0 && tid == 0) {
                 status->rmax_bits[group] = m;
@@ -308,7 +353,7 @@ k_resident_sor(const __grid_constant__ ResidentArgs a, float* __restrict__ P, co
             }
             if (done) break;
             ++group;
-            __syncthreads();
+            if constexpr (!GATHER) __syncthreads();
         }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -573,7 +618,7 @@ bool resident_plan(const Grid& g, bool velocity, int sms, ResidentPlan* out) {
 
 size_t resident_exchange_bytes(const ResidentPlan& p) {
     const size_t ctas = (size_t)p.cy * (size_t)p.cz;
-    return (2 * ctas * 2 * (size_t)(p.by + p.bz) * (size_t)p.hx + 2 * ctas) * sizeof(unsigned long long);
+    return (2 * ctas * 2 * (size_t)(p.by + p.bz) * (size_t)p.hx + 2 * ctas + 2) * sizeof(unsigned long long);
 }
 
 int prepare_resident_kernels() {

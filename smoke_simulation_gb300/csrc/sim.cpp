@@ -676,8 +676,8 @@ void smk_sim::choose_sweep(int sms) {
 
 // Every grid with a plan takes it (up to about 128^3; us per 30 sweeps or iterations, one pass per launch /
 // blocked / resident).  Velocity form: 32^3 113 / - / 66, 64^3 155 / - / 82, 80^3 261 / - / 129, 100^3 380 /
-// 369 / 234, 127^3 552 / 592 / 369.  Pressure form with a check every 6 sweeps: 32^3 155 / 208 / 87, 64^3
-// 275 / 205 / 96, 100^3 648 / 238 / 162, 127^3 978 / 286 / 265; without checks 127^3 308 / 242 / 228.
+// 369 / 234, 127^3 552 / 592 / 369.  Pressure form with a check every 6 sweeps: 32^3 155 / 208 / 68, 64^3
+// 275 / 205 / 78, 100^3 648 / 238 / 150, 127^3 978 / 286 / 265; without checks 127^3 308 / 242 / 228.
 void smk_sim::choose_resident() {
     const int sms = device_sms();
     res_p_fits = resident_plan(g, false, sms, &res_p);
