@@ -91,6 +91,7 @@ def test_forms_may_change_between_steps_and_streams(gpu):
         s.close()
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("graphs", [True, False])
 def test_resident_solves_on_several_streams_at_once(gpu, graphs):
     """Simulations stepped on their own streams, their resident solves (each a cooperative launch over the
